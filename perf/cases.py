@@ -189,3 +189,67 @@ def tolerance(case):
     # rel 2.9e-4 to 3.0e-4 in fp16 and 2.1e-3 to 2.6e-3 in bf16 (largest single difference 0.011 and 0.082 of the
     # root mean square); the bounds are four times that.
     return {"rel": 1.2e-3, "max": 0.045} if case["dtype"] == "fp16" else {"rel": 1e-2, "max": 0.33}
+
+
+def _quantised(x):
+    """int8 per block of 128 tokens and back: round-half-even(x / scale) * scale, scale = max|x| / 127 in fp32."""
+    B, H, N, D = x.shape
+    pad = (N + 127) // 128 * 128 - N
+    blocks = torch.nn.functional.pad(x.float(), (0, 0, 0, pad)).view(B, H, -1, 128, D)
+    scale = blocks.abs().amax((3, 4), keepdim=True) / 127.0
+    scale = torch.where(scale > 0, scale, torch.ones_like(scale))
+    q = (blocks / scale).round().clamp(-127, 127).double() * scale.double()
+    return q.view(B, H, N + pad, D)[:, :, :N]
+
+
+def _attention64(q, k, v, causal):
+    """(B,H,N,D) -> fp64 output and log-sum-exp; causal rows are the last positions."""
+    B, Hq, Nq, D = q.shape
+    Hkv, Nk = k.shape[1], k.shape[2]
+    out = torch.empty((B, Hq, Nq, D), dtype=torch.float64, device=q.device)
+    lse = torch.empty((B, Hq, Nq), dtype=torch.float64, device=q.device)
+    step = max(1, (1 << 26) // Nk)
+    cols = torch.arange(Nk, device=q.device)
+    for b in range(B):
+        for h in range(Hq):
+            kh, vh = k[b, h // (Hq // Hkv)].double(), v[b, h // (Hq // Hkv)].double()
+            for r0 in range(0, Nq, step):
+                s = q[b, h, r0:r0 + step].double() @ kh.T / math.sqrt(D)
+                if causal:
+                    rows = torch.arange(r0, r0 + s.shape[0], device=q.device) + (Nk - Nq)
+                    s.masked_fill_(cols[None, :] > rows[:, None], float("-inf"))
+                z = torch.logsumexp(s, 1)
+                lse[b, h, r0:r0 + step] = z
+                out[b, h, r0:r0 + step] = torch.exp_(s.sub_(z[:, None])) @ vh
+    return out, lse
+
+
+def exact(case, seed):
+    """The outputs of ``run`` in 64 bits, in plain torch; None where that would take long."""
+    c = case
+    if c["B"] * c["Hq"] * c["Nq"] * c["Nk"] > 2e10:
+        return None
+    s = prepare(c, seed)
+    if c["op"] == "module":
+        m, x = s["m"], s["x"].double()
+        lin = lambda layer, y: y @ layer.weight.double().T + layer.bias.double()  # noqa: E731
+        B, N, d = x.shape
+        q = lin(m.w_q, x).view(B, N, c["Hq"], c["D"]).transpose(1, 2)
+        kv = lin(m.kv, x).view(B, N, 2, c["Hkv"], c["D"])
+        o, _ = _attention64(q, kv[:, :, 0].transpose(1, 2), kv[:, :, 1].transpose(1, 2), True)
+        return lin(m.w_o, o.transpose(1, 2).reshape(B, N, d))
+    q, k, v = (t if c["layout"] == "bhnd" else t.transpose(1, 2) for t in (s["q"], s["k"], s["v"]))
+    if c["op"] == "int8":
+        mean = k.double().mean(2, keepdim=True).float()
+        q, k = _quantised(q), _quantised(k.float() - mean)
+    if c["op"] == "shard":
+        G = c["Hq"] // c["Hkv"]
+        out = torch.zeros(q.shape, dtype=torch.float64, device=q.device)
+        for b, hk in parallel.shard_units(c["B"], c["Hkv"], c["world"], 0):
+            qs = slice(hk * G, (hk + 1) * G)
+            out[b:b + 1, qs] = _attention64(q[b:b + 1, qs], k[b:b + 1, hk:hk + 1], v[b:b + 1, hk:hk + 1], c["causal"])[0]
+        return out
+    o, lse = _attention64(q, k, v, c["causal"])
+    if c["layout"] == "bnhd":
+        o = o.transpose(1, 2)
+    return (o, lse) if c["lse"] else o
