@@ -123,6 +123,11 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p);
  * gain (many rounds, or too little work per item) the launch is the plain one and scratch is not
  * touched.  Results equal miniattn_fwd's up to fp32 summation order.
  *
+ * A call with few query rows per KV head (decode: see plan_decode, csrc/plan.cu) runs another
+ * kernel under MINIATTN_KERNEL_AUTO, with and without scratch; with it, the key range of its items
+ * is cut over CTAs by the same contract, and no CTA waits for another.  miniattn_plan_fwd below
+ * describes the general kernel's launch.
+ *
  * scratch: device memory, 256-byte aligned, at least miniattn_fwd_balanced_scratch_bytes(p)
  * bytes.  Its first 16384 bytes (the arrival counters) must be zero before the first launch that
  * uses it; every launch leaves them zero again, unless a bounded device wait ran out (status

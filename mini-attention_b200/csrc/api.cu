@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -25,6 +26,10 @@ cudaError_t launch_fwd_ws_int8qk(int D, bool bf16, const CUtensorMap* tm, const 
                                  int sm_count, cudaStream_t st);
 cudaError_t launch_fwd_ws_plan(int D, bool bf16, bool qk8, const CUtensorMap* tm, const FwdArgs& a,
                                const FwdPlan& plan, cudaStream_t st);
+cudaError_t launch_fwd_decode(int D, bool bf16, const CUtensorMap* tm, const DecodeArgs& a, int rg, int n_ctas,
+                              cudaStream_t st);
+void plan_decode(int B, int Hq, int Hkv, int Nq, int Nk, int D, int causal, long long diag, int sms, bool cut,
+                 DecodePlan* d);
 void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan);
 cudaError_t launch_quant_qk(int D, bool bf16, const void* q, const long long* qs, const void* k,
                             const long long* ks, int B, int Hq, int Hkv, int Nq, int Nk, float q_fold,
@@ -350,6 +355,71 @@ static int bind_scratch(const ma::FwdPlan& plan, int D, void* scratch, size_t sc
   return MINIATTN_OK;
 }
 
+// ---- calls with few query rows per KV head (fwd_decode.cu) ----
+static void decode_plan_of(const MiniAttnFwdParams* p, int sms, bool cut, ma::DecodePlan* d) {
+  *d = ma::DecodePlan{};
+  if (p->kernel != MINIATTN_KERNEL_AUTO || p->carry_in || p->carry_out) return;
+  if (p->B <= 0 || p->Hkv <= 0 || p->Hq <= 0 || p->Hq % p->Hkv != 0 || p->Nq <= 0 || p->Nk <= 0) return;
+  ma::plan_decode(p->B, p->Hq, p->Hkv, p->Nq, p->Nk, kernel_head_dim(p->D), p->causal, p->q_pos0 - p->k_pos0, sms, cut, d);
+}
+
+static size_t decode_scratch_bytes(const ma::DecodePlan& d, int D) {
+  if (d.rg == 0 || d.total / d.tiles == d.n_ctas) return 0;  // one whole item per CTA: nothing is cut
+  const size_t rows = static_cast<size_t>(2 * d.n_ctas) * 16 * d.rg;
+  return kCounterBytes + align256(rows * sizeof(float2)) + rows * kernel_head_dim(D) * sizeof(float);
+}
+
+static int fwd_decode(const MiniAttnFwdParams* p, const ma::DecodePlan& d, void* scratch, size_t scratch_bytes,
+                      cudaStream_t st) {
+  const CUtensorMapDataType dt =
+      p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  CUtensorMap tm[2];
+  int rc;
+  if ((rc = make_map(&tm[0], p->k, 2, dt, p->D, p->Nk, p->Hkv, p->B, p->k_stride, ma::kBoxCols, 64, "k")) != 0)
+    return rc;
+  if ((rc = make_map(&tm[1], p->v, 2, dt, p->D, p->Nk, p->Hkv, p->B, p->v_stride, ma::kBoxCols, 64, "v")) != 0)
+    return rc;
+  ma::DecodeArgs a{};
+  a.q = static_cast<const uint16_t*>(p->q);
+  a.o = static_cast<uint16_t*>(p->o);
+  for (int i = 0; i < 3; ++i) {
+    a.qs[i] = p->q_stride[i];
+    a.os[i] = p->o_stride[i];
+  }
+  a.lse = p->lse;
+  a.status = p->status;
+  a.diag = p->q_pos0 - p->k_pos0;
+  a.total = d.total;
+  a.Nq = p->Nq;
+  a.Nk = p->Nk;
+  a.Hq = p->Hq;
+  a.Hkv = p->Hkv;
+  a.G = p->Hq / p->Hkv;
+  a.D = p->D;
+  a.causal = p->causal;
+  a.rows = a.G * p->Nq;
+  a.n_rb = d.n_rb;
+  a.tiles = d.tiles;
+  a.scale_log2 = (p->softmax_scale > 0.f ? p->softmax_scale : 1.0f / sqrtf((float)p->D)) * 1.4426950408889634f;
+  const size_t need = decode_scratch_bytes(d, p->D);
+  if (need > 0) {
+    if (scratch_bytes < need)
+      return fail(MINIATTN_EINVAL, "scratch holds %zu bytes, this launch needs %zu "
+                  "(miniattn_fwd_balanced_scratch_bytes)", scratch_bytes, need);
+    if (reinterpret_cast<uintptr_t>(scratch) % 256 != 0)
+      return fail(MINIATTN_EINVAL, "scratch must be 256-byte aligned");
+    uint8_t* base = static_cast<uint8_t*>(scratch);
+    const size_t rows = static_cast<size_t>(2 * d.n_ctas) * 16 * d.rg;
+    a.counters = reinterpret_cast<int*>(base);
+    a.part_ml = reinterpret_cast<float2*>(base + kCounterBytes);
+    a.part_o = reinterpret_cast<float*>(base + kCounterBytes + align256(rows * sizeof(float2)));
+  }
+  const cudaError_t e =
+      ma::launch_fwd_decode(kernel_head_dim(p->D), p->dtype == MINIATTN_BF16, tm, a, d.rg, d.n_ctas, st);
+  if (e != cudaSuccess) return fail(MINIATTN_ECUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+  return MINIATTN_OK;
+}
+
 // Forward launch shared by miniattn_fwd and miniattn_fwd_balanced (scratch == nullptr: plain).
 static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_bytes, void* stream) {
   g_err[0] = 0;
@@ -358,6 +428,9 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   const bool has_keys = p->Nk > 0;
   int sms = 0;
   if ((rc = check_device(&sms)) != 0) return rc;
+  ma::DecodePlan dec;
+  decode_plan_of(p, sms, scratch != nullptr, &dec);
+  if (dec.rg != 0) return fwd_decode(p, dec, scratch, scratch_bytes, reinterpret_cast<cudaStream_t>(stream));
 
   const CUtensorMapDataType dt =
       p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -492,7 +565,11 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p) {
 int64_t miniattn_fwd_balanced_scratch_bytes(const MiniAttnFwdParams* p) {
   MiniAttnPlanInfo info;
   const int rc = miniattn_plan_fwd(p, 0, &info, nullptr, 0);
-  return rc != 0 ? rc : info.scratch_bytes;
+  if (rc != 0) return rc;
+  // the larger of the two launches' needs: the INT8-QK entry sizes its scratch with the same call
+  ma::DecodePlan dec;
+  decode_plan_of(p, info.sm_count, true, &dec);
+  return std::max<int64_t>(info.scratch_bytes, static_cast<int64_t>(decode_scratch_bytes(dec, p->D)));
 }
 
 static int check_int8_params(const MiniAttnInt8Params* p, bool need_v) {

@@ -60,6 +60,31 @@ struct FwdPlan {
   PlanTable table;
 };
 
+// Few query rows per KV head (fwd_decode.cu): an item is (batch, KV head, block of rows), its rows are
+// token * G + (head of the group); the tiles of all items, one after the other, are cut evenly over the CTAs.
+struct DecodeArgs {
+  const uint16_t* q;
+  uint16_t* o;
+  long long qs[3], os[3];  // element strides: batch, head, token
+  float*   lse;
+  int32_t* status;
+  long long diag;          // q_pos0 - k_pos0
+  long long total;         // tiles of all items
+  int Nq, Nk, Hq, Hkv, G, D, causal;
+  int rows;                // G * Nq
+  int n_rb;                // row blocks per (batch, KV head)
+  int tiles;               // 64-key tiles of an item
+  float scale_log2;
+  float*  part_o;          // [2 * CTAs][rows of an item][D] fp32: pieces of cut items, un-normalised
+  float2* part_ml;         // [2 * CTAs][rows of an item]: (row maximum in log2 units, row sum)
+  int*    counters;        // [CTAs]: pieces published of the item that starts in that CTA; zero between launches
+};
+struct DecodePlan {
+  int rg;                  // 16-row groups of an item (1, 2 or 4); 0: the call is not one for this kernel
+  int n_rb, tiles, n_ctas;
+  long long total;
+};
+
 constexpr int kTileM = 128;   // query rows per MMA tile (TMEM lanes)
 constexpr int kTileN = 128;   // keys per K/V tile
 constexpr int kBoxCols = 64;  // 16-bit elements per 128-byte swizzled row

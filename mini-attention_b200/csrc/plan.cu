@@ -269,4 +269,50 @@ void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan) {
   }
 }
 
+// Calls with few query rows per KV head (fwd_decode.cu).  d->rg stays 0 where fwd_ws.cu is the faster one.
+void plan_decode(int B, int Hq, int Hkv, int Nq, int Nk, int D, int causal, long long diag, int sms, bool cut,
+                 DecodePlan* d) {
+  *d = DecodePlan{};
+  long long kv_end = Nk;
+  if (causal) kv_end = std::min(kv_end, diag + Nq);
+  const int G = Hq / Hkv;
+  const long long rows = static_cast<long long>(G) * Nq;
+  if (kv_end <= 0 || Nq > 64) return;
+  const int rg = rows <= 16 ? 1 : rows <= 32 ? 2 : 4;
+  const long long n_rb = (rows + 16 * rg - 1) / (16 * rg);
+  const long long items = static_cast<long long>(B) * Hkv * n_rb;
+  if (items > 0x3fffffffll) return;
+  const int tiles = static_cast<int>((kv_end + 63) / 64);
+  const long long total = items * tiles;
+  const long long slots = 2ll * sms;  // two CTAs per SM
+  // Which kernel.  Measured on B200 (us, fwd_ws / this one, bf16, causal, the last Nq of Nk positions):
+  //   up to 16 rows   bound by HBM here, never slower: 8x8 KV heads, D=128, Nk=4096: G=1 Nq=1 42 / 37,
+  //                   G=8 Nq=1 194 / 38; 1x2 KV heads, Nk=1024, G=1: 18.5 / 14.3
+  //   17 to 32 rows   a tile costs its warps about as long as HBM takes to deliver it: G=4 Nq=8, Nk=1024:
+  //                   1x2 KV heads 20.5 / 20.5, 8x8 36.9 / 24.6; but one query head (G=1 Nq=32, 8x8,
+  //                   Nk=4096) 42.0 / 45.1 at D=128, 33.8 / 30.8 at D=64
+  //   more            bound by mma.sync: a block of 64 rows takes as long as two tcgen05 tiles of fwd_ws,
+  //                   which needs one per query head (8x8, Nk=16384: G=2 Nq=32 189 / 150, G=8 Nq=32
+  //                   671 / 464, G=4 Nq=64 353 / 465), and only where there is work for every SM: fwd_ws cuts
+  //                   few long items better (1x2, G=8 Nq=8, Nk=4096: 27.8 / 43.0)
+  if (rg == 2 && G == 1 && D == 128) return;
+  if (rg == 4 && (G < 2 * n_rb || G * total < 16 * slots)) return;
+  d->rg = rg;
+  d->n_rb = static_cast<int>(n_rb);
+  d->tiles = tiles;
+  d->total = total;
+  if (!cut) {
+    d->n_ctas = static_cast<int>(items);
+    return;
+  }
+  // Pieces of an item: at least four tiles long, and no more than balances a tile's time against what the
+  // CTA that folds them spends on each (in us: a round trip to L2 shared by eight, and the piece's rows at
+  // what one SM reads).
+  const double t_tile = rg == 1 ? 0.5 : rg == 2 ? 0.8 : 1.5;
+  const double t_fold = 0.02 + std::min<double>(rows, 16 * rg) * D * 4 / 55e3;
+  const long long most = std::max(1ll, std::min<long long>(tiles / 4, static_cast<long long>(std::sqrt(tiles * t_tile / t_fold))));
+  if (items * most >= slots && total >= 8 * slots) d->n_ctas = static_cast<int>(slots);
+  else d->n_ctas = static_cast<int>(std::min(slots, items * std::max(1ll, std::min(most, slots / items))));
+}
+
 }  // namespace ma

@@ -18,6 +18,7 @@ from . import _lib
 
 _DTYPES = {torch.float16: _lib.FP16, torch.bfloat16: _lib.BF16}
 _status_words: dict = {}
+_COUNTER_BYTES = 16384        # arrival counters at the start of a balanced launch's scratch
 _balance_scratch: dict = {}   # (device index, stream) -> zero-initialised uint8 scratch tensor
 # Parameter blocks of recent calls, keyed by everything that goes into one (pointers, shapes, strides,
 # dtype, flags).  A training or serving loop calls the operator with the same tensors again and again;
@@ -64,7 +65,13 @@ def check_device_status(device: Union[torch.device, str, None] = None) -> None:
 
 def _scratch_for(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
     """Scratch of a balanced launch: one buffer per (device, stream), zeroed when created (the
-    kernels leave the arrival counters at its start zero again), grown on demand."""
+    kernels leave the arrival counters at its start zero again), grown on demand.  A call that is being
+    captured gets a buffer of its own from the graph's memory, its counters cleared by the graph: a
+    captured launch may be replayed on any stream."""
+    if torch.cuda.is_current_stream_capturing():
+        t = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        t[:_COUNTER_BYTES].zero_()
+        return t
     key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
     t = _balance_scratch.get(key)
     if t is None or t.numel() < nbytes:

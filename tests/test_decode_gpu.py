@@ -1,0 +1,103 @@
+"""Calls with few query rows per KV head (csrc/fwd_decode.cu): the rows of all query heads of a KV head form
+one item, and the 64-key tiles of all items are cut evenly over the CTAs of the launch.
+
+Each case is compared with the CPU oracle and, with ``kernel="ws"``, with the general kernel.  Tolerances: the
+oracle bars of conftest.TOL; between the two kernels twice the 16-bit rounding of outputs of this size (both
+round the same value once, to either side), lse to fp32 summation order."""
+import pytest
+import torch
+
+import miniattn
+from conftest import TOL
+from oracle.attention_oracle import attention_reference, make_inputs
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# B, Hq, Hkv, Nq, Nk, D: rows per KV head around 16 / 32 / 64 and past it; keys around the 64-key tile; few and
+# many items; pieces that start and end inside an item; D = 96 (columns past it are zero-filled)
+CASES = [
+    (1, 1, 1, 1, 1, 128), (1, 1, 1, 1, 64, 64), (1, 3, 1, 5, 65, 96), (2, 16, 1, 1, 63, 128),
+    (1, 17, 17, 1, 700, 64), (1, 16, 1, 1, 4099, 128), (3, 8, 2, 4, 257, 128), (3, 10, 5, 8, 1025, 64),
+    (2, 24, 8, 6, 333, 96), (1, 8, 1, 4, 5000, 128), (1, 2, 1, 16, 511, 128), (1, 1, 1, 32, 130, 64),
+    (1, 8, 1, 5, 40000, 128), (16, 64, 8, 5, 1030, 128), (16, 64, 8, 8, 1100, 64), (8, 64, 8, 9, 2500, 128),
+    (8, 64, 8, 32, 1200, 64), (160, 4, 2, 2, 100, 64), (37, 8, 8, 1, 513, 128),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("causal,layout,balance", [(True, "bhnd", True), (True, "bnhd", True), (False, "bnhd", True),
+                                                   (True, "bhnd", False)])
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D", CASES)
+def test_matches_the_oracle_and_the_general_kernel(B, Hq, Hkv, Nq, Nk, D, causal, layout, balance, dtype):
+    q, k, v = make_inputs(B, Hq, Hkv, Nq, Nk, D, dtype, seed=Nk + Nq)
+    pos = Nk - Nq  # negative where there are more queries than keys: the first rows see nothing
+    put = (lambda t: t.to(DEV)) if layout == "bhnd" else (lambda t: t.transpose(1, 2).contiguous().to(DEV))
+    room = torch.full((B, Hkv, Nk + 70, D), float("nan"), dtype=dtype)  # the cache behind the filled part
+    kc, vc = room.clone(), room.clone()
+    kc[:, :, :Nk], vc[:, :, :Nk] = k, v
+    cut = (lambda t: t[:, :, :Nk]) if layout == "bhnd" else (lambda t: t[:, :Nk])
+    qd, kd, vd = put(q), cut(put(kc)), cut(put(vc))
+    kw = dict(causal=causal, layout=layout, q_pos0=pos if causal else 0, return_lse=True)
+    outs = [miniattn.flash_attn_fwd(qd, kd, vd, balance=balance, **kw) for _ in range(2)]
+    ws, ws_lse = miniattn.flash_attn_fwd(qd, kd, vd, kernel="ws", **kw)
+    assert miniattn.device_status(DEV) == 0
+    back = (lambda t: t.float().cpu()) if layout == "bhnd" else (lambda t: t.float().cpu().transpose(1, 2))
+    if B * Hq * Nq * Nk <= 4_000_000:
+        ref, ref_lse = attention_reference(q, k, v, causal=causal, q_pos0=kw["q_pos0"], return_lse=True,
+                                           out_dtype=torch.float32)
+    else:
+        ref, ref_lse = back(ws), ws_lse.cpu()
+    finite = torch.isfinite(ref_lse)
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    for out, lse in outs:
+        o, lse = back(out), lse.cpu()
+        assert (o - ref).abs().max().item() <= TOL[dtype]
+        assert (o - back(ws)).abs().max().item() <= 2 * ulp * max(1.0, ref.abs().max().item())
+        assert torch.equal(torch.isfinite(lse), finite)
+        assert float(o[~finite].abs().max() if (~finite).any() else 0.0) == 0.0
+        if finite.any():
+            assert (lse[finite] - ref_lse[finite]).abs().max().item() <= 1e-3
+
+
+def test_strided_views_and_output_views():
+    """Heads and tokens picked out of wider tensors, the result into a view: no form is copied first."""
+    g = torch.Generator().manual_seed(3)
+    wide_q = torch.randn(2, 12, 7, 160, generator=g).to(torch.float16).to(DEV)
+    wide_k = torch.randn(2, 4, 900, 136, generator=g).to(torch.float16).to(DEV)
+    wide_v = torch.randn(2, 900, 6, 128, generator=g).to(torch.float16).to(DEV)
+    q, k, v = wide_q[:, ::2, 1:6, 16:144], wide_k[:, ::2, 5:805, :128], wide_v[:, 50:850, 1:5:2].transpose(1, 2)
+    big = torch.zeros(2, 6, 9, 128, dtype=torch.float16, device=DEV)
+    out = big[:, :, 2:7]
+    miniattn.flash_attn_fwd(q, k, v, causal=True, q_pos0=795, out=out)
+    ref = attention_reference(q.cpu(), k.cpu(), v.cpu(), causal=True, q_pos0=795, out_dtype=torch.float32)
+    assert (out.float().cpu() - ref).abs().max().item() <= TOL[torch.float16]
+    assert float(big[:, :, :2].abs().max()) == 0.0 and float(big[:, :, 7:].abs().max()) == 0.0
+    assert miniattn.device_status(DEV) == 0
+
+
+def test_captured_calls_have_scratch_of_their_own():
+    """Graphs captured one after the other share torch's capture stream; replayed on two streams at once, and
+    beside eager calls, their partial results must not meet."""
+    def make(seed):
+        q, k, v = make_inputs(2, 8, 2, 1, 6000, 128, torch.float16, seed=seed)
+        return q.to(DEV), k.to(DEV), v.to(DEV)
+    ins = [make(s) for s in (1, 2)]
+    want = [miniattn.flash_attn_fwd(*x).clone() for x in ins]
+    graphs, outs = [], []
+    for x in ins:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            outs.append(miniattn.flash_attn_fwd(*x))
+        graphs.append(g)
+    streams = [torch.cuda.Stream() for _ in ins]
+    torch.cuda.synchronize()
+    for _ in range(50):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        miniattn.flash_attn_fwd(*ins[0])
+    torch.cuda.synchronize()
+    for o, w in zip(outs, want):
+        assert (o.float() - w.float()).abs().max().item() <= 2.0 ** -10  # fp32 order of the folds, one rounding
+    assert miniattn.device_status(DEV) == 0
