@@ -1,17 +1,17 @@
 // Forward attention, warp-specialised sm_100a kernel.
 //
-// One CTA (512 threads) per work item = two 128-row Q tiles of one (batch, head).  Same math as
+// One CTA (384 threads) per work item = two 128-row Q tiles of one (batch, head).  Same math as
 // the reference mainloop (kernels/flash_attn/cuda/sm_120/kernel/include/forward_kernel.cuh:137-221
 // and softmax.cuh:29-138), restructured for tcgen05 / TMEM / TMA:
 //
 //   warps 0-3   softmax of Q tile 0   (thread = one query row; S row read from TMEM), then its
-//               epilogue (O / l -> 16 bit -> swizzled smem -> TMA store)
-//   warps 4-7   softmax and epilogue of Q tile 1
-//   warps 8-11  correction: rescales the O accumulators in TMEM when a row maximum moved (rare)
-//   warp 12     MMA issuer of Q tile 0 (one thread issues its tcgen05.mma stream)
-//   warp 14     MMA issuer of Q tile 1
-//   warp 13     TMA producer: Q tiles once, then K_0, V_0, K_1, V_1, ... through a ring
-//   warp 15     idle (donates its registers)
+//               epilogue (O / l -> 16 bit -> swizzled smem -> TMA store); they also rescale the
+//               tile's O accumulator in TMEM where a row maximum moved (rare)
+//   warps 4-7   the same for Q tile 1
+//   warp 8      MMA issuer of Q tile 0 (one thread issues its tcgen05.mma stream)
+//   warp 10     MMA issuer of Q tile 1
+//   warp 9      TMA producer: Q tiles once, then K_0, V_0, K_1, V_1, ... through a ring
+//   warp 11     idle (donates its registers)
 //
 // A 128-key K/V tile is worked on as two 64-key halves ("a", "b").  Each Q tile owns two S
 // buffers of 64 TMEM columns; the 16-bit P of a half overwrites the first 32 columns of its own
@@ -27,7 +27,18 @@
 //
 // The row maximum is updated lazily: a row keeps exponentiating against a stale maximum until the
 // true maximum has grown by more than 2^8 (in the exp2 domain), so the O accumulator is rescaled
-// only rarely; l is accumulated against the same maximum, which keeps O / l exact.
+// only rarely; l is accumulated against the same maximum, which keeps O / l exact.  The exponentials
+// of a half are taken before its maximum is known (it is found in the same instruction stream) and
+// taken again where it turns out to have grown that much.
+//
+// What bounds it (clock stamps, N = 2048, D = 128, per 128-key step of a CTA, about 2980 clk): the MMAs
+// of a step need 2608 clk of the tensor pipe, and they and TMA 2560 clk of the 128 B/clk shared-memory
+// port (Q is re-read for each half); a softmax thread is busy 2380 clk of it and waits 570.  With the
+// maximum found before the exponentials and handed to four correction warps it was 2650 busy of 3140:
+// N = 8192 (2 x 8 heads, fp16) 446 -> 428 us, 4096 GQA causal bf16 524 -> 500, 32768 (16 heads) 3956 ->
+// 3743.  At D = 64 the softmax thread is the bound (2700 clk, 330 of them waiting).  One MMA of 128 keys
+// for S (2080 clk of tensor work) measured slower, 49 against 41 us at N = 2048: TMEM has room for one
+// S buffer per Q tile then, and the thread waits 1600 clk per step for PV and the next S.
 //
 // Softmax arithmetic runs two scores per issue slot (packed f32x2 FMA / ADD); a share of the
 // exponentials is evaluated by a cubic on the FMA pipe instead of the exp2 unit.
@@ -47,13 +58,14 @@ namespace ma {
 
 namespace {
 
-constexpr int kNumThreads = 512;
+constexpr int kNumThreads = 384;
+constexpr int kWarpMma0 = 8, kWarpTma = 9, kWarpMma1 = 10;  // warp 11 only donates its registers
 constexpr int kHalfN = kTileN / 2;      // keys per half tile
 constexpr float kLazyThreshold = 8.0f;  // log2 units
-// Register split per thread after setmaxnreg (8 softmax + 4 correction + 4 other warps;
-// 8*176 + 4*88 + 4*72 = 2048 = the 64 K registers of an SM divided by 32 lanes).
-constexpr int kRegSoftmax = 176;
-constexpr int kRegCorr = 88;
+// Register split per thread after setmaxnreg: 8 softmax warps + 4 others.  The launch allocates 168
+// registers for each of the 384 threads (65536 / 384, rounded down to a multiple of 8), and
+// 8*216 + 4*72 = 12*168: what the others release is what the softmax warps take.
+constexpr int kRegSoftmax = 216;
 constexpr int kRegOther = 72;
 
 template <int D, bool QK8 = false>
@@ -68,18 +80,14 @@ struct WsLayout {
   static constexpr int kOffBiasA = kOffRing + kStages * kTileBytes;
   static constexpr int kOffBiasB = kOffBiasA + kTileM * 128;
   static constexpr int kBiasBytes = QK8 ? (kTileM + kTileN / 2) * 128 : 0;
-  static constexpr int kOffAlpha = kOffBiasA + kBiasBytes;           // float[2 tiles][2 halves][128]
-  static constexpr int kOffL = kOffAlpha + 2048;                     // float[2][128]
-  static constexpr int kOffBar = kOffL + 1024;
+  static constexpr int kOffBar = kOffBiasA + kBiasBytes;
   // barrier indices (8 bytes each); [t][h] = index + 2*t + h
   static constexpr int kBarQFull = 0;                      // [2]
   static constexpr int kBarKvFull = 2;                     // [kStages]
   static constexpr int kBarKvEmpty = kBarKvFull + kStages; // [kStages]
   static constexpr int kBarSFull = kBarKvEmpty + kStages;  // [2][2] MMA -> softmax
   static constexpr int kBarPReady = kBarSFull + 4;         // [2][2] softmax -> MMA
-  static constexpr int kBarAlpha = kBarPReady + 4;         // [2][2] softmax -> correction
-  static constexpr int kBarOReady = kBarAlpha + 4;         // [2][2] correction -> MMA
-  static constexpr int kBarODone = kBarOReady + 4;         // [2][2] MMA -> correction
+  static constexpr int kBarODone = kBarPReady + 4;         // [2][2] MMA -> softmax (rescale, epilogue)
   static constexpr int kBarStagger = kBarODone + 4;        // one-shot: tile 0 published its first row maxima
   static constexpr int kNumBars = kBarStagger + 1;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;  // tmem slot, abort flag, arrival order [2]
@@ -137,7 +145,6 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   const uint32_t sQ = sbase + L::kOffQ;
   const uint32_t sRing = sbase + L::kOffRing;
-  float* alpha_smem = reinterpret_cast<float*>(gbase + L::kOffAlpha);
   const uint32_t bars = sbase + L::kOffBar;
   auto bar = [&](int idx) -> uint32_t { return bars + 8u * idx; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + L::kOffMisc);
@@ -227,12 +234,12 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int n_fill = 2 * n_tiles;
   const int n_early = min(n_fill, L::kStages);  // first use of every ring slot: nothing to wait for
 
-  if (warp == 13) {
+  if (warp == kWarpTma) {
     // one barrier per lane: arrival counts by index range
     for (int i = lane; i < L::kNumBars; i += 32) {
       uint32_t count = 1;  // Q full, K/V full, S full, O done: one arrival (a TMA or MMA commit)
       if (i >= L::kBarKvEmpty && i < L::kBarSFull) count = nt;      // one release per issuing thread
-      else if (i >= L::kBarPReady && i < L::kBarODone) count = 4;   // P ready, alpha, O ready: 4 warps
+      else if (i >= L::kBarPReady && i < L::kBarODone) count = 4;   // P ready: 4 warps
       else if (i == L::kBarStagger) count = 4;                      // the 4 softmax warps of tile 0, once
       mbar_init(bar(i), count);
     }
@@ -240,7 +247,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     fence_mbar_init();
     __syncwarp();
   }
-  if (warp == 13 && lane == 0) {
+  if (warp == kWarpTma && lane == 0) {
     fence_proxy_async_smem();
     // The first loads start here, before TMEM is allocated and the CTA synchronises: their
     // latency overlaps the rest of the set-up.
@@ -250,7 +257,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     prefetch_tmap(&tm_o);
   }
-  if (warp == 12) {
+  if (warp == kWarpMma0) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), L::kTmemCols);
     tmem_relinquish();
   }
@@ -286,6 +293,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const int vis_row = static_cast<int>(max(0ll, vis_ll));
       float m_cur = -INFINITY;  // running (lazily updated) row maximum, log2 units
       float l_run = 0.f;
+      float sO = 1.f;           // factor of O when the maximum moves
       float sq_t = 0.f, sk_next = 0.f;
       const float* sk_row = nullptr;
       if constexpr (QK8) {
@@ -323,67 +331,95 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               for (int i = 0; i < 32; ++i)
                 if (q * 32 + i >= lim) s[q][i] = __float_as_uint(-INFINITY);
           }
-          // row maximum of the half: four independent chains of 3-input max
-          float mx4[4];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const uint32_t* sp = &s[q >> 1][(q & 1) * 16];
-            float m = fmaxf(__uint_as_float(sp[0]), __uint_as_float(sp[1]));
-#pragma unroll
-            for (int i = 2; i < 16; i += 2) m = fmax3(m, __uint_as_float(sp[i]), __uint_as_float(sp[i + 1]));
-            mx4[q] = m;
-          }
-          // running maximum m_cur is kept in log2 units (raw maximum * cj)
+          // The exponentials do not wait for this half's row maximum: they are taken against the maximum
+          // of the halves before it, while this half's maximum is found on the side (four chains of
+          // 3-input max on the ALU pipe, which the exponentials leave idle).  Only where some row of the
+          // warp outgrew its old maximum by more than 2^8 (rare past the first half) the maximum moves,
+          // O is rescaled here, and the exponentials are taken again: the loop below runs once or twice.
           constexpr float kBias = QK8 ? 12582912.f : 0.f;
-          float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-          if constexpr (QK8) mx -= kBias;
-          mx *= cj;
-          float alpha = 1.f;
-          if (j == 0 && hb == 0) {
-            m_cur = mx;
-          } else {
-            const float m_new = fmaxf(m_cur, mx);
-            if (m_new - m_cur > kLazyThreshold) {  // also taken when m_cur = -inf
-              alpha = ex2(m_cur - m_new);
-              m_cur = m_new;
+          auto row_max = [&](float (&mx4)[4]) {  // in log2 units, like m_cur
+            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            if constexpr (QK8) mx -= kBias;
+            return mx * cj;
+          };
+          const bool first = (j == 0 && hb == 0);
+          if (first) {
+            float mx4[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              mx4[q] = -INFINITY;
+#pragma unroll
+              for (int i = 0; i < 16; i += 2)
+                mx4[q] = fmax3(mx4[q], __uint_as_float(s[q >> 1][(q & 1) * 16 + i]),
+                               __uint_as_float(s[q >> 1][(q & 1) * 16 + i + 1]));
             }
+            m_cur = row_max(mx4);
+            if (t == 0) warp_arrive(bar(L::kBarStagger));
           }
-          alpha_smem[(2 * t + hb) * kTileM + r] = alpha;
-          warp_arrive(bar(L::kBarAlpha + 2 * t + hb));
-          if (t == 0 && j == 0 && hb == 0) warp_arrive(bar(L::kBarStagger));
-
-          // exponent of a score x: x*cj - m; for the int8 variant x carries kBias, taken out here
-          float mc = (m_cur == -INFINITY) ? 0.f : m_cur;
-          if constexpr (QK8) mc = fmaf(kBias, cj, mc);
-          // two scores per FMA / ADD issue slot (packed f32x2); the exp2 itself is one per lane,
-          // except that one pair in eight (one in four at D = 64, where the exp2 unit is the
-          // bound) is evaluated by a polynomial on the FMA pipe: the exp2 unit (16 results per
-          // clock per SM) is co-critical with the tensor pipe, the FMA pipe has room.  Larger
-          // shares measured slower (3/8 and 1/2: the issue slots run out).
-          constexpr int kPolyMask = (D == 64) ? 7 : 15;
-          uint64_t psum = pack_f32x2(0.f, 0.f);
-          const uint64_t cj2 = pack_f32x2(cj, cj), mc2 = pack_f32x2(-mc, -mc);
+          uint64_t psum;
           uint32_t pk[32];
+          for (;;) {
+            // exponent of a score x: x*cj - m; for the int8 variant x carries kBias, taken out here
+            float mc = (m_cur == -INFINITY) ? 0.f : m_cur;
+            if constexpr (QK8) mc = fmaf(kBias, cj, mc);
+            // two scores per FMA / ADD issue slot (packed f32x2); the exp2 itself is one per lane,
+            // except that one pair in eight (one in four at D = 64, where the exp2 unit is the
+            // bound) is evaluated by a polynomial on the FMA pipe: the exp2 unit (16 results per
+            // clock per SM) is co-critical with the tensor pipe, the FMA pipe has room.  None and one in
+            // four at D = 128 measured 435 and 444 us where one in eight takes 428 (N = 8192).
+            constexpr int kPolyMask = (D == 64) ? 7 : 15;
+            psum = pack_f32x2(0.f, 0.f);
+            const uint64_t cj2 = pack_f32x2(cj, cj), mc2 = pack_f32x2(-mc, -mc);
+            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-          for (int q = 0; q < 2; ++q)
+            for (int q = 0; q < 2; ++q)
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
-              float x0, x1;
-              unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])), cj2, mc2),
-                           x0, x1);
-              float p0, p1;
-              if ((i & kPolyMask) == 0) {
-                exp2_poly_f32x2(x0, x1, p0, p1);
-              } else {
-                p0 = ex2(x0);
-                p1 = ex2(x1);
+              for (int i = 0; i < 32; i += 2) {
+                const float s0 = __uint_as_float(s[q][i]), s1 = __uint_as_float(s[q][i + 1]);
+                float x0, x1;
+                unpack_f32x2(fma_f32x2(pack_f32x2(s0, s1), cj2, mc2), x0, x1);
+                mx4[(i >> 1) & 3] = fmax3(mx4[(i >> 1) & 3], s0, s1);
+                float p0, p1;
+                if ((i & kPolyMask) == 0) {
+                  exp2_poly_f32x2(x0, x1, p0, p1);
+                } else {
+                  p0 = ex2(x0);
+                  p1 = ex2(x1);
+                }
+                psum = add_f32x2(psum, pack_f32x2(p0, p1));
+                pk[q * 16 + (i >> 1)] = pack2<BF16>(p0, p1);
               }
-              psum = add_f32x2(psum, pack_f32x2(p0, p1));
-              pk[q * 16 + (i >> 1)] = pack2<BF16>(p0, p1);
+            const float mx = row_max(mx4);
+            const bool moved = mx - m_cur > kLazyThreshold;  // also taken when m_cur = -inf
+            if (!__any_sync(0xffffffffu, moved)) break;
+            if (moved) {
+              const float alpha = ex2(m_cur - mx);
+              l_run *= alpha;
+              m_cur = mx;
+              sO = alpha;
             }
+            if (!first) {
+              // every PV issued so far into O_t must have finished: the previous half-step's
+              if (hb == 0) mbar_wait(bar(L::kBarODone + 2 * t + 1), (j - 1) & 1, wc, kErrWaitO);
+              else mbar_wait(bar(L::kBarODone + 2 * t + 0), j & 1, wc, kErrWaitO);
+              tc_fence_after();
+              const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
+#pragma unroll
+              for (int q = 0; q < D / 32; ++q) {
+                uint32_t o[32];
+                tmem_ld32(tO + q * 32, o);
+                tmem_wait_ld();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * sO);
+                tmem_st32(tO + q * 32, o);
+              }
+              tmem_wait_st();
+            }
+            sO = 1.f;
+          }
           float psum0, psum1;
           unpack_f32x2(psum, psum0, psum1);
-          l_run = l_run * alpha + (psum0 + psum1);
+          l_run += psum0 + psum1;
           tmem_st32(tS + hb * kHalfN, pk);  // P of this half over the first 32 columns of its S
           tmem_wait_st();
           tc_fence_before();
@@ -650,48 +686,14 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
       tc_fence_before();
     }
-  } else if (warp < 12) {
-    // =========================== correction ========================================
-    reg_dec<kRegCorr>();
-    const int r = tid & 127;
-    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    for (int j = 0; j < n_tiles; ++j) {
-#pragma unroll
-      for (int hb = 0; hb < 2; ++hb) {
-        for (int t = 0; t < nt; ++t) {
-          mbar_wait(bar(L::kBarAlpha + 2 * t + hb), j & 1, wc, kErrWaitCorr);
-          const float alpha = alpha_smem[(2 * t + hb) * kTileM + r];
-          if ((j > 0 || hb > 0) && __any_sync(0xffffffffu, alpha != 1.f)) {
-            // every PV issued so far into O_t must have finished: the previous half-step's
-            if (hb == 0) mbar_wait(bar(L::kBarODone + 2 * t + 1), (j - 1) & 1, wc, kErrWaitO);
-            else mbar_wait(bar(L::kBarODone + 2 * t + 0), j & 1, wc, kErrWaitO);
-            tc_fence_after();
-            const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
-#pragma unroll
-            for (int q = 0; q < D / 32; ++q) {
-              uint32_t o[32];
-              tmem_ld32(tO + q * 32, o);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-              tmem_st32(tO + q * 32, o);
-            }
-            tmem_wait_st();
-            tc_fence_before();
-          }
-          warp_arrive(bar(L::kBarOReady + 2 * t + hb));
-        }
-      }
-    }
-    tc_fence_before();
   } else {
     reg_dec<kRegOther>();
-    if (warp == 12 || warp == 14) {
+    if (warp == kWarpMma0 || warp == kWarpMma1) {
       // =========================== MMA issuers =====================================
       // One issuing thread per Q tile (warp 12 -> tile 0, warp 14 -> tile 1).  Each walks its
       // tile's halves in the order the softmax group publishes them: PV_a(j) S_a(j+1) PV_b(j)
       // S_b(j+1).  The tensor pipe interleaves the two streams.
-      const int t = (warp == 12) ? 0 : 1;
+      const int t = (warp == kWarpMma0) ? 0 : 1;
       if (lane == 0 && n_tiles > 0 && t < nt) {
         // kind::f16: D fmt f32, A/B f16 or bf16.  kind::i8: D fmt s32 (2), A/B signed int8 (1).
         constexpr uint32_t idesc_s =
@@ -757,7 +759,6 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const uint32_t kpar = (cons / L::kStages) & 1;
 #pragma unroll
           for (int hb = 0; hb < 2; ++hb) {
-            mbar_wait(bar(L::kBarOReady + 2 * t + hb), j & 1, wc, kErrWaitCorr);
             mbar_wait(bar(L::kBarPReady + 2 * t + hb), j & 1, wc, kErrWaitP);
             tc_fence_after();
             const uint32_t tP = tSt + kHalfN * hb;
@@ -784,7 +785,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
       __syncwarp();
-    } else if (warp == 13) {
+    } else if (warp == kWarpTma) {
       // =========================== TMA producer ====================================
       if (lane == 0 && n_tiles > 0) {
         for (int i = n_early; i < n_fill; ++i) {
@@ -807,7 +808,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == kWarpMma0) {
     tc_fence_after();
     tmem_dealloc(tmem_base, L::kTmemCols);
   }
