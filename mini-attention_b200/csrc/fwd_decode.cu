@@ -98,6 +98,7 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + L::kOffMisc);
   volatile int* order = abort_flag + 1;
 
+  grid_dep_launch();
   const int tid = threadIdx.x, lane = tid & 31;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const WaitCtx wc{abort_flag, a.status, MINIATTN_WAIT_LIMIT_NS};
@@ -113,8 +114,11 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
   }
   __syncthreads();
+  grid_dep_wait();
 
   if (warp == 4) {
     if (lane == 0) {
@@ -477,8 +481,7 @@ static cudaError_t launch_decode_t(const CUtensorMap* tm, const DecodeArgs& a, i
   static std::atomic<unsigned long long> smem_set{0};
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), DecLayout<D>::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
-  kern<<<n_ctas, kDecThreads, DecLayout<D>::kDynSmem, st>>>(tm[0], tm[1], a);
-  return cudaGetLastError();
+  return launch_overlapped(kern, n_ctas, kDecThreads, DecLayout<D>::kDynSmem, st, tm[0], tm[1], a);
 }
 
 template <int D, bool BF16>

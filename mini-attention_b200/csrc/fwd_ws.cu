@@ -151,6 +151,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + L::kOffMisc + 8);
   volatile int* arrival = reinterpret_cast<volatile int*>(gbase + L::kOffMisc + 16);  // [2 tiles]
 
+  grid_dep_launch();
   const int tid = threadIdx.x;
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // warp-uniform for the compiler
   const int lane = tid & 31;
@@ -249,6 +250,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   if (warp == kWarpTma && lane == 0) {
     fence_proxy_async_smem();
+    prefetch_tmap(&tm_q);
+    prefetch_tmap(&tm_k);
+    prefetch_tmap(&tm_v);
+    grid_dep_wait();
     // The first loads start here, before TMEM is allocated and the CTA synchronises: their
     // latency overlaps the rest of the set-up.
     if (n_tiles > 0) {
@@ -276,6 +281,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dep_wait();  // every thread: some read scales and running state, or write results
   const WaitCtx wc{abort_flag, a.status, MINIATTN_WAIT_LIMIT_NS};
   const float c = a.scale_log2;
 
@@ -841,9 +847,8 @@ static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_c
     args.n_pair_items = static_cast<int>(items - rest);
     grid = items + rest;
   }
-  kern<<<static_cast<unsigned>(grid), kNumThreads, L::kDynSmem, st>>>(tm[0], tm[1], tm[2], tm[3],
-                                                                      args, NoPlanTable{0});
-  return cudaGetLastError();
+  return launch_overlapped(kern, static_cast<unsigned>(grid), kNumThreads, L::kDynSmem, st, tm[0], tm[1], tm[2],
+                           tm[3], args, NoPlanTable{0});
 }
 
 template <int D, bool BF16, bool QK8>
@@ -857,8 +862,7 @@ static cudaError_t launch_plan_t(const CUtensorMap* tm, const FwdArgs& a, const 
   FwdArgs args = a;
   args.n_pair_items = plan.n_whole;
   const unsigned grid = static_cast<unsigned>(plan.n_whole + plan.n_table);
-  kern<<<grid, kNumThreads, L::kDynSmem, st>>>(tm[0], tm[1], tm[2], tm[3], args, plan.table);
-  return cudaGetLastError();
+  return launch_overlapped(kern, grid, kNumThreads, L::kDynSmem, st, tm[0], tm[1], tm[2], tm[3], args, plan.table);
 }
 
 // Balanced launch: a.part_o / a.part_ml / a.counters point into the caller's scratch.  qk8: the

@@ -46,6 +46,14 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// ---- programmatic dependent launch ---------------------------------------------
+// The launches below carry the attribute that lets their CTAs start while the kernel before them in
+// the stream drains.  Nothing in global memory may be touched before grid_dep_wait() has returned:
+// it waits until that kernel has finished and its writes are visible.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may start its CTAs on SMs that have room, once every CTA of this one is running.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier ---------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
