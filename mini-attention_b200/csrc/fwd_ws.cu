@@ -25,20 +25,19 @@
 // MMA order per Q tile and K/V tile j:  PV_a(j) S_a(j+1) PV_b(j) S_b(j+1); the two tiles have
 // one issuing thread each and the tensor pipe interleaves their streams.
 //
-// The row maximum is updated lazily: a row keeps exponentiating against a stale maximum until the
-// true maximum has grown by more than 2^8 (in the exp2 domain), so the O accumulator is rescaled
-// only rarely; l is accumulated against the same maximum, which keeps O / l exact.  The exponentials
-// of a half are taken before its maximum is known (it is found in the same instruction stream) and
-// taken again where it turns out to have grown that much.
+// The reference that a row's exponentials are taken against is updated lazily: it stays what it is, and
+// no maximum is searched for, until the sum of a half's exponentials exceeds 2^8; only then the row's
+// maximum is found, O and l are rescaled, and the half is taken again.  l is accumulated against the same
+// reference, which keeps O / l exact.
 //
-// What bounds it (clock stamps, N = 2048, D = 128, per 128-key step of a CTA, about 2980 clk): the MMAs
+// What bounds it (clock stamps, N = 2048, D = 128, per 128-key step of a CTA, about 2950 clk): the MMAs
 // of a step need 2608 clk of the tensor pipe, and they and TMA 2560 clk of the 128 B/clk shared-memory
-// port (Q is re-read for each half); a softmax thread is busy 2380 clk of it and waits 570.  With the
-// maximum found before the exponentials and handed to four correction warps it was 2650 busy of 3140:
-// N = 8192 (2 x 8 heads, fp16) 446 -> 428 us, 4096 GQA causal bf16 524 -> 500, 32768 (16 heads) 3956 ->
-// 3743.  At D = 64 the softmax thread is the bound (2700 clk, 330 of them waiting).  One MMA of 128 keys
-// for S (2080 clk of tensor work) measured slower, 49 against 41 us at N = 2048: TMEM has room for one
-// S buffer per Q tile then, and the thread waits 1600 clk per step for PV and the next S.
+// port (Q is re-read for each half).  Finding the maximum of a half first and handing the factor to four
+// correction warps made it 3140: 3956 us for 16 heads at N = 32768, 3743 with the maximum found beside the
+// exponentials, 3685 without one.  At D = 64 the softmax thread is the bound: N = 8192 (2 x 16 heads) 706 /
+// 694 / 654 us.  One MMA of 128 keys for S (2080 clk of tensor work) measured slower, 49 against 41 us at
+// N = 2048: TMEM has room for one S buffer per Q tile then, and the thread waits 1600 clk per step for PV
+// and the next S.
 //
 // Softmax arithmetic runs two scores per issue slot (packed f32x2 FMA / ADD); a share of the
 // exponentials is evaluated by a cubic on the FMA pipe instead of the exp2 unit.
@@ -61,7 +60,7 @@ namespace {
 constexpr int kNumThreads = 384;
 constexpr int kWarpMma0 = 8, kWarpTma = 9, kWarpMma1 = 10;  // warp 11 only donates its registers
 constexpr int kHalfN = kTileN / 2;      // keys per half tile
-constexpr float kLazyThreshold = 8.0f;  // log2 units
+constexpr float kSumLimit = 256.0f;     // a half's sum of P above which the row's reference moves
 // Register split per thread after setmaxnreg: 8 softmax warps + 4 others.  The launch allocates 168
 // registers for each of the 384 threads (65536 / 384, rounded down to a multiple of 8), and
 // 8*216 + 4*72 = 12*168: what the others release is what the softmax warps take.
@@ -299,7 +298,6 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const int vis_row = static_cast<int>(max(0ll, vis_ll));
       float m_cur = -INFINITY;  // running (lazily updated) row maximum, log2 units
       float l_run = 0.f;
-      float sO = 1.f;           // factor of O when the maximum moves
       float sq_t = 0.f, sk_next = 0.f;
       const float* sk_row = nullptr;
       if constexpr (QK8) {
@@ -309,6 +307,13 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (n_tiles > 0) sk_next = __ldg(sk_row);
       }
 
+      // How much of the loop is unrolled.  A short launch pays for every line of code it fetches once: one
+      // copy of the body for both halves of a tile, and a rescale that is a loop, take 9.55 instead of 9.86 us
+      // at N = 512, 32.4 / 33.1 at N = 2048, 434 / 441 at N = 8192 (cut items), 19.3 / 20.2 for D = 96 N = 1001.
+      // Unrolled, the steady state is the faster one: ring steps (16 heads, 256 tiles an item: 3663 / 3789) and
+      // INT8-QK (642 / 657) keep that.  At D = 64 only the rescale is a loop (18.6 / 19.4 us at N = 1024).
+      constexpr int kHalvesUnrolled = (D == 128 && !CARRY && !QK8) ? 1 : 2;
+      constexpr int kRescaleUnrolled = (CARRY || QK8) ? D / 32 : 1;
       for (int j = 0; j < n_tiles; ++j) {
         // cj turns a raw score into log2 units: softmax scale * log2e, times the two
         // de-quantisation scales of this (Q block, K block) for the int8 variant.
@@ -317,7 +322,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           cj = sq_t * sk_next;
           if (j + 1 < n_tiles) sk_next = __ldg(sk_row + j + 1);
         }
-#pragma unroll
+#pragma unroll (kHalvesUnrolled)
         for (int hb = 0; hb < 2; ++hb) {
           mbar_wait(bar(L::kBarSFull + 2 * t + hb), j & 1, wc, kErrWaitS);
           tc_fence_after();
@@ -337,57 +342,79 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               for (int i = 0; i < 32; ++i)
                 if (q * 32 + i >= lim) s[q][i] = __float_as_uint(-INFINITY);
           }
-          // The exponentials do not wait for this half's row maximum: they are taken against the maximum
-          // of the halves before it, while this half's maximum is found on the side (four chains of
-          // 3-input max on the ALU pipe, which the exponentials leave idle).  Only where some row of the
-          // warp outgrew its old maximum by more than 2^8 (rare past the first half) the maximum moves,
-          // O is rescaled here, and the exponentials are taken again: the loop below runs once or twice.
+          // No row maximum is searched for in the usual half: the exponentials are taken against the
+          // reference m_cur the row already has, and their sum, which is wanted anyway, says whether it
+          // still serves.  A sum of at most 2^8 bounds every term by 2^8, the headroom the lazy update
+          // always allowed.  Where some row of the warp has none yet (its first visible keys) or its sum
+          // came out larger, the maxima are found, O is rescaled here, and the exponentials are taken
+          // (again): at most twice per half, and rare past the first.
           constexpr float kBias = QK8 ? 12582912.f : 0.f;
-          auto row_max = [&](float (&mx4)[4]) {  // in log2 units, like m_cur
-            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-            if constexpr (QK8) mx -= kBias;
-            return mx * cj;
-          };
           const bool first = (j == 0 && hb == 0);
-          if (first) {
-            float mx4[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              mx4[q] = -INFINITY;
-#pragma unroll
-              for (int i = 0; i < 16; i += 2)
-                mx4[q] = fmax3(mx4[q], __uint_as_float(s[q >> 1][(q & 1) * 16 + i]),
-                               __uint_as_float(s[q >> 1][(q & 1) * 16 + i + 1]));
-            }
-            m_cur = row_max(mx4);
-            if (t == 0) warp_arrive(bar(L::kBarStagger));
-          }
-          uint64_t psum;
+          float psum0, psum1;
           uint32_t pk[32];
-          for (;;) {
+          bool fix = first;
+          for (int pass = 0;; ++pass) {
+            if (fix) {
+              float mx4[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                mx4[q] = -INFINITY;
+#pragma unroll
+                for (int i = 0; i < 16; i += 2)
+                  mx4[q] = fmax3(mx4[q], __uint_as_float(s[q >> 1][(q & 1) * 16 + i]),
+                                 __uint_as_float(s[q >> 1][(q & 1) * 16 + i + 1]));
+              }
+              float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+              if constexpr (QK8) mx -= kBias;
+              mx *= cj;  // log2 units, like m_cur
+              float alpha = 1.f;
+              if (mx > m_cur) {
+                alpha = ex2(m_cur - mx);
+                m_cur = mx;
+              }
+              if (!first && __any_sync(0xffffffffu, alpha != 1.f)) {
+                l_run *= alpha;
+                // every PV issued so far into O_t must have finished: the previous half-step's
+                if (hb == 0) mbar_wait(bar(L::kBarODone + 2 * t + 1), (j - 1) & 1, wc, kErrWaitO);
+                else mbar_wait(bar(L::kBarODone + 2 * t + 0), j & 1, wc, kErrWaitO);
+                tc_fence_after();
+                const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
+#pragma unroll (kRescaleUnrolled)
+                for (int q = 0; q < D / 32; ++q) {
+                  uint32_t o[32];
+                  tmem_ld32(tO + q * 32, o);
+                  tmem_wait_ld();
+#pragma unroll
+                  for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                  tmem_st32(tO + q * 32, o);
+                }
+                tmem_wait_st();
+              }
+              if (t == 0 && first) warp_arrive(bar(L::kBarStagger));
+            }
             // exponent of a score x: x*cj - m; for the int8 variant x carries kBias, taken out here
             float mc = (m_cur == -INFINITY) ? 0.f : m_cur;
             if constexpr (QK8) mc = fmaf(kBias, cj, mc);
             // two scores per FMA / ADD issue slot (packed f32x2); the exp2 itself is one per lane,
-            // except that one pair in eight (one in four at D = 64, where the exp2 unit is the
-            // bound) is evaluated by a polynomial on the FMA pipe: the exp2 unit (16 results per
-            // clock per SM) is co-critical with the tensor pipe, the FMA pipe has room.  None and one in
-            // four at D = 128 measured 435 and 444 us where one in eight takes 428 (N = 8192).
-            constexpr int kPolyMask = (D == 64) ? 7 : 15;
-            psum = pack_f32x2(0.f, 0.f);
+            // except that some pairs are evaluated by a polynomial on the FMA pipe: the exp2 unit
+            // (16 results per clock per SM) is co-critical with the tensor pipe, the FMA pipe has room.
+            // D = 64: one pair in four, by the cubic (shares of 0, 3/16, 1/4, 3/8: 754, 697, 654, 678 us,
+            // 2 x 16 heads, N = 8192).  D = 128: three pairs in sixteen, by the quartic (1/8, 3/16, 1/4:
+            // 3945, 3685, 3760 us, 16 heads, N = 32768; 62.8, 61.6, 62.0 us, 16 causal heads, N = 4096),
+            // whose error is below that of a cubic on one pair in eight.
+            auto on_fma_pipe = [](int i) { return D == 64 ? (i & 7) == 0 : (i == 0 || i == 10 || i == 20); };
+            uint64_t psum = pack_f32x2(0.f, 0.f);
             const uint64_t cj2 = pack_f32x2(cj, cj), mc2 = pack_f32x2(-mc, -mc);
-            float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
             for (int q = 0; q < 2; ++q)
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
-                const float s0 = __uint_as_float(s[q][i]), s1 = __uint_as_float(s[q][i + 1]);
                 float x0, x1;
-                unpack_f32x2(fma_f32x2(pack_f32x2(s0, s1), cj2, mc2), x0, x1);
-                mx4[(i >> 1) & 3] = fmax3(mx4[(i >> 1) & 3], s0, s1);
+                unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(s[q][i]), __uint_as_float(s[q][i + 1])), cj2, mc2),
+                             x0, x1);
                 float p0, p1;
-                if ((i & kPolyMask) == 0) {
-                  exp2_poly_f32x2(x0, x1, p0, p1);
+                if (on_fma_pipe(i)) {
+                  exp2_poly_f32x2<D != 64>(x0, x1, p0, p1);
                 } else {
                   p0 = ex2(x0);
                   p1 = ex2(x1);
@@ -395,36 +422,11 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 psum = add_f32x2(psum, pack_f32x2(p0, p1));
                 pk[q * 16 + (i >> 1)] = pack2<BF16>(p0, p1);
               }
-            const float mx = row_max(mx4);
-            const bool moved = mx - m_cur > kLazyThreshold;  // also taken when m_cur = -inf
-            if (!__any_sync(0xffffffffu, moved)) break;
-            if (moved) {
-              const float alpha = ex2(m_cur - mx);
-              l_run *= alpha;
-              m_cur = mx;
-              sO = alpha;
-            }
-            if (!first) {
-              // every PV issued so far into O_t must have finished: the previous half-step's
-              if (hb == 0) mbar_wait(bar(L::kBarODone + 2 * t + 1), (j - 1) & 1, wc, kErrWaitO);
-              else mbar_wait(bar(L::kBarODone + 2 * t + 0), j & 1, wc, kErrWaitO);
-              tc_fence_after();
-              const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
-#pragma unroll
-              for (int q = 0; q < D / 32; ++q) {
-                uint32_t o[32];
-                tmem_ld32(tO + q * 32, o);
-                tmem_wait_ld();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * sO);
-                tmem_st32(tO + q * 32, o);
-              }
-              tmem_wait_st();
-            }
-            sO = 1.f;
+            unpack_f32x2(psum, psum0, psum1);
+            // a sum that is not a number stays one, a row without visible keys stays without: no third pass
+            if (pass == 1 || !__any_sync(0xffffffffu, !(psum0 + psum1 <= kSumLimit) || m_cur == -INFINITY)) break;
+            fix = true;
           }
-          float psum0, psum1;
-          unpack_f32x2(psum, psum0, psum1);
           l_run += psum0 + psum1;
           tmem_st32(tS + hb * kHalfN, pk);  // P of this half over the first 32 columns of its S
           tmem_wait_st();

@@ -329,17 +329,28 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   return r;
 }
 // 2^x for a pair on the FMA pipe instead of the exp2 unit: x = n + f with n = round(x) taken from
-// the low mantissa bits of x + 1.5*2^23 and f in [-0.5, 0.5]; 2^f by a cubic (max relative error
-// 1.0e-4, below the half-ulp of a 16-bit P), n added into the exponent field.  Inputs below -126
+// the low mantissa bits of x + 1.5*2^23 and f in [-0.5, 0.5]; 2^f by the cubic
+// whose relative error has the least mean square over that range (rms 4.6e-5, mean 0, at most 1.4e-4: below
+// the half-ulp of a 16-bit P, and no bias in a row's sum), n added into the exponent field.  Inputs below -126
 // (masked scores are -inf) give 2^-126, which rounds to 0 in 16 bit.
+// FINE: the quartic with the least maximum relative error (2.6e-6), one FMA more.
+template <bool FINE>
 __device__ __forceinline__ void exp2_poly_f32x2(float x0, float x1, float& p0, float& p1) {
   const uint64_t x = pack_f32x2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
   const uint64_t xr = add_f32x2(x, pack_f32x2(12582912.f, 12582912.f));
   const uint64_t n = add_f32x2(xr, pack_f32x2(-12582912.f, -12582912.f));
   const uint64_t f = fma_f32x2(n, pack_f32x2(-1.f, -1.f), x);
-  uint64_t p = fma_f32x2(f, pack_f32x2(0.05592204f, 0.05592204f), pack_f32x2(0.24264008f, 0.24264008f));
-  p = fma_f32x2(p, f, pack_f32x2(0.69312103f, 0.69312103f));
-  p = fma_f32x2(p, f, pack_f32x2(0.99992448f, 0.99992448f));
+  uint64_t p;
+  if constexpr (FINE) {
+    p = fma_f32x2(f, pack_f32x2(0.00957010221f, 0.00957010221f), pack_f32x2(0.0559178591f, 0.0559178591f));
+    p = fma_f32x2(p, f, pack_f32x2(0.240247443f, 0.240247443f));
+    p = fma_f32x2(p, f, pack_f32x2(0.693121791f, 0.693121791f));
+    p = fma_f32x2(p, f, pack_f32x2(0.999999285f, 0.999999285f));
+  } else {
+    p = fma_f32x2(f, pack_f32x2(0.0550293114f, 0.0550293114f), pack_f32x2(0.242256792f, 0.242256792f));
+    p = fma_f32x2(p, f, pack_f32x2(0.693253035f, 0.693253035f));
+    p = fma_f32x2(p, f, pack_f32x2(0.999951348f, 0.999951348f));
+  }
   float r0, r1, q0, q1;
   unpack_f32x2(xr, r0, r1);
   unpack_f32x2(p, q0, q1);
