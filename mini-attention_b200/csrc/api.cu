@@ -134,6 +134,39 @@ int make_map(CUtensorMap* out, const void* base, int elem_bytes, CUtensorMapData
   return MINIATTN_OK;
 }
 
+// Q or O for fwd_ws.cu: dims (fastest first) = (d, head of a group of `pack`, token, group, batch);
+// box = 64 x pack x tpt x 1 x 1, so that a tile's rows are (token, head) with the head fastest.
+int make_map_packed(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int D, int N, int groups, int B,
+                    const int64_t stride[3], int pack, int tpt, const char* what) {
+  thread_local MapSlot cache[kMapSlots] = {};
+  thread_local unsigned next_slot = 0;
+  const MapKey key{base, {stride[0], stride[1], stride[2]}, pack, static_cast<int>(dt), D, N, groups, B, tpt, 0, 0};
+  for (int i = 0; i < kMapSlots; ++i)
+    if (cache[i].valid && cache[i].key == key) {
+      *out = cache[i].map;
+      return MINIATTN_OK;
+    }
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return fail(MINIATTN_ECUDA, "cuTensorMapEncodeTiled entry point not found");
+  cuuint64_t dims[5] = {(cuuint64_t)D, (cuuint64_t)pack, (cuuint64_t)N, (cuuint64_t)groups, (cuuint64_t)B};
+  cuuint64_t strides[4] = {(cuuint64_t)stride[1] * 2, (cuuint64_t)stride[2] * 2, (cuuint64_t)stride[1] * pack * 2,
+                           (cuuint64_t)stride[0] * 2};
+  cuuint32_t box[5] = {ma::kBoxCols, (cuuint32_t)pack, (cuuint32_t)tpt, 1, 1};
+  cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  // a size-1 dim may carry any stride; give the encoder a legal one
+  for (int i = 0; i < 4; ++i)
+    if (dims[i + 1] == 1) strides[i] = (cuuint64_t)D * 2;
+  CUresult r = enc(out, dt, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return fail(MINIATTN_ECUDA, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r);
+  MapSlot& slot = cache[next_slot++ % kMapSlots];
+  slot.key = key;
+  slot.map = *out;
+  slot.valid = true;
+  return MINIATTN_OK;
+}
+
 int check_tensor(const void* p, const int64_t s[3], int D, const char* name) {
   if (p == nullptr) return fail(MINIATTN_EINVAL, "%s is null", name);
   if (reinterpret_cast<uintptr_t>(p) % 16 != 0)
@@ -243,10 +276,10 @@ static int check_fwd_params(const MiniAttnFwdParams* p) {
 #define MINIATTN_GROUP_TOTAL_MB 48
 #define MINIATTN_GROUP_SHARE_MB 40
 #endif
-static int head_group(const MiniAttnFwdParams* p) {
-  const long long bh_total = static_cast<long long>(p->B) * p->Hq;
+static int head_group(const MiniAttnFwdParams* p, int pack) {
+  const long long bh_total = static_cast<long long>(p->B) * (p->Hq / pack);
   if (p->Hkv <= 0 || p->Hq % p->Hkv != 0) return static_cast<int>(bh_total > 0 ? bh_total : 1);
-  const long long g = p->Hq / p->Hkv;                               // query heads per KV head
+  const long long g = p->Hq / p->Hkv / pack;                        // work-item heads per KV head
   const long long kv_heads = static_cast<long long>(p->B) * p->Hkv;
   const long long per_kv = 2ll * p->Nk * kernel_head_dim(p->D) * 2; // K and V bytes of one KV head
   if (per_kv * kv_heads < (static_cast<long long>(MINIATTN_GROUP_TOTAL_MB) << 20)) return static_cast<int>(bh_total);
@@ -258,22 +291,58 @@ static int head_group(const MiniAttnFwdParams* p) {
   return static_cast<int>(d * g);
 }
 
-static void fill_args(const MiniAttnFwdParams* p, ma::FwdArgs* a) {
+// Query heads that share a Q tile: all G heads of a KV head, or 1.  Packed, a tile holds 128 / G tokens of
+// each head: the tail of a token count that is no multiple of 128 is padded once per KV head instead of once
+// per query head, and under a causal mask a pair of tiles spans 256 / G tokens, so that its rows share more
+// of their last K/V tiles (N = 1024, G = 4: 4.5 instead of 5 tiles per pair on average).  Taken where that
+// saves at least 1 % of the K/V tiles to visit; where G does not divide 128 some rows are lost to padding.
+// Measured (one head per tile / packed, causal bf16, D = 128): 777 against 3333 keys, 2 x 24/8 heads 69.0 /
+// 62.5 us; N = 4096, 4 x 32/8 heads 500 / 488, 1 x 16/4 heads 58.3 / 56.5; N = 1024, 2 x 16/4 heads 19.1 / 19.1
+// (one wave, as long as its longest item).  With nothing to save the packed kernel is 0.3 us slower (two more
+// divisions and 5-D copies), so it is not taken then.
+static int head_pack(const MiniAttnFwdParams* p) {
+  const int g = p->Hkv > 0 ? p->Hq / p->Hkv : 1;
+  if (g < 2 || g > ma::kTileM || p->Hq % g != 0 || p->Hq / g != p->Hkv || p->Nq <= 0 || p->Nk <= 0) return 1;
+  if (p->kernel == MINIATTN_KERNEL_SIMPLE || p->carry_in || p->carry_out) return 1;
+  long long visits[2];
+  for (int packed = 0; packed < 2; ++packed) {
+    ma::FwdArgs a{};
+    a.Nq = p->Nq;
+    a.Nk = p->Nk;
+    a.causal = p->causal;
+    a.q_pos0 = p->q_pos0;
+    a.k_pos0 = p->k_pos0;
+    a.tpt = ma::kTileM / (packed ? g : 1);
+    const int n_tiles = (p->Nq + a.tpt - 1) / a.tpt;
+    visits[packed] = 0;
+    for (int t = 0; t < n_tiles; t += 2) {
+      const int nt = t + 1 < n_tiles ? 2 : 1;
+      // a step of a tile alone takes two thirds of a pair's (2000 and 2950 clk)
+      visits[packed] += (nt == 2 ? 3 : 2) * static_cast<long long>(ma::kv_tiles_of(a, t * a.tpt, nt));
+    }
+    if (!packed) visits[0] *= g;
+  }
+  return visits[1] * 100 <= visits[0] * 99 ? g : 1;
+}
+
+static void fill_args(const MiniAttnFwdParams* p, ma::FwdArgs* a, int pack) {
   a->lse = p->lse;
   a->status = p->status;
   a->q_pos0 = p->q_pos0;
   a->k_pos0 = p->k_pos0;
   a->Nq = p->Nq;
   a->Nk = p->Nk;
-  a->Hq = p->Hq;
+  a->Hq = p->Hq / pack;
   a->Hkv = p->Hkv;
   a->B = p->B;
   a->causal = p->causal;
   a->scale = p->softmax_scale > 0.f ? p->softmax_scale : 1.0f / sqrtf((float)p->D);
   a->scale_log2 = a->scale * 1.4426950408889634f;
-  a->n_q_tiles = (p->Nq + ma::kTileM - 1) / ma::kTileM;
+  a->pack = pack;
+  a->tpt = ma::kTileM / pack;
+  a->n_q_tiles = (p->Nq + a->tpt - 1) / a->tpt;
   a->n_pair_items = 0;  // set by the warp-specialised launcher
-  a->bh_group = head_group(p);
+  a->bh_group = head_group(p, pack);
   a->sq = nullptr;
   a->sk = nullptr;
   a->part_o = nullptr;
@@ -300,11 +369,11 @@ static int check_device(int* sms) {
 // repeat).  Guarded by a mutex; an entry is copied out under the lock.
 namespace {
 struct PlanKey {
-  int Nq, Nk, B, Hq, causal, D, sms, group;
+  int Nq, Nk, B, Hq, causal, D, sms, group, pack;
   long long diag;
   bool operator==(const PlanKey& o) const {
     return Nq == o.Nq && Nk == o.Nk && B == o.B && Hq == o.Hq && causal == o.causal && D == o.D &&
-           sms == o.sms && group == o.group && diag == o.diag;
+           sms == o.sms && group == o.group && pack == o.pack && diag == o.diag;
   }
 };
 struct PlanSlot {
@@ -315,7 +384,7 @@ std::shared_ptr<const ma::FwdPlan> cached_plan(const ma::FwdArgs& a, int D, int 
   static std::mutex mu;
   static std::vector<PlanSlot> cache;
   static size_t next = 0;
-  const PlanKey key{a.Nq, a.Nk, a.B, a.Hq, a.causal, D, sms, a.bh_group, a.causal ? a.q_pos0 - a.k_pos0 : 0};
+  const PlanKey key{a.Nq, a.Nk, a.B, a.Hq, a.causal, D, sms, a.bh_group, a.pack, a.causal ? a.q_pos0 - a.k_pos0 : 0};
   {
     std::lock_guard<std::mutex> g(mu);
     for (const PlanSlot& s : cache)
@@ -435,9 +504,14 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   const CUtensorMapDataType dt =
       p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tm[4];
-  if ((rc = make_map(&tm[0], p->q, 2, dt, p->D, p->Nq, p->Hq, p->B, p->q_stride, ma::kBoxCols,
-                     ma::kTileM, "q")) != 0)
-    return rc;
+  const bool simple = p->kernel == MINIATTN_KERNEL_SIMPLE;
+  ma::FwdArgs a;
+  fill_args(p, &a, head_pack(p));
+  auto q_map = [&](CUtensorMap* out, const void* base, const int64_t stride[3], const char* what) {
+    return a.pack == 1 ? make_map(out, base, 2, dt, p->D, p->Nq, p->Hq, p->B, stride, ma::kBoxCols, ma::kTileM, what)
+                       : make_map_packed(out, base, dt, p->D, p->Nq, a.Hq, p->B, stride, a.pack, a.tpt, what);
+  };
+  if ((rc = q_map(&tm[0], p->q, p->q_stride, "q")) != 0) return rc;
   if (has_keys) {
     if ((rc = make_map(&tm[1], p->k, 2, dt, p->D, p->Nk, p->Hkv, p->B, p->k_stride, ma::kBoxCols,
                        ma::kTileN, "k")) != 0)
@@ -451,13 +525,10 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   }
   if (p->o == nullptr) {
     tm[3] = tm[0];  // state-only call: the kernel never stores through the output map
-  } else if ((rc = make_map(&tm[3], p->o, 2, dt, p->D, p->Nq, p->Hq, p->B, p->o_stride, ma::kBoxCols,
-                            ma::kTileM, "o")) != 0) {
+  } else if ((rc = q_map(&tm[3], p->o, p->o_stride, "o")) != 0) {
     return rc;
   }
 
-  ma::FwdArgs a;
-  fill_args(p, &a);
   const int kd = kernel_head_dim(p->D);
   const bool carry = p->carry_in || p->carry_out;
   if (carry) {
@@ -470,10 +541,8 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   }
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int kernel = p->kernel;
-  if (kernel == MINIATTN_KERNEL_AUTO) kernel = MINIATTN_KERNEL_WS;
   cudaError_t e;
-  if (kernel == MINIATTN_KERNEL_SIMPLE) {
+  if (simple) {
     e = ma::launch_fwd_simple(kd, p->dtype == MINIATTN_BF16, tm, a, st);
   } else {
     // a call that carries ring state always takes the plain launch
@@ -502,8 +571,8 @@ int miniattn_fwd_balanced(const MiniAttnFwdParams* p, void* scratch, size_t scra
 }
 
 // Plan of a forward launch for `sm_count` SMs (<= 0: the current device's).  Host arithmetic only.
-int miniattn_plan_fwd(const MiniAttnFwdParams* p, int sm_count, MiniAttnPlanInfo* info,
-                      MiniAttnPlanPiece* pieces, int32_t cap) {
+static int plan_info_of(const MiniAttnFwdParams* p, bool may_pack, int sm_count, MiniAttnPlanInfo* info,
+                        MiniAttnPlanPiece* pieces, int32_t cap) {
   g_err[0] = 0;
   if (info == nullptr) return fail(MINIATTN_EINVAL, "info is null");
   memset(info, 0, sizeof(*info));
@@ -519,8 +588,8 @@ int miniattn_plan_fwd(const MiniAttnFwdParams* p, int sm_count, MiniAttnPlanInfo
     if ((rc = check_device(&sms)) != 0) return rc;
   }
   ma::FwdArgs a;
-  fill_args(p, &a);
-  const long long n_items = static_cast<long long>((a.n_q_tiles + 1) / 2) * p->Hq * p->B;
+  fill_args(p, &a, may_pack ? head_pack(p) : 1);
+  const long long n_items = static_cast<long long>((a.n_q_tiles + 1) / 2) * a.Hq * p->B;
   info->sm_count = sms;
   info->n_ctas = n_items;
   info->head_group = a.bh_group;
@@ -552,6 +621,11 @@ int miniattn_plan_fwd(const MiniAttnFwdParams* p, int sm_count, MiniAttnPlanInfo
   return MINIATTN_OK;
 }
 
+int miniattn_plan_fwd(const MiniAttnFwdParams* p, int sm_count, MiniAttnPlanInfo* info,
+                      MiniAttnPlanPiece* pieces, int32_t cap) {
+  return plan_info_of(p, true, sm_count, info, pieces, cap);
+}
+
 int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p) {
   g_err[0] = 0;
   if (p == nullptr) return fail(MINIATTN_EINVAL, "params is null");
@@ -563,13 +637,15 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p) {
 }
 
 int64_t miniattn_fwd_balanced_scratch_bytes(const MiniAttnFwdParams* p) {
-  MiniAttnPlanInfo info;
-  const int rc = miniattn_plan_fwd(p, 0, &info, nullptr, 0);
+  MiniAttnPlanInfo info, unpacked;
+  int rc = miniattn_plan_fwd(p, 0, &info, nullptr, 0);
   if (rc != 0) return rc;
-  // the larger of the two launches' needs: the INT8-QK entry sizes its scratch with the same call
+  // the largest need of the launches that size their scratch with this call: the general kernel, the
+  // INT8-QK one (which does not pack heads), and the one for few rows
+  if ((rc = plan_info_of(p, false, info.sm_count, &unpacked, nullptr, 0)) != 0) return rc;
   ma::DecodePlan dec;
   decode_plan_of(p, info.sm_count, true, &dec);
-  return std::max<int64_t>(info.scratch_bytes, static_cast<int64_t>(decode_scratch_bytes(dec, p->D)));
+  return std::max({info.scratch_bytes, unpacked.scratch_bytes, static_cast<int64_t>(decode_scratch_bytes(dec, p->D))});
 }
 
 static int check_int8_params(const MiniAttnInt8Params* p, bool need_v) {
@@ -668,7 +744,7 @@ static int int8_common(const MiniAttnInt8Params* p, void* scratch, size_t scratc
                      "o")) != 0)
     return rc;
   ma::FwdArgs a;
-  fill_args(&f, &a);
+  fill_args(&f, &a, 1);
   a.sq = p->q_scale;
   a.sk = p->k_scale;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);

@@ -15,7 +15,10 @@ struct FwdArgs {
   int causal;
   float scale;         // softmax scale
   float scale_log2;    // softmax scale * log2(e)
-  int n_q_tiles;       // ceil(Nq / 128)
+  int pack;            // query heads that share a Q tile: row r of a tile is token r / pack, head r % pack
+                       // of the group.  Hq counts such groups (1: plain heads).  See head_pack, api.cu
+  int tpt;             // query tokens per Q tile: 128 / pack, rounded down
+  int n_q_tiles;       // ceil(Nq / tpt)
   int n_pair_items;    // warp-specialised kernel: CTAs [0, n_pair_items) take two Q tiles each,
                        // the CTAs after them one Q tile each (the tail of the last wave)
   int bh_group;        // work items are ordered in groups of this many consecutive (batch, head)
@@ -101,12 +104,12 @@ __host__ __device__ inline void item_to_pair_bh(const FwdArgs& a, int n_pairs, i
   *bh = (item / per_group) * a.bh_group + within % a.bh_group;
 }
 
-// Number of K/V tiles the Q rows [q0, q0 + nt*128) have to visit (all of them without a mask,
+// Number of K/V tiles the Q tiles whose first token is q0 have to visit (all of them without a mask,
 // up to the diagonal of the last row with one).  Shared by the kernels and the host planner.
 __host__ __device__ inline int kv_tiles_of(const FwdArgs& a, int q0, int nt) {
   long long kv_end = a.Nk;
   if (a.causal) {
-    long long last_row = q0 + nt * kTileM - 1;
+    long long last_row = q0 + nt * a.tpt - 1;
     if (last_row > a.Nq - 1) last_row = a.Nq - 1;
     long long vis = a.q_pos0 + last_row - a.k_pos0 + 1;
     if (vis < kv_end) kv_end = vis;

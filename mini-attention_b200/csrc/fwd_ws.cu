@@ -58,7 +58,7 @@ namespace ma {
 namespace {
 
 constexpr int kNumThreads = 384;
-constexpr int kWarpMma0 = 8, kWarpTma = 9, kWarpMma1 = 10;  // warp 11 only donates its registers
+constexpr int kWarpMma0 = 8, kWarpTma = 9, kWarpMma1 = 10, kWarpIdle = 11;
 constexpr int kHalfN = kTileN / 2;      // keys per half tile
 constexpr float kSumLimit = 256.0f;     // a half's sum of P above which the row's reference moves
 // Register split per thread after setmaxnreg: 8 softmax warps + 4 others.  The launch allocates 168
@@ -130,7 +130,10 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar) {
 // -- un-normalised O (fp32, the layout of a balanced launch's partial) and (row maximum, row sum)
 // -- lives in global memory between launches.  With a.carry_mode bit 0 the epilogue folds that state
 // into this launch's result; with bit 1 it writes the new state instead of the 16-bit output.
-template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false>
+//
+// PACK: the a.pack query heads that share a KV head share Q tiles too, a.tpt tokens of each: row r of a tile
+// is token r / a.pack, head r % a.pack of the group (head_pack in api.cu says when).
+template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false, bool PACK = false>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -159,7 +162,6 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // CTAs past n_pair_items take a single Q tile: the launcher cuts the pairs that would form a
   // less-than-half-full last wave into two CTAs each, so that the wave ends sooner.
   const int n_pairs = (a.n_q_tiles + 1) >> 1;
-  const int bh_total = a.Hq * a.B;
   int item = blockIdx.x;
   int single = -1;  // which tile of its pair a single-tile CTA takes
   int pe_t0 = 0, pe_t1 = -1, pe_part = 0, pe_nparts = 1, pe_slot0 = 0, pe_counter = 0;
@@ -179,19 +181,20 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       single = s_idx & 1;
     }
   }
+  const int tpt = PACK ? a.tpt : kTileM;  // query tokens per Q tile
   int pair, bh;
   item_to_pair_bh(a, n_pairs, item, &pair, &bh);
   const int h = bh % a.Hq;
   const int b = bh / a.Hq;
   const int hk = h / (a.Hq / a.Hkv);
-  const int q0 = (pair * 2 + (single > 0 ? 1 : 0)) * kTileM;
+  const int q0 = (pair * 2 + (single > 0 ? 1 : 0)) * tpt;  // first query token
   // Q tiles of this CTA that hold real rows
-  const int nt = (single < 0 && q0 + kTileM < a.Nq) ? 2 : 1;
+  const int nt = (single < 0 && q0 + tpt < a.Nq) ? 2 : 1;
 
   // K/V tiles [kv_t0, kv_t0 + n_tiles) of this CTA: all the rows can see, or the table's range
   int kv_end = a.Nk;
   if (a.causal) {
-    const int last_row = min(q0 + nt * kTileM - 1, a.Nq - 1);
+    const int last_row = min(q0 + nt * tpt - 1, a.Nq - 1);
     const long long vis = a.q_pos0 + last_row - a.k_pos0 + 1;
     kv_end = static_cast<int>(max(0ll, min(static_cast<long long>(a.Nk), vis)));
   }
@@ -208,6 +211,13 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     if constexpr (QK8) {  // one box of D bytes x 128 rows
       mbar_expect_tx(bar(L::kBarQFull + t), kTileM * D);
       tma_load_4d(sQ + t * L::kTileBytes, &tm_q, bar(L::kBarQFull + t), 0, q0 + t * kTileM, h, b);
+    } else if constexpr (PACK) {
+      // a box holds tpt tokens of pack heads, heads fastest: rows [0, pack * tpt) of the tile
+      mbar_expect_tx(bar(L::kBarQFull + t), L::kBoxes * a.pack * tpt * 128);
+#pragma unroll
+      for (int bx = 0; bx < L::kBoxes; ++bx)
+        tma_load_5d(sQ + t * L::kTileBytes + bx * kBoxBytes, &tm_q, bar(L::kBarQFull + t),
+                    bx * kBoxCols, 0, q0 + t * tpt, h, b);
     } else {
       mbar_expect_tx(bar(L::kBarQFull + t), L::kTileBytes);
 #pragma unroll
@@ -276,6 +286,19 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     fence_proxy_async_smem();
   }
+  if constexpr (PACK) {
+    // pack does not divide 128: the last rows of the Q tiles (at most pack - 1) belong to nobody; zeros
+    // keep their scores finite
+    const int pad = kTileM - a.pack * tpt;
+    if (warp == kWarpIdle && pad > 0) {
+      for (int i = lane; i < 2 * L::kBoxes * pad * 8; i += 32) {
+        const int box = i / (pad * 8), at = i % (pad * 8);
+        *reinterpret_cast<uint4*>(gbase + L::kOffQ + box * kBoxBytes + (kTileM - pad) * 128 + at * 16) =
+            make_uint4(0u, 0u, 0u, 0u);
+      }
+      fence_proxy_async_smem();
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -290,7 +313,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int t = warp >> 2;
     if (t < nt) {
       const int r = tid & 127;
-      const int row = q0 + t * kTileM + r;
+      const int row = q0 + t * tpt + (PACK ? r / a.pack : r);  // query token of this thread
       const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
       const uint32_t tS = tmem_base + L::kColS + 128 * t + lane_off;
       long long vis_ll = a.Nk;
@@ -437,7 +460,12 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
       if ((!PLAN || pe_nparts == 1) && !(CARRY && a.carry_mode != 0) && a.lse != nullptr && row < a.Nq) {
         const float lse = (l_run > 0.f) ? (m_cur * 0.6931471805599453f + __logf(l_run)) : -INFINITY;
-        a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Nq + row] = lse;
+        if constexpr (PACK) {
+          if (r < a.pack * tpt)
+            a.lse[((static_cast<long long>(b) * a.Hq + h) * a.pack + r % a.pack) * a.Nq + row] = lse;
+        } else {
+          a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Nq + row] = lse;
+        }
       }
       const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
       if (n_tiles > 0) {
@@ -526,9 +554,11 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             }
             const float mt = (m_tot == -INFINITY) ? 0.f : m_tot;
             const float inv_l = (l_tot > 0.f) ? (1.f / l_tot) : 0.f;
-            if (a.lse != nullptr && row < a.Nq)
-              a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Nq + row] =
-                  (l_tot > 0.f) ? (m_tot * 0.6931471805599453f + __logf(l_tot)) : -INFINITY;
+            if (a.lse != nullptr && row < a.Nq && (!PACK || r < a.pack * tpt)) {
+              const long long head = PACK ? (static_cast<long long>(b) * a.Hq + h) * a.pack + r % a.pack
+                                          : static_cast<long long>(b) * a.Hq + h;
+              a.lse[head * a.Nq + row] = (l_tot > 0.f) ? (m_tot * 0.6931471805599453f + __logf(l_tot)) : -INFINITY;
+            }
             s_part = reinterpret_cast<const float4*>(gbase + ring_off) + r;
             uint32_t phase = 1;  // the Q barrier of this tile completed its phase 0 with the Q load
             bool own_scaled = false;
@@ -687,7 +717,8 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (r == 0) {
 #pragma unroll
           for (int bx = 0; bx < L::kBoxes; ++bx)
-            tma_store_4d(&tm_o, stage + bx * kBoxBytes, bx * kBoxCols, q0 + t * kTileM, h, b);
+            if constexpr (PACK) tma_store_5d(&tm_o, stage + bx * kBoxBytes, bx * kBoxCols, 0, q0 + t * tpt, h, b);
+            else tma_store_4d(&tm_o, stage + bx * kBoxBytes, bx * kBoxCols, q0 + t * kTileM, h, b);
           tma_store_commit();
           tma_store_wait_read0();  // the staging buffer must outlive the copy's reads, no more
         }
@@ -823,10 +854,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------------
-template <int D, bool BF16, bool QK8, bool CARRY = false>
+template <int D, bool BF16, bool QK8, bool CARRY = false, bool PACK = false>
 static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_count, cudaStream_t st) {
   using L = WsLayout<D, QK8>;
-  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY>;
+  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY, PACK>;
   static std::atomic<unsigned long long> smem_set{0};  // per instantiation: devices already configured
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
@@ -853,11 +884,11 @@ static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_c
                            tm[3], args, NoPlanTable{0});
 }
 
-template <int D, bool BF16, bool QK8>
+template <int D, bool BF16, bool QK8, bool PACK = false>
 static cudaError_t launch_plan_t(const CUtensorMap* tm, const FwdArgs& a, const FwdPlan& plan,
                                  cudaStream_t st) {
   using L = WsLayout<D, QK8>;
-  auto kern = fwd_ws_kernel<D, BF16, QK8, true>;
+  auto kern = fwd_ws_kernel<D, BF16, QK8, true, false, PACK>;
   static std::atomic<unsigned long long> smem_set{0};
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
@@ -867,36 +898,33 @@ static cudaError_t launch_plan_t(const CUtensorMap* tm, const FwdArgs& a, const 
   return launch_overlapped(kern, grid, kNumThreads, L::kDynSmem, st, tm[0], tm[1], tm[2], tm[3], args, plan.table);
 }
 
+template <int D, bool BF16>
+static cudaError_t launch_plan_d(bool qk8, const CUtensorMap* tm, const FwdArgs& a, const FwdPlan& plan, cudaStream_t st) {
+  if (qk8) return launch_plan_t<D, BF16, true>(tm, a, plan, st);
+  return a.pack > 1 ? launch_plan_t<D, BF16, false, true>(tm, a, plan, st) : launch_plan_t<D, BF16, false>(tm, a, plan, st);
+}
+
 // Balanced launch: a.part_o / a.part_ml / a.counters point into the caller's scratch.  qk8: the
 // INT8-QK variant (tm[0], tm[1] are the int8 Q / K maps).
 cudaError_t launch_fwd_ws_plan(int D, bool bf16, bool qk8, const CUtensorMap* tm, const FwdArgs& a,
                                const FwdPlan& plan, cudaStream_t st) {
-  if (D == 128) {
-    if (qk8) return bf16 ? launch_plan_t<128, true, true>(tm, a, plan, st) : launch_plan_t<128, false, true>(tm, a, plan, st);
-    return bf16 ? launch_plan_t<128, true, false>(tm, a, plan, st) : launch_plan_t<128, false, false>(tm, a, plan, st);
-  }
-  if (D == 64) {
-    if (qk8) return bf16 ? launch_plan_t<64, true, true>(tm, a, plan, st) : launch_plan_t<64, false, true>(tm, a, plan, st);
-    return bf16 ? launch_plan_t<64, true, false>(tm, a, plan, st) : launch_plan_t<64, false, false>(tm, a, plan, st);
-  }
+  if (D == 128) return bf16 ? launch_plan_d<128, true>(qk8, tm, a, plan, st) : launch_plan_d<128, false>(qk8, tm, a, plan, st);
+  if (D == 64) return bf16 ? launch_plan_d<64, true>(qk8, tm, a, plan, st) : launch_plan_d<64, false>(qk8, tm, a, plan, st);
   return cudaErrorInvalidValue;
+}
+
+template <int D, bool BF16>
+static cudaError_t launch_ws_d(const CUtensorMap* tm, const FwdArgs& a, int sm_count, cudaStream_t st) {
+  if (a.carry_mode != 0)  // a ring step: running state in, state or output out
+    return launch_ws_t<D, BF16, false, true>(tm, a, sm_count, st);
+  return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true>(tm, a, sm_count, st)
+                    : launch_ws_t<D, BF16, false>(tm, a, sm_count, st);
 }
 
 cudaError_t launch_fwd_ws(int D, bool bf16, const CUtensorMap* tm, const FwdArgs& a, int sm_count,
                           cudaStream_t st) {
-  if (a.carry_mode != 0) {  // a ring step: running state in, state or output out
-    if (D == 128)
-      return bf16 ? launch_ws_t<128, true, false, true>(tm, a, sm_count, st)
-                  : launch_ws_t<128, false, false, true>(tm, a, sm_count, st);
-    if (D == 64)
-      return bf16 ? launch_ws_t<64, true, false, true>(tm, a, sm_count, st)
-                  : launch_ws_t<64, false, false, true>(tm, a, sm_count, st);
-    return cudaErrorInvalidValue;
-  }
-  if (D == 128)
-    return bf16 ? launch_ws_t<128, true, false>(tm, a, sm_count, st) : launch_ws_t<128, false, false>(tm, a, sm_count, st);
-  if (D == 64)
-    return bf16 ? launch_ws_t<64, true, false>(tm, a, sm_count, st) : launch_ws_t<64, false, false>(tm, a, sm_count, st);
+  if (D == 128) return bf16 ? launch_ws_d<128, true>(tm, a, sm_count, st) : launch_ws_d<128, false>(tm, a, sm_count, st);
+  if (D == 64) return bf16 ? launch_ws_d<64, true>(tm, a, sm_count, st) : launch_ws_d<64, false>(tm, a, sm_count, st);
   return cudaErrorInvalidValue;
 }
 

@@ -62,7 +62,10 @@ float list_schedule(const std::vector<float>& cost, int sms, std::vector<float>*
   return end;
 }
 
-constexpr int kMinPiece = 6;       // K/V tiles; shorter pieces cost more than they balance (measured: a 4-tile piece loses)
+// K/V tiles; shorter pieces cost more than they balance.  A cut costs the same whatever the launch, so one
+// that is short overall is better off with idle SMs (4-tile pieces: N = 1024, 2 x 8 heads 18.4 us against 15.3
+// uncut; 777 against 3333 keys, 2 x 24/8 heads, 65.2 against 66.9 with 6-tile pieces; N = 4096 116.9 / 117.9).
+int min_piece(float plain_steps) { return plain_steps >= 24.f ? 4 : 6; }
 constexpr int kMaxParts = 64;      // pieces per item
 
 // Cost model, in steps (one K/V tile of a two-Q-tile CTA, about 2 us at D = 128): fixed cost of
@@ -76,7 +79,7 @@ float piece_cost() { return 1.3f; }
 // Phase 2, from the first item that does not: the SMs are filled one after the other up to T
 // (most room first); an item that crosses the end of an SM's room is cut there and continues on
 // the next SM.  Returns false when an item would need too many pieces.
-bool fill(const std::vector<int>& w, int sms, float T, float h, float fee, std::vector<Piece>* out) {
+bool fill(const std::vector<int>& w, int sms, float T, float h, float fee, int least, std::vector<Piece>* out) {
   out->clear();
   const int n = static_cast<int>(w.size());
   MinHeap heap = empty_sms(sms);
@@ -120,18 +123,18 @@ bool fill(const std::vector<int>& w, int sms, float T, float h, float fee, std::
         if (!whole_fits) {  // a piece of a cut item: it also pays the fee
           const int room = static_cast<int>(std::floor(Ts - load[si] - h - fee));
           if (room < rem) {
-            if (room < kMinPiece) {
+            if (room < least) {
               ++si;  // nothing useful fits here any more
               continue;
             }
-            // both sides of a cut at least kMinPiece long; a rest too short to cut stays whole
-            // (and overruns this SM's target by less than kMinPiece)
-            if (rem >= 2 * kMinPiece) take = std::min(room, rem - kMinPiece);
+            // both sides of a cut at least `least` long; a rest too short to cut stays whole
+            // (and overruns this SM's target by less than that)
+            if (rem >= 2 * least) take = std::min(room, rem - least);
           }
         }
         load[si] += take + h + (whole_fits ? 0.f : fee);
         round = placed[si]++;
-        if (Ts - load[si] - h - fee < kMinPiece) ++si;
+        if (Ts - load[si] - h - fee < least) ++si;
       }
       out->push_back(Piece{i, t0, t0 + take, 0, 0, round});
       t0 += take;
@@ -167,8 +170,8 @@ void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan) {
   for (int i = 0; i < n; ++i) {
     int pair, bh_i;
     item_to_pair_bh(a, static_cast<int>(n_pairs), i, &pair, &bh_i);
-    const int q0 = pair * 2 * kTileM;
-    const int nt = (q0 + kTileM < a.Nq) ? 2 : 1;
+    const int q0 = pair * 2 * a.tpt;
+    const int nt = (q0 + a.tpt < a.Nq) ? 2 : 1;
     w[i] = kv_tiles_of(a, q0, nt);
     if (w[i] > 65535) return;  // tile ranges travel as 16-bit numbers
     total += w[i];
@@ -180,6 +183,7 @@ void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan) {
   const float bound = (static_cast<float>(total) + h * n) / sms;
   if (plain <= 1.03f * bound) return;
 
+  const int least = min_piece(plain);
   std::vector<Piece> best, cur;
   float best_t = plain;
   int best_whole = 0;
@@ -189,8 +193,8 @@ void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan) {
   const float fine = std::max(0.5f, 0.004f * bound), coarse = std::max(fine, w_max / 16.f);
   for (int attempt = 0; attempt < 18; ++attempt) {
     const float up = attempt < 10 ? fine * attempt : fine * 9 + coarse * (attempt - 9);
-    const float T = std::max(bound + 0.75f * (h + fee) + up, kMinPiece + h + fee);
-    if (!fill(w, sms, T, h, fee, &cur)) continue;
+    const float T = std::max(bound + 0.75f * (h + fee) + up, least + h + fee);
+    if (!fill(w, sms, T, h, fee, least, &cur)) continue;
     int first_cut = n;
     for (const Piece& p : cur)
       if (p.nparts > 1) {
