@@ -24,6 +24,7 @@ _balance_scratch: dict = {}   # (device index, stream) -> zero-initialised uint8
 # dtype, flags).  A training or serving loop calls the operator with the same tensors again and again;
 # validating and filling the block costs more host time than a short-sequence kernel runs for.
 _param_cache: dict = {}
+_byref = C.byref
 _PARAM_CACHE_MAX = 256
 
 
@@ -267,33 +268,32 @@ def flash_attn_fwd(
                 _param_cache.clear()
             _param_cache[key] = (p, need)
     if p is not None:
-        dev_index = q.device.index
-        if torch.cuda.current_device() == dev_index:
-            rc = _launch_fwd(p, need, q.device, _current_raw_stream(dev_index))
+        dev = q.device
+        dev_index = dev.index
+        if _current_device() == dev_index:
+            rc = _launch_fwd(p, need, dev, _current_raw_stream(dev_index))
         else:
-            with torch.cuda.device(q.device):
-                rc = _launch_fwd(p, need, q.device, _current_raw_stream(dev_index))
-        _lib.check(rc, "miniattn_fwd")
+            with torch.cuda.device(dev):
+                rc = _launch_fwd(p, need, dev, _current_raw_stream(dev_index))
+        if rc != _lib.OK:
+            _lib.check(rc, "miniattn_fwd")
     if carry_out:
         return None
     return (out, lse) if return_lse else out
 
 
-def _current_raw_stream(device_index: int) -> int:
-    """cudaStream_t of torch's current stream on the device, without building a Stream object (3 us
-    of the 13 us a short-sequence call spends on the host)."""
-    try:
-        return torch._C._cuda_getCurrentRawStream(device_index)
-    except AttributeError:
-        return torch.cuda.current_stream(device_index).cuda_stream
+# cudaStream_t of torch's current stream on a device without building a Stream object, and the current device
+# without torch.cuda's initialisation check (a tensor on the GPU is at hand): 4 us of a short call's host time.
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda index: torch.cuda.current_stream(index).cuda_stream)
+_current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
 def _launch_fwd(p, need: int, device: torch.device, stream: int) -> int:
     if need > 0:
         scratch = _scratch_for(device, stream, need)
-        return _lib.lib.miniattn_fwd_balanced(C.byref(p), C.c_void_p(scratch.data_ptr()),
-                                              C.c_size_t(scratch.numel()), C.c_void_p(stream))
-    return _lib.lib.miniattn_fwd(C.byref(p), C.c_void_p(stream))
+        return _lib.lib.miniattn_fwd_balanced(_byref(p), scratch.data_ptr(), scratch.numel(), stream)
+    return _lib.lib.miniattn_fwd(_byref(p), stream)
 
 
 def carry_state(q: torch.Tensor, layout: str = "bhnd") -> torch.Tensor:
