@@ -315,8 +315,23 @@ void plan_decode(int B, int Hq, int Hkv, int Nq, int Nk, int D, int causal, long
   const double t_tile = rg == 1 ? 0.5 : rg == 2 ? 0.8 : 1.5;
   const double t_fold = 0.02 + std::min<double>(rows, 16 * rg) * D * 4 / 55e3;
   const long long most = std::max(1ll, std::min<long long>(tiles / 4, static_cast<long long>(std::sqrt(tiles * t_tile / t_fold))));
-  if (items * most >= slots && total >= 8 * slots) d->n_ctas = static_cast<int>(slots);
-  else d->n_ctas = static_cast<int>(std::min(slots, items * std::max(1ll, std::min(most, slots / items))));
+  // A CTA works on one item only wherever that leaves enough of them: one that ends a piece of one item and
+  // begins the next pays for two ends (about 5 us of syncs, publishing and folding) and so does the launch.
+  // 16 items of 563 tiles, D = 64: 39.3 us in 292 CTAs that straddle, 31.9 in 288 of one piece each, 30.0 in
+  // 256; 128 items of 63 tiles, D = 128: 49.0 in 296, 46.6 in 256; 512 items of 16 tiles: 49.5 in 296, 46.0 in
+  // 256 of two items each.  HBM is saturated by fewer CTAs than fit (208 to 272), and pieces cost; where the
+  // tiles are bound by mma.sync (rg > 1) every slot counts.
+  const long long room = rg == 1 ? slots * 7 / 8 : slots;
+  if (items <= room) {
+    d->n_ctas = static_cast<int>(items * std::max(1ll, std::min(most, room / items)));
+    return;
+  }
+  d->n_ctas = static_cast<int>(slots);
+  for (long long j = (items + slots - 1) / slots; items / j >= slots * 2 / 3; ++j)
+    if (items % j == 0) {
+      d->n_ctas = static_cast<int>(items / j);
+      return;
+    }
 }
 
 }  // namespace ma
