@@ -133,7 +133,7 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar) {
 //
 // PACK: the a.pack query heads that share a KV head share Q tiles too, a.tpt tokens of each: row r of a tile
 // is token r / a.pack, head r % a.pack of the group (head_pack in api.cu says when).
-template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false, bool PACK = false>
+template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false, bool PACK = false, bool LONG = false>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -333,10 +333,12 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // How much of the loop is unrolled.  A short launch pays for every line of code it fetches once: one
       // copy of the body for both halves of a tile, and a rescale that is a loop, take 9.55 instead of 9.86 us
       // at N = 512, 32.4 / 33.1 at N = 2048, 434 / 441 at N = 8192 (cut items), 19.3 / 20.2 for D = 96 N = 1001.
-      // Unrolled, the steady state is the faster one: ring steps (16 heads, 256 tiles an item: 3663 / 3789) and
-      // INT8-QK (642 / 657) keep that.  At D = 64 only the rescale is a loop (18.6 / 19.4 us at N = 1024).
-      constexpr int kHalvesUnrolled = (D == 128 && !CARRY && !QK8) ? 1 : 2;
-      constexpr int kRescaleUnrolled = (CARRY || QK8) ? D / 32 : 1;
+      // Unrolled, the steady state is the faster one: ring steps, INT8-QK (642 / 657 us, N = 8192) and, at
+      // D = 128, launches over 64 K/V tiles and more (LONG; 32 causal heads, N = 131072: 114.2 / 119.5 ms;
+      // 16 causal heads, N = 32768: 3555 / 3681 us, N = 8192: 217.6 / 218.6).  At D = 64 only the rescale is a
+      // loop (18.6 / 19.4 us at N = 1024).
+      constexpr int kHalvesUnrolled = (D == 128 && !CARRY && !QK8 && !LONG) ? 1 : 2;
+      constexpr int kRescaleUnrolled = (CARRY || QK8 || LONG) ? D / 32 : 1;
       for (int j = 0; j < n_tiles; ++j) {
         // cj turns a raw score into log2 units: softmax scale * log2e, times the two
         // de-quantisation scales of this (Q block, K block) for the int8 variant.
@@ -854,10 +856,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------------
-template <int D, bool BF16, bool QK8, bool CARRY = false, bool PACK = false>
+template <int D, bool BF16, bool QK8, bool CARRY = false, bool PACK = false, bool LONG = false>
 static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_count, cudaStream_t st) {
   using L = WsLayout<D, QK8>;
-  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY, PACK>;
+  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY, PACK, LONG>;
   static std::atomic<unsigned long long> smem_set{0};  // per instantiation: devices already configured
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
@@ -913,10 +915,16 @@ cudaError_t launch_fwd_ws_plan(int D, bool bf16, bool qk8, const CUtensorMap* tm
   return cudaErrorInvalidValue;
 }
 
+constexpr int kLongTiles = 64;  // K/V tiles from which on the unrolled loop pays (see kHalvesUnrolled)
 template <int D, bool BF16>
 static cudaError_t launch_ws_d(const CUtensorMap* tm, const FwdArgs& a, int sm_count, cudaStream_t st) {
   if (a.carry_mode != 0)  // a ring step: running state in, state or output out
     return launch_ws_t<D, BF16, false, true>(tm, a, sm_count, st);
+  if constexpr (D == 128) {
+    if (a.Nk >= kLongTiles * kTileN)
+      return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true, true>(tm, a, sm_count, st)
+                        : launch_ws_t<D, BF16, false, false, false, true>(tm, a, sm_count, st);
+  }
   return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true>(tm, a, sm_count, st)
                     : launch_ws_t<D, BF16, false>(tm, a, sm_count, st);
 }
