@@ -183,6 +183,12 @@ def ring_forward(
     bufs = [(torch.empty_like(k_cur), torch.empty_like(v_cur)) for _ in range(2 if world > 1 else 0)]
     q_blocks = (q_local[:, :, :L], q_local[:, :, L:])
     out = torch.empty_like(q_local)
+    if fused and world == 1 and L2 == 2 * L:
+        # the two blocks of a ring of one are neighbours: one causal launch, no state to carry (three launches
+        # otherwise, each with the tail of its own)
+        from .ops import flash_attn_fwd
+        flash_attn_fwd(q_local, k_cur, v_cur, causal=causal, softmax_scale=softmax_scale, out=out)
+        return out
     if fused:
         from .ops import carry_state, flash_attn_fwd
         # one state buffer for all 2L local rows; a launch on one block addresses its half of it
