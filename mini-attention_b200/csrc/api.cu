@@ -336,6 +336,7 @@ static void fill_args(const MiniAttnFwdParams* p, ma::FwdArgs* a, int pack) {
   a->Hkv = p->Hkv;
   a->B = p->B;
   a->causal = p->causal;
+  a->d96 = p->D == 96;
   a->scale = p->softmax_scale > 0.f ? p->softmax_scale : 1.0f / sqrtf((float)p->D);
   a->scale_log2 = a->scale * 1.4426950408889634f;
   a->pack = pack;

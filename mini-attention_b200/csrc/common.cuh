@@ -13,6 +13,7 @@ struct FwdArgs {
   long long k_pos0;    // global position of key token 0
   int Nq, Nk, Hq, Hkv, B;
   int causal;
+  int d96;             // head dim 96 on the D = 128 kernels: selects the NARROW form
   float scale;         // softmax scale
   float scale_log2;    // softmax scale * log2(e)
   int pack;            // query heads that share a Q tile: row r of a tile is token r / pack, head r % pack

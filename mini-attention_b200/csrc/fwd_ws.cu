@@ -133,13 +133,20 @@ __device__ __forceinline__ void warp_arrive(uint32_t bar) {
 //
 // PACK: the a.pack query heads that share a KV head share Q tiles too, a.tpt tokens of each: row r of a tile
 // is token r / a.pack, head r % a.pack of the group (head_pack in api.cu says when).
-template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false, bool PACK = false, bool LONG = false>
+//
+// NARROW: head dim 96 on the D = 128 tiles, whose columns 96..127 hold zeros (Q, K, V).  The MMAs and the
+// epilogue leave those columns out, a quarter of the tensor work; what O's hold there is clipped by its map.
+// N = 1001, 3 x 7 heads 19.0 -> 17.7 us; N = 4096, 2 x 16 heads 211 -> 199; N = 16002, 3 x 2 causal 293 -> 275
+// (a run-time switch instead of the template cost D = 128 0.15 us a launch).
+template <int D, bool BF16, bool QK8, bool PLAN, bool CARRY = false, bool PACK = false, bool LONG = false,
+          bool NARROW = false>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
               const FwdArgs a,
               const __grid_constant__ std::conditional_t<PLAN, PlanTable, NoPlanTable> plan) {
   using L = WsLayout<D, QK8>;
+  constexpr int kCols = NARROW ? 96 : D;  // head dim the MMAs work on
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sbase = (raw + 1023u) & ~1023u;
@@ -338,7 +345,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // 16 causal heads, N = 32768: 3555 / 3681 us, N = 8192: 217.6 / 218.6).  At D = 64 only the rescale is a
       // loop (18.6 / 19.4 us at N = 1024).
       constexpr int kHalvesUnrolled = (D == 128 && !CARRY && !QK8 && !LONG) ? 1 : 2;
-      constexpr int kRescaleUnrolled = (CARRY || QK8 || LONG) ? D / 32 : 1;
+      constexpr int kRescaleUnrolled = (CARRY || QK8 || LONG) ? kCols / 32 : 1;
       for (int j = 0; j < n_tiles; ++j) {
         // cj turns a raw score into log2 units: softmax scale * log2e, times the two
         // de-quantisation scales of this (Q block, K block) for the int8 variant.
@@ -405,7 +412,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 tc_fence_after();
                 const uint32_t tO = tmem_base + L::kColO + D * t + lane_off;
 #pragma unroll (kRescaleUnrolled)
-                for (int q = 0; q < D / 32; ++q) {
+                for (int q = 0; q < kCols / 32; ++q) {
                   uint32_t o[32];
                   tmem_ld32(tO + q * 32, o);
                   tmem_wait_ld();
@@ -496,7 +503,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             const long long my = (static_cast<long long>(pe_slot0 + pe_part) * 2 + t) * kTileM;
             float4* po = reinterpret_cast<float4*>(a.part_o + my * D) + r;
 #pragma unroll
-            for (int q = 0; q < D / 32; ++q) {
+            for (int q = 0; q < kCols / 32; ++q) {
               uint32_t o[32];
               tmem_ld32(tO + q * 32, o);
               tmem_wait_ld();
@@ -578,7 +585,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               }
               // more than two pieces: accumulate into the TMEM accumulator
 #pragma unroll
-              for (int q = 0; q < D / 32; ++q) {
+              for (int q = 0; q < kCols / 32; ++q) {
                 uint32_t o[32];
                 tmem_ld32(tO + q * 32, o);
                 tmem_wait_ld();
@@ -636,7 +643,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             write_out = false;
             float4* po = reinterpret_cast<float4*>(c_o) + r;
 #pragma unroll
-            for (int q = 0; q < D / 32; ++q) {
+            for (int q = 0; q < kCols / 32; ++q) {
               uint32_t o[32];
               if (n_tiles > 0) {
                 tmem_ld32(tO + q * 32, o);
@@ -675,7 +682,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         //      O / l -> 16 bit -> swizzled smem (the tile's Q buffer) -> TMA store
         const uint32_t stage = sQ + t * L::kTileBytes;
 #pragma unroll
-        for (int q = 0; q < D / 32; ++q) {
+        for (int q = 0; q < kCols / 32; ++q) {
           float o[32];
           if (n_tiles > 0) {
             uint32_t u[32];
@@ -739,7 +746,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // kind::f16: D fmt f32, A/B f16 or bf16.  kind::i8: D fmt s32 (2), A/B signed int8 (1).
         constexpr uint32_t idesc_s =
             QK8 ? make_idesc(2, 1, 0, 0, kTileM, kHalfN) : make_idesc(1, BF16 ? 1 : 0, 0, 0, kTileM, kHalfN);
-        constexpr uint32_t idesc_o = make_idesc(1, BF16 ? 1 : 0, 0, 1, kTileM, D);
+        constexpr uint32_t idesc_o = make_idesc(1, BF16 ? 1 : 0, 0, 1, kTileM, kCols);
         const uint32_t sQt = sQ + t * L::kTileBytes;
         const uint32_t tO = tmem_base + L::kColO + D * t;
         const uint32_t tSt = tmem_base + L::kColS + 128 * t;
@@ -768,7 +775,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           } else {
             const uint32_t kb = sRing + slot * L::kTileBytes + hb * kHalfN * 128;
 #pragma unroll
-            for (int k = 0; k < D / 16; ++k) {
+            for (int k = 0; k < kCols / 16; ++k) {
               const uint32_t off = (k / 4) * kBoxBytes + (k % 4) * 32;
               const uint64_t da = make_smem_desc(sQt + off, 16, 1024);
               const uint64_t db = make_smem_desc(kb + off, 16, 1024);
@@ -856,10 +863,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------------------------
-template <int D, bool BF16, bool QK8, bool CARRY = false, bool PACK = false, bool LONG = false>
+template <int D, bool BF16, bool QK8, bool CARRY = false, bool PACK = false, bool LONG = false, bool NARROW = false>
 static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_count, cudaStream_t st) {
   using L = WsLayout<D, QK8>;
-  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY, PACK, LONG>;
+  auto kern = fwd_ws_kernel<D, BF16, QK8, false, CARRY, PACK, LONG, NARROW>;
   static std::atomic<unsigned long long> smem_set{0};  // per instantiation: devices already configured
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
@@ -886,11 +893,11 @@ static cudaError_t launch_ws_t(const CUtensorMap* tm, const FwdArgs& a, int sm_c
                            tm[3], args, NoPlanTable{0});
 }
 
-template <int D, bool BF16, bool QK8, bool PACK = false>
+template <int D, bool BF16, bool QK8, bool PACK = false, bool NARROW = false>
 static cudaError_t launch_plan_t(const CUtensorMap* tm, const FwdArgs& a, const FwdPlan& plan,
                                  cudaStream_t st) {
   using L = WsLayout<D, QK8>;
-  auto kern = fwd_ws_kernel<D, BF16, QK8, true, false, PACK>;
+  auto kern = fwd_ws_kernel<D, BF16, QK8, true, false, PACK, false, NARROW>;
   static std::atomic<unsigned long long> smem_set{0};
   cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void*>(kern), L::kDynSmem, &smem_set);
   if (e != cudaSuccess) return e;
@@ -903,6 +910,11 @@ static cudaError_t launch_plan_t(const CUtensorMap* tm, const FwdArgs& a, const 
 template <int D, bool BF16>
 static cudaError_t launch_plan_d(bool qk8, const CUtensorMap* tm, const FwdArgs& a, const FwdPlan& plan, cudaStream_t st) {
   if (qk8) return launch_plan_t<D, BF16, true>(tm, a, plan, st);
+  if constexpr (D == 128) {
+    if (a.d96)
+      return a.pack > 1 ? launch_plan_t<D, BF16, false, true, true>(tm, a, plan, st)
+                        : launch_plan_t<D, BF16, false, false, true>(tm, a, plan, st);
+  }
   return a.pack > 1 ? launch_plan_t<D, BF16, false, true>(tm, a, plan, st) : launch_plan_t<D, BF16, false>(tm, a, plan, st);
 }
 
@@ -921,7 +933,15 @@ static cudaError_t launch_ws_d(const CUtensorMap* tm, const FwdArgs& a, int sm_c
   if (a.carry_mode != 0)  // a ring step: running state in, state or output out
     return launch_ws_t<D, BF16, false, true>(tm, a, sm_count, st);
   if constexpr (D == 128) {
-    if (a.Nk >= kLongTiles * kTileN)
+    const bool is_long = a.Nk >= kLongTiles * kTileN;
+    if (a.d96) {
+      if (is_long)
+        return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true, true, true>(tm, a, sm_count, st)
+                          : launch_ws_t<D, BF16, false, false, false, true, true>(tm, a, sm_count, st);
+      return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true, false, true>(tm, a, sm_count, st)
+                        : launch_ws_t<D, BF16, false, false, false, false, true>(tm, a, sm_count, st);
+    }
+    if (is_long)
       return a.pack > 1 ? launch_ws_t<D, BF16, false, false, true, true>(tm, a, sm_count, st)
                         : launch_ws_t<D, BF16, false, false, false, true>(tm, a, sm_count, st);
   }
