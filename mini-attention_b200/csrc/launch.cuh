@@ -24,10 +24,10 @@ inline cudaError_t allow_dynamic_smem(const void* kern, int bytes, std::atomic<u
 // A launch after a launch costs 1 to 2 us less for it (measured back to back: N = 512, 2 x 8 heads 11.6 ->
 // 11.2 us; D = 64, N = 1024, 4 x 12 heads causal 20.5 -> 18.6; decode of 16 x 4001 keys 50.5 -> 48.7).
 template <typename Kernel, typename... Args>
-inline cudaError_t launch_overlapped(Kernel kern, unsigned grid, unsigned threads, size_t smem, cudaStream_t st,
+inline cudaError_t launch_overlapped(Kernel kern, dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
                                      const Args&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

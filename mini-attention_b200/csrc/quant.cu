@@ -8,7 +8,8 @@
 // Two launches: stage 1 quantises Q and sums the columns of K (independent work, one grid), stage 2
 // smooths and quantises K.  Stage 2 is launched as a programmatic dependent of stage 1: its CTAs
 // become resident while stage 1 drains and load their K slabs before they wait for stage 1's
-// column sums, so the second launch's ramp and first loads hide under the first one's tail.
+// column sums, so the second launch's ramp and first loads hide under the first one's tail; stage 1 stands in
+// the same relation to the kernel before it, and the attention kernel to stage 2.
 // HBM-bound byte movers: 16-byte loads, 8-byte int8 stores, one CTA per
 // (128-token block, head, batch) or per 1024-token column-sum chunk.  Algorithmic traffic per element: K 2 B (mean pass) + 2 B + 1 B,
 // Q 2 B + 1 B, plus 4 B per 128 x D slab for the scale.
@@ -18,6 +19,8 @@
 
 #include <cstdint>
 #include <mutex>
+
+#include "launch.cuh"
 
 namespace ma {
 
@@ -108,6 +111,7 @@ __device__ __forceinline__ void quant_body(const uint16_t* __restrict__ x, long 
   if (SMOOTH) {
     // everything above is independent of stage 1; its column sums are complete and visible from here
     cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();  // the attention kernel's set-up may overlap the rest
     if (threadIdx.x < D) {
       float s = 0.f;
       const float* p = partial + (static_cast<long long>(b) * H + h) * n_chunks * D + threadIdx.x;
@@ -186,7 +190,10 @@ prepass_stage1_kernel(const uint16_t* __restrict__ q, long long qsb, long long q
                       int Hq, int nqb, int8_t* __restrict__ q8, float* __restrict__ sq, float fold,
                       const uint16_t* __restrict__ k, long long ksb, long long ksh, long long ksn, int Nk,
                       int Hkv, int nch, float* __restrict__ partial, int q_blocks) {
-  // the dependent launch (stage 2) may start as soon as every CTA of this grid is under way
+  // This launch may start while the kernel before it drains (an earlier call's attention still reads the
+  // buffers written here).  The dependent launch (stage 2) may start as soon as every CTA of this grid is
+  // past that wait, no earlier: it reads K before its own wait.
+  cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();
   // the column-sum CTAs read eight times as much as a quantiser CTA: they go first
   const int s_blocks = static_cast<int>(gridDim.x) - q_blocks;
@@ -222,24 +229,16 @@ static cudaError_t launch_quant_t(const void* q, const long long* qs, const void
   const long long q_blocks = static_cast<long long>(nqb) * Hq * B;
   const long long s_blocks = static_cast<long long>(nch) * Hkv * B;
   if (q_blocks + s_blocks > 0x7fffffffll) return cudaErrorInvalidValue;
-  if (q_blocks + s_blocks > 0)
-    prepass_stage1_kernel<D, BF16><<<static_cast<unsigned>(q_blocks + s_blocks), 256, 0, st>>>(
-        static_cast<const uint16_t*>(q), qs[0], qs[1], qs[2], Nq, Hq, nqb, q8, sq, q_fold,
-        static_cast<const uint16_t*>(k), ks[0], ks[1], ks[2], Nk, Hkv, nch, partial, static_cast<int>(q_blocks));
-  if (Nk > 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nkb, Hkv, B);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = (q_blocks + s_blocks > 0) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, quant_k_kernel<D, BF16>, static_cast<const uint16_t*>(k), ks[0], ks[1],
-                                       ks[2], Nk, static_cast<const float*>(partial), nch, k8, sk, k_mean);
+  if (q_blocks + s_blocks > 0) {
+    cudaError_t e = launch_overlapped(prepass_stage1_kernel<D, BF16>, static_cast<unsigned>(q_blocks + s_blocks), 256, 0, st,
+                                      static_cast<const uint16_t*>(q), qs[0], qs[1], qs[2], Nq, Hq, nqb, q8, sq, q_fold,
+                                      static_cast<const uint16_t*>(k), ks[0], ks[1], ks[2], Nk, Hkv, nch, partial,
+                                      static_cast<int>(q_blocks));
     if (e != cudaSuccess) return e;
   }
+  if (Nk > 0)
+    return launch_overlapped(quant_k_kernel<D, BF16>, dim3(nkb, Hkv, B), 256, 0, st, static_cast<const uint16_t*>(k), ks[0],
+                             ks[1], ks[2], Nk, static_cast<const float*>(partial), nch, k8, sk, k_mean);
   return cudaGetLastError();
 }
 
