@@ -224,6 +224,16 @@ def run_reference_arm(args, w, rank):
     print(json.dumps(line), flush=True)
 
 
+def ring_launches(rank, world, causal, block):
+    """Attention launches of one ring pass on this rank: one for a ring of one, else what the launcher's plan says."""
+    from miniattn import parallel as par
+    if world == 1:
+        return 1
+    steps = [par.ring_step_tasks(rank, world, s, causal) for s in range(world)]
+    remaining, started = [sum(t.q_half == h for st in steps for t in st) for h in (0, 1)], [False, False]
+    return sum(len(par.ring_step_launches(st, remaining, started, block % 128 == 0)) for st in steps)
+
+
 def reference_gpu_kernel_leg(B, H, N_list, D, dev, flush, stream):
     """Optional baseline: the reference's own mma.sync kernel (newest tree) rebuilt for sm_100 by
     oracle/build_ref_kernel.py, timed on this GPU with the same protocol in two of its configurations:
@@ -404,7 +414,7 @@ def main():
         elif key == "c5":
             grp = get_ring_group()
             ms = timed(lambda: par.ring_forward(ql, kl, vl, causal=True, rank=rank, world=world, group=grp), steps, warmup)
-            res["launches_per_step"] = sum(len(par.ring_step_tasks(rank, world, s_, True)) for s_ in range(world))
+            res["launches_per_step"] = ring_launches(rank, world, True, ql.shape[2] // 2)
             res["parity_check"] = ring_parity_check(grp)
         else:
             ol = torch.empty_like(ql)
@@ -440,7 +450,7 @@ def main():
         def attend():
             miniattn.flash_attn_fwd_int8qk(q, k, v, causal=causal, out=o, buffers=bufs)
     elif ring:
-        launches_per_step = sum(len(par.ring_step_tasks(rank, world, s_, causal)) for s_ in range(world))
+        launches_per_step = ring_launches(rank, world, causal, sN // 2)
         ring_out = [o]
         grp_main = get_ring_group()
 
