@@ -88,7 +88,8 @@ struct WsLayout {
   static constexpr int kBarPReady = kBarSFull + 4;         // [2][2] softmax -> MMA
   static constexpr int kBarODone = kBarPReady + 4;         // [2][2] MMA -> softmax (rescale, epilogue)
   static constexpr int kBarStagger = kBarODone + 4;        // one-shot: tile 0 published its first row maxima
-  static constexpr int kNumBars = kBarStagger + 1;
+  static constexpr int kBarTileDone = kBarStagger + 1;     // [2] one-shot: every MMA of Q tile t has finished
+  static constexpr int kNumBars = kBarTileDone + 2;
   static constexpr int kOffMisc = kOffBar + kNumBars * 8;  // tmem slot, abort flag, arrival order [2]
   static constexpr int kBytes = kOffMisc + 32;
   static constexpr int kDynSmem = kBytes + 1024;
@@ -532,9 +533,12 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             named_bar_sync(kBarEpilogue + t, 128);
             __threadfence();
             // The other pieces' partials come in through the K/V ring (this tile's half of it),
-            // one bulk copy each; the ring is free once the other Q tile's MMAs are done too.
+            // one bulk copy each; the ring is free once the other Q tile's MMAs are done too.  That wait has a
+            // one-shot barrier: this thread did not follow the phases of the other tile's kBarODone, the other
+            // tile may be two and more of them behind (the ring holds two K/V tiles, four at D = 64), and a
+            // parity that is two phases old reads as done.
             // The first copy is started before anything else so that the rest overlaps it.
-            if (nt == 2) mbar_wait(bar(L::kBarODone + 2 * (1 - t) + 1), (n_tiles - 1) & 1, wc, kErrWaitO);
+            if (nt == 2) mbar_wait(bar(L::kBarTileDone + 1 - t), 0, wc, kErrWaitO);
             constexpr uint32_t kPartBytes = D * kTileM * 4;
             const uint32_t ring_off = L::kOffRing + t * (L::kStages / 2) * L::kTileBytes;
             const int first_other = (pe_part == 0) ? 1 : 0;
@@ -620,9 +624,8 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           float m_tot = m_cur, l_tot = l_run, w_self = 1.f, w_c = 0.f;
           if (a.carry_mode & 1) {
             // The state comes in through this tile's half of the K/V ring, idle once the other
-            // Q tile's MMAs are done too.
-            if (n_tiles > 0 && nt == 2)
-              mbar_wait(bar(L::kBarODone + 2 * (1 - t) + 1), (n_tiles - 1) & 1, wc, kErrWaitO);
+            // Q tile's MMAs are done too (the one-shot barrier: see the wait of a cut item above).
+            if (n_tiles > 0 && nt == 2) mbar_wait(bar(L::kBarTileDone + 1 - t), 0, wc, kErrWaitO);
             if (r == 0) {
               fence_proxy_async_all();
               mbar_expect_tx(bar(L::kBarQFull + t), kPartBytes);
@@ -831,6 +834,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
           if (has_next) ++cons;
         }
+        if constexpr (PLAN || CARRY) mma_commit(bar(L::kBarTileDone + t));
       }
       __syncwarp();
     } else if (warp == kWarpTma) {
