@@ -423,7 +423,9 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 }
                 tmem_wait_st();
               }
-              if (t == 0 && first) warp_arrive(bar(L::kBarStagger));
+              // once: in the second pass of this half (a row without visible keys, a NaN) it would arrive for the
+              // next phase, and a late waiter of the first would miss it
+              if (t == 0 && first && pass == 0) warp_arrive(bar(L::kBarStagger));
             }
             // exponent of a score x: x*cj - m; for the int8 variant x carries kBias, taken out here
             float mc = (m_cur == -INFINITY) ? 0.f : m_cur;

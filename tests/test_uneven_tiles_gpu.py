@@ -54,3 +54,21 @@ def test_carried_chains(Nq, cuts, D, climbing):
                                           carry_out=b < cuts[-1])
         assert miniattn.device_status(DEV) == 0
         assert (out.float().cpu() - ref).abs().max().item() <= TOL[torch.float16]
+
+
+@pytest.mark.parametrize("balance", [True, False])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Nq,Nk,pos", [(256, 256, -128), (384, 700, -192), (1024, 2000, -500)])
+def test_first_tile_without_visible_keys(Nq, Nk, pos, D, balance):
+    """All rows of the first Q tile lie before every key: their softmax takes each half twice, the first one too,
+    and the second tile, which starts on a signal of the first, must start once and be right."""
+    q, k, v = make_inputs(2, 4, 4, Nq, Nk, D, torch.float16, seed=Nq)
+    ref, ref_lse = attention_reference(q, k, v, causal=True, q_pos0=pos, return_lse=True, out_dtype=torch.float32)
+    qd, kd, vd = q.to(DEV), k.to(DEV), v.to(DEV)
+    for _ in range(4):
+        out, lse = miniattn.flash_attn_fwd(qd, kd, vd, causal=True, q_pos0=pos, return_lse=True, kernel="ws",
+                                           balance=balance)
+        assert miniattn.device_status(DEV) == 0
+        assert float(out[:, :, :-pos].abs().max()) == 0.0 and bool((lse[:, :, :-pos] == float("-inf")).all())
+        assert (out.float().cpu() - ref).abs().max().item() <= TOL[torch.float16]
+        assert (lse.cpu()[:, :, -pos:] - ref_lse[:, :, -pos:]).abs().max().item() <= 1e-3
