@@ -377,8 +377,9 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
           // No row maximum is searched for in the usual half: the exponentials are taken against the
           // reference m_cur the row already has, and their sum, which is wanted anyway, says whether it
-          // still serves.  A sum of at most 2^8 bounds every term by 2^8, the headroom the lazy update
-          // always allowed.  Where some row of the warp has none yet (its first visible keys) or its sum
+          // still serves.  No term is negative, and none is smaller than its exponential unless that is
+          // above 2^126 (where the polynomial stops), so a sum of at most 2^8 bounds every one by 2^8, the
+          // headroom the lazy update always allowed.  Where some row of the warp has none yet (its first visible keys) or its sum
           // came out larger, the maxima are found, O is rescaled here, and the exponentials are taken
           // (again): at most twice per half, and rare past the first.
           constexpr float kBias = QK8 ? 12582912.f : 0.f;

@@ -343,15 +343,26 @@ __device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b) {
   asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+// x held to [-b, b] (b > 0) by one instruction; a NaN comes out as b (the sign of the NaNs that arithmetic makes
+// is positive)
+__device__ __forceinline__ float clamp_abs(float x, float b) {
+  float d;
+  asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(d) : "f"(x), "f"(b));
+  return d;
+}
 // 2^x for a pair on the FMA pipe instead of the exp2 unit: x = n + f with n = round(x) taken from
 // the low mantissa bits of x + 1.5*2^23 and f in [-0.5, 0.5]; 2^f by the cubic
 // whose relative error has the least mean square over that range (rms 4.6e-5, mean 0, at most 1.4e-4: below
-// the half-ulp of a 16-bit P, and no bias in a row's sum), n added into the exponent field.  Inputs below -126
-// (masked scores are -inf) give 2^-126, which rounds to 0 in 16 bit.
+// the half-ulp of a 16-bit P, and no bias in a row's sum), n added into the exponent field.  Arguments are held
+// to [-126, 126]: below (masked scores are -inf) the result is 2^-126, which rounds to 0 in 16 bit; above it is
+// 2^126, too large for any sum to hide.  Without the upper end n would carry out of the exponent field: 2^150 came
+// out as -1.2e-32.  One instruction holds both ends, as many as the lower end alone took: N = 8192 (2 x 8 heads,
+// D = 128) 422 us before and 423 after, D = 64 (2 x 16) 647 / 646; min after max 421 / 654, in the unrolled loops 3 %
+// slower; the largest of the arguments compared beside the sum 1 to 4 % slower.
 // FINE: the quartic with the least maximum relative error (2.6e-6), one FMA more.
 template <bool FINE>
 __device__ __forceinline__ void exp2_poly_f32x2(float x0, float x1, float& p0, float& p1) {
-  const uint64_t x = pack_f32x2(fmaxf(x0, -126.f), fmaxf(x1, -126.f));
+  const uint64_t x = pack_f32x2(clamp_abs(x0, 126.f), clamp_abs(x1, 126.f));
   const uint64_t xr = add_f32x2(x, pack_f32x2(12582912.f, 12582912.f));
   const uint64_t n = add_f32x2(xr, pack_f32x2(-12582912.f, -12582912.f));
   const uint64_t f = fma_f32x2(n, pack_f32x2(-1.f, -1.f), x);
