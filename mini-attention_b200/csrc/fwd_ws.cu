@@ -395,14 +395,17 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 mx4[q] = -INFINITY;
 #pragma unroll
                 for (int i = 0; i < 16; i += 2)
-                  mx4[q] = fmax3(mx4[q], __uint_as_float(s[q >> 1][(q & 1) * 16 + i]),
-                                 __uint_as_float(s[q >> 1][(q & 1) * 16 + i + 1]));
+                  mx4[q] = fmax3_nan(mx4[q], __uint_as_float(s[q >> 1][(q & 1) * 16 + i]),
+                                     __uint_as_float(s[q >> 1][(q & 1) * 16 + i + 1]));
               }
-              float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+              float mx = fmax3_nan(fmax3_nan(mx4[0], mx4[1], mx4[2]), mx4[3], mx4[3]);
               if constexpr (QK8) mx -= kBias;
               mx *= cj;  // log2 units, like m_cur
+              // A NaN among the scores, or +inf (inf - inf), makes the row's result a NaN.  On a column of the
+              // polynomial neither would show, so the reference becomes one, and with it every exponential.
+              if (!(mx < INFINITY)) mx = __int_as_float(0x7fffffff);
               float alpha = 1.f;
-              if (mx > m_cur) {
+              if (!(mx <= m_cur)) {
                 alpha = ex2(m_cur - mx);
                 m_cur = mx;
               }

@@ -323,6 +323,11 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+__device__ __forceinline__ float fmax3_nan(float a, float b, float c) {  // NaN where any of them is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 // Packed fp32 pairs (one issue slot for two lanes of FMA / ADD on sm_100): a pair lives in a
 // 64-bit register, low word first.
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
