@@ -170,7 +170,9 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     const int hk = kvh % a.Hkv, b = kvh / a.Hkv;
     const int row0 = rb * kRows;
 
-    // Q fragments of this warp's 16 rows, and how many keys its two rows of this lane may see
+    // Q fragments of this warp's 16 rows, and how many keys its two rows of this lane may see.  Ordinary
+    // loads, not the read-only kind: the kernel before this one may write Q while this one already runs, and with
+    // o = q this one writes it.  (Past L1 they cost 2 us of 24 at 4 tokens of 64/8 heads: four warps share the rows.)
     uint32_t qf[D / 16][4];
     int vis[2];
 #pragma unroll
@@ -185,8 +187,8 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 #pragma unroll
       for (int ks = 0; ks < D / 16; ++ks) {
         const int col = ks * 16 + tig * 2;  // D = 96 runs on the D = 128 kernel: columns past it are 0
-        qf[ks][e] = (ok && col < a.D) ? __ldg(reinterpret_cast<const uint32_t*>(qp + col)) : 0u;
-        qf[ks][2 + e] = (ok && col + 8 < a.D) ? __ldg(reinterpret_cast<const uint32_t*>(qp + col + 8)) : 0u;
+        qf[ks][e] = (ok && col < a.D) ? *reinterpret_cast<const uint32_t*>(qp + col) : 0u;
+        qf[ks][2 + e] = (ok && col + 8 < a.D) ? *reinterpret_cast<const uint32_t*>(qp + col + 8) : 0u;
       }
     }
     const int vis_min = __reduce_min_sync(0xffffffffu, min(vis[0], vis[1]));

@@ -331,11 +331,11 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       float l_run = 0.f;
       float sq_t = 0.f, sk_next = 0.f;
       const float* sk_row = nullptr;
-      if constexpr (QK8) {
-        sq_t = __ldg(a.sq + (static_cast<long long>(b) * a.Hq + h) * a.n_q_tiles + (q0 / kTileM + t));
+      if constexpr (QK8) {  // scales through L2: the pre-pass may still write them while this kernel already runs
+        sq_t = __ldcg(a.sq + (static_cast<long long>(b) * a.Hq + h) * a.n_q_tiles + (q0 / kTileM + t));
         sk_row = a.sk + (static_cast<long long>(b) * a.Hkv + hk) * ((a.Nk + kTileN - 1) / kTileN);
         sk_row += kv_t0;
-        if (n_tiles > 0) sk_next = __ldg(sk_row);
+        if (n_tiles > 0) sk_next = __ldcg(sk_row);
       }
 
       // How much of the loop is unrolled.  A short launch pays for every line of code it fetches once: one
@@ -353,7 +353,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         float cj = c;
         if constexpr (QK8) {
           cj = sq_t * sk_next;
-          if (j + 1 < n_tiles) sk_next = __ldg(sk_row + j + 1);
+          if (j + 1 < n_tiles) sk_next = __ldcg(sk_row + j + 1);
         }
 #pragma unroll (kHalvesUnrolled)
         for (int hb = 0; hb < 2; ++hb) {

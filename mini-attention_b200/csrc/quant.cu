@@ -13,6 +13,8 @@
 // HBM-bound byte movers: 16-byte loads, 8-byte int8 stores, one CTA per
 // (128-token block, head, batch) or per 1024-token column-sum chunk.  Algorithmic traffic per element: K 2 B (mean pass) + 2 B + 1 B,
 // Q 2 B + 1 B, plus 4 B per 128 x D slab for the scale.
+// What these kernels read is not declared __restrict__: the compiler would take it for read-only over the whole
+// kernel, and the kernel before may still write it while this one already runs (before its grid dependency wait).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -55,7 +57,7 @@ constexpr int kSumRows = 1024;  // tokens per partial column sum
 
 // partial[b, h, chunk, d] = sum over the chunk's tokens of k[b, h, token, d]
 template <int D, bool BF16>
-__device__ __forceinline__ void colsum_body(const uint16_t* __restrict__ k, long long sb, long long sh,
+__device__ __forceinline__ void colsum_body(const uint16_t* k, long long sb, long long sh,
                                             long long sn, int N, float* __restrict__ partial,
                                             int n_chunks, int chunk, int h, int b, int H) {
   constexpr int CPR = D / 8;          // 16-byte chunks per row
@@ -85,8 +87,8 @@ __device__ __forceinline__ void colsum_body(const uint16_t* __restrict__ k, long
 
 // One CTA per (128-token block, head, batch): x8 = round(x' / scale), x' = x - mean (K) or x (Q).
 template <int D, bool BF16, bool SMOOTH>
-__device__ __forceinline__ void quant_body(const uint16_t* __restrict__ x, long long sb, long long sh,
-                                           long long sn, int N, const float* __restrict__ partial,
+__device__ __forceinline__ void quant_body(const uint16_t* x, long long sb, long long sh,
+                                           long long sn, int N, const float* partial,
                                            int n_chunks, int8_t* __restrict__ x8,
                                            float* __restrict__ scale_out, float fold,
                                            float* __restrict__ mean_out, int blk, int h, int b, int H,
@@ -186,9 +188,9 @@ __device__ __forceinline__ void quant_body(const uint16_t* __restrict__ x, long 
 // partial column sums of K.  The first gridDim.x - q_blocks blocks sum K, the rest quantise Q.
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
-prepass_stage1_kernel(const uint16_t* __restrict__ q, long long qsb, long long qsh, long long qsn, int Nq,
+prepass_stage1_kernel(const uint16_t* q, long long qsb, long long qsh, long long qsn, int Nq,
                       int Hq, int nqb, int8_t* __restrict__ q8, float* __restrict__ sq, float fold,
-                      const uint16_t* __restrict__ k, long long ksb, long long ksh, long long ksn, int Nk,
+                      const uint16_t* k, long long ksb, long long ksh, long long ksn, int Nk,
                       int Hkv, int nch, float* __restrict__ partial, int q_blocks) {
   // This launch may start while the kernel before it drains (an earlier call's attention still reads the
   // buffers written here).  The dependent launch (stage 2) may start as soon as every CTA of this grid is
@@ -211,8 +213,8 @@ prepass_stage1_kernel(const uint16_t* __restrict__ q, long long qsb, long long q
 // Stage 2: smooth and quantise K (needs every column sum of stage 1).
 template <int D, bool BF16>
 __global__ void __launch_bounds__(256)
-quant_k_kernel(const uint16_t* __restrict__ k, long long sb, long long sh, long long sn, int N,
-               const float* __restrict__ partial, int n_chunks, int8_t* __restrict__ k8,
+quant_k_kernel(const uint16_t* k, long long sb, long long sh, long long sn, int N,
+               const float* partial, int n_chunks, int8_t* __restrict__ k8,
                float* __restrict__ scale_out, float* __restrict__ mean_out) {
   quant_body<D, BF16, true>(k, sb, sh, sn, N, partial, n_chunks, k8, scale_out, 1.0f, mean_out,
                             blockIdx.x, blockIdx.y, blockIdx.z, gridDim.y, gridDim.x);
