@@ -137,8 +137,15 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p);
 int miniattn_fwd_balanced(const MiniAttnFwdParams* p, void* scratch, size_t scratch_bytes, void* stream);
 
 /* Bytes of scratch the balanced launch of `p` needs on the current device (0: it would run the
- * plain launch); a negative MINIATTN_E* code on error. */
+ * plain launch); a negative MINIATTN_E* code on error.  Enough for miniattn_fwd_balanced(p) and for
+ * miniattn_fwd_int8qk_balanced alike, so it looks at both launches. */
 int64_t miniattn_fwd_balanced_scratch_bytes(const MiniAttnFwdParams* p);
+
+/* The same for one of the two: int8qk = 0 for miniattn_fwd_balanced, 1 for
+ * miniattn_fwd_int8qk_balanced (p = its fwd member).  Nothing else is planned, which is what a caller
+ * whose sizes change from call to call wants: sizing a decode call takes no plan at all.  sm_count as
+ * for miniattn_plan_fwd (<= 0: the current device's).  Pointers in `p` are not read. */
+int64_t miniattn_fwd_scratch_bytes(const MiniAttnFwdParams* p, int32_t int8qk, int sm_count);
 
 /* The plan itself, for inspection and tests: host arithmetic only, no device call when
  * sm_count > 0 (sm_count <= 0 asks the current device).  Pointers in `p` are not read. */
@@ -200,7 +207,8 @@ int miniattn_quant_qk_int8(const MiniAttnInt8Params* p, void* stream);
 int miniattn_fwd_int8qk(const MiniAttnInt8Params* p, void* stream);
 
 /* The INT8-QK attention kernel through the balanced launch: same scratch contract and the same
- * plan as miniattn_fwd_balanced (size it with miniattn_fwd_balanced_scratch_bytes(&p->fwd)). */
+ * plan as miniattn_fwd_balanced, with one query head per Q tile (size it with
+ * miniattn_fwd_balanced_scratch_bytes(&p->fwd) or miniattn_fwd_scratch_bytes(&p->fwd, 1, 0)). */
 int miniattn_fwd_int8qk_balanced(const MiniAttnInt8Params* p, void* scratch, size_t scratch_bytes, void* stream);
 
 /*

@@ -30,6 +30,7 @@ cudaError_t launch_fwd_decode(int D, bool bf16, const CUtensorMap* tm, const Dec
                               cudaStream_t st);
 void plan_decode(int B, int Hq, int Hkv, int Nq, int Nk, int D, int causal, long long diag, int sms, bool cut,
                  DecodePlan* d);
+bool plan_considered(const FwdArgs& a, int sms);
 void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan);
 cudaError_t launch_quant_qk(int D, bool bf16, const void* q, const long long* qs, const void* k,
                             const long long* ks, int B, int Hq, int Hkv, int Nq, int Nk, float q_fold,
@@ -366,8 +367,10 @@ static int check_device(int* sms) {
   return MINIATTN_OK;
 }
 
-// Plans of recent shapes (planning costs up to a millisecond of host time; launches of one shape
-// repeat).  Guarded by a mutex; an entry is copied out under the lock.
+// Plans of recent shapes (planning costs up to a few milliseconds of host time; launches of one shape repeat).
+// A plan depends on the sizes only through the K/V tiles that each pair of Q tiles visits, so a call whose sizes
+// are new is looked up a second time by those: while a context grows a token at a time, 128 calls share a plan.
+// Guarded by a mutex; what is handed out is shared and never changed.
 namespace {
 struct PlanKey {
   int Nq, Nk, B, Hq, causal, D, sms, group, pack;
@@ -378,24 +381,46 @@ struct PlanKey {
   }
 };
 struct PlanSlot {
-  PlanKey key;
+  PlanKey key;              // the sizes it was last used for
+  std::vector<int> tiles;   // of each pair
   std::shared_ptr<const ma::FwdPlan> plan;
+  bool serves(const PlanKey& k, const std::vector<int>& t) const {
+    return static_cast<long long>(key.B) * key.Hq == static_cast<long long>(k.B) * k.Hq && key.D == k.D &&
+           key.sms == k.sms && key.group == k.group && tiles == t;
+  }
 };
+constexpr size_t kPlanSlots = 64;
 std::shared_ptr<const ma::FwdPlan> cached_plan(const ma::FwdArgs& a, int D, int sms) {
   static std::mutex mu;
   static std::vector<PlanSlot> cache;
   static size_t next = 0;
+  static const auto never_cut = std::make_shared<const ma::FwdPlan>(ma::FwdPlan{});
+  if (!ma::plan_considered(a, sms)) return never_cut;
   const PlanKey key{a.Nq, a.Nk, a.B, a.Hq, a.causal, D, sms, a.bh_group, a.pack, a.causal ? a.q_pos0 - a.k_pos0 : 0};
   {
     std::lock_guard<std::mutex> g(mu);
     for (const PlanSlot& s : cache)
       if (s.key == key) return s.plan;
   }
+  std::vector<int> tiles((a.n_q_tiles + 1) / 2);
+  for (size_t i = 0; i < tiles.size(); ++i) {
+    const int q0 = static_cast<int>(i) * 2 * a.tpt;
+    tiles[i] = ma::kv_tiles_of(a, q0, q0 + a.tpt < a.Nq ? 2 : 1);
+  }
+  {
+    std::lock_guard<std::mutex> g(mu);
+    for (PlanSlot& s : cache)
+      if (s.serves(key, tiles)) {
+        s.key = key;
+        return s.plan;
+      }
+  }
   auto plan = std::make_shared<ma::FwdPlan>();
   ma::plan_fwd(a, D, sms, plan.get());
   std::lock_guard<std::mutex> g(mu);
-  if (cache.size() < 16) cache.push_back(PlanSlot{key, plan});
-  else cache[next++ % 16] = PlanSlot{key, plan};
+  PlanSlot slot{key, std::move(tiles), plan};
+  if (cache.size() < kPlanSlots) cache.push_back(std::move(slot));
+  else cache[next++ % kPlanSlots] = std::move(slot);
   return plan;
 }
 
@@ -571,23 +596,25 @@ int miniattn_fwd_balanced(const MiniAttnFwdParams* p, void* scratch, size_t scra
   return fwd_common(p, scratch, scratch_bytes, stream);
 }
 
-// Plan of a forward launch for `sm_count` SMs (<= 0: the current device's).  Host arithmetic only.
-static int plan_info_of(const MiniAttnFwdParams* p, bool may_pack, int sm_count, MiniAttnPlanInfo* info,
-                        MiniAttnPlanPiece* pieces, int32_t cap) {
-  g_err[0] = 0;
-  if (info == nullptr) return fail(MINIATTN_EINVAL, "info is null");
-  memset(info, 0, sizeof(*info));
+static int check_plan_params(const MiniAttnFwdParams* p, int sm_count, int* sms) {
   if (p == nullptr) return fail(MINIATTN_EINVAL, "params is null");
   if (p->D != 64 && p->D != 96 && p->D != 128)
     return fail(MINIATTN_EUNSUPPORTED, "head dim %d not supported (64, 96 or 128)", p->D);
   if (p->B < 0 || p->Hq < 0 || p->Nq < 0 || p->Nk < 0) return fail(MINIATTN_EINVAL, "negative size");
   if (p->Hq > 65535 || p->B > 65535)
     return fail(MINIATTN_EUNSUPPORTED, "B and Hq must not exceed 65535");
-  int sms = sm_count;
-  if (sms <= 0) {
-    int rc;
-    if ((rc = check_device(&sms)) != 0) return rc;
-  }
+  *sms = sm_count;
+  return sm_count > 0 ? MINIATTN_OK : check_device(sms);
+}
+
+// Plan of a forward launch for `sm_count` SMs (<= 0: the current device's).  Host arithmetic only.
+static int plan_info_of(const MiniAttnFwdParams* p, bool may_pack, int sm_count, MiniAttnPlanInfo* info,
+                        MiniAttnPlanPiece* pieces, int32_t cap) {
+  g_err[0] = 0;
+  if (info == nullptr) return fail(MINIATTN_EINVAL, "info is null");
+  memset(info, 0, sizeof(*info));
+  int sms = 0, rc;
+  if ((rc = check_plan_params(p, sm_count, &sms)) != 0) return rc;
   ma::FwdArgs a;
   fill_args(p, &a, may_pack ? head_pack(p) : 1);
   const long long n_items = static_cast<long long>((a.n_q_tiles + 1) / 2) * a.Hq * p->B;
@@ -637,16 +664,25 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p) {
   return tiles * ma::kTileM * (kernel_head_dim(p->D) * 4 + 8);
 }
 
+int64_t miniattn_fwd_scratch_bytes(const MiniAttnFwdParams* p, int32_t int8qk, int sm_count) {
+  g_err[0] = 0;
+  int sms = 0, rc;
+  if ((rc = check_plan_params(p, sm_count, &sms)) != 0) return rc;
+  if (!int8qk) {  // a call for the few-rows kernel needs no plan of the general one: a decode loop never makes any
+    ma::DecodePlan dec;
+    decode_plan_of(p, sms, true, &dec);
+    if (dec.rg != 0) return static_cast<int64_t>(decode_scratch_bytes(dec, p->D));
+  }
+  MiniAttnPlanInfo info;
+  if ((rc = plan_info_of(p, !int8qk, sms, &info, nullptr, 0)) != 0) return rc;  // INT8-QK does not pack heads
+  return info.scratch_bytes;
+}
+
 int64_t miniattn_fwd_balanced_scratch_bytes(const MiniAttnFwdParams* p) {
-  MiniAttnPlanInfo info, unpacked;
-  int rc = miniattn_plan_fwd(p, 0, &info, nullptr, 0);
-  if (rc != 0) return rc;
-  // the largest need of the launches that size their scratch with this call: the general kernel, the
-  // INT8-QK one (which does not pack heads), and the one for few rows
-  if ((rc = plan_info_of(p, false, info.sm_count, &unpacked, nullptr, 0)) != 0) return rc;
-  ma::DecodePlan dec;
-  decode_plan_of(p, info.sm_count, true, &dec);
-  return std::max({info.scratch_bytes, unpacked.scratch_bytes, static_cast<int64_t>(decode_scratch_bytes(dec, p->D))});
+  const int64_t plain = miniattn_fwd_scratch_bytes(p, 0, 0);
+  if (plain < 0 || p->D == 96) return plain;
+  const int64_t int8 = miniattn_fwd_scratch_bytes(p, 1, 0);
+  return int8 < 0 ? int8 : std::max(plain, int8);
 }
 
 static int check_int8_params(const MiniAttnInt8Params* p, bool need_v) {

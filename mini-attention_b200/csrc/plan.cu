@@ -151,17 +151,20 @@ bool fill(const std::vector<int>& w, int sms, float T, float h, float fee, int l
 
 }  // namespace
 
+// Many rounds balance themselves; the table holds every CTA from the first cut item on.
+bool plan_considered(const FwdArgs& a, int sms) {
+  const long long n_items = static_cast<long long>((a.n_q_tiles + 1) / 2) * a.Hq * a.B;
+  return sms > 0 && n_items > 0 && n_items <= 16ll * sms && n_items <= 4096;
+}
+
 // Items in launch order (item_to_pair_bh): latest rows first within each group of heads.
 void plan_fwd(const FwdArgs& a, int D, int sms, FwdPlan* plan) {
   plan->split = false;
   plan->n_whole = plan->n_table = plan->n_slots = plan->n_cut_items = 0;
   plan->est_plain = plan->est_balanced = 0.f;
+  if (!plan_considered(a, sms)) return;
   const long long n_pairs = (a.n_q_tiles + 1) / 2;
-  const long long bh = static_cast<long long>(a.Hq) * a.B;
-  const long long n_items = n_pairs * bh;
-  // Many rounds balance themselves; the table holds every CTA from the first cut item on.
-  if (sms <= 0 || n_items <= 0 || n_items > 16ll * sms || n_items > 4096) return;
-  const int n = static_cast<int>(n_items);
+  const int n = static_cast<int>(n_pairs * a.Hq * a.B);
   const float h = cta_cost(D);
   const float fee = piece_cost();
 

@@ -87,6 +87,8 @@ def _load() -> C.CDLL:
     lib.miniattn_fwd_balanced.restype = C.c_int
     lib.miniattn_fwd_balanced_scratch_bytes.argtypes = [C.POINTER(FwdParams)]
     lib.miniattn_fwd_balanced_scratch_bytes.restype = C.c_int64
+    lib.miniattn_fwd_scratch_bytes.argtypes = [C.POINTER(FwdParams), C.c_int32, C.c_int]
+    lib.miniattn_fwd_scratch_bytes.restype = C.c_int64
     lib.miniattn_fwd_carry_bytes.argtypes = [C.POINTER(FwdParams)]
     lib.miniattn_fwd_carry_bytes.restype = C.c_int64
     lib.miniattn_plan_fwd.argtypes = [C.POINTER(FwdParams), C.c_int, C.POINTER(PlanInfo),

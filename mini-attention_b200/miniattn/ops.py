@@ -259,9 +259,9 @@ def flash_attn_fwd(
         need = 0
         if p is not None and balance and not use_carry:
             with torch.cuda.device(q.device):
-                need = int(_lib.lib.miniattn_fwd_balanced_scratch_bytes(C.byref(p)))
+                need = int(_lib.lib.miniattn_fwd_scratch_bytes(C.byref(p), 0, 0))
             if need < 0:
-                _lib.check(need, "miniattn_fwd_balanced_scratch_bytes")
+                _lib.check(need, "miniattn_fwd_scratch_bytes")
         # a freshly allocated output keeps the same strides from call to call (torch.empty_like)
         if p is not None and key is not None and (out_given or out is None or out.stride() == q.stride()):
             if len(_param_cache) >= _PARAM_CACHE_MAX:
@@ -365,9 +365,9 @@ def flash_attn_fwd_int8qk(
         if quantize:
             _lib.check(_lib.lib.miniattn_quant_qk_int8(C.byref(p8), C.c_void_p(stream)), "miniattn_quant_qk_int8")
         if attend:
-            need = _lib.lib.miniattn_fwd_balanced_scratch_bytes(C.byref(p)) if balance else 0
+            need = _lib.lib.miniattn_fwd_scratch_bytes(C.byref(p), 1, 0) if balance else 0
             if need < 0:
-                _lib.check(int(need), "miniattn_fwd_balanced_scratch_bytes")
+                _lib.check(int(need), "miniattn_fwd_scratch_bytes")
             if need > 0:
                 scratch = _scratch_for(q.device, stream, int(need))
                 rc = _lib.lib.miniattn_fwd_int8qk_balanced(C.byref(p8), C.c_void_p(scratch.data_ptr()),
@@ -420,9 +420,9 @@ class HostPipeline:
             for b, h0, h1 in self.chunks:
                 p, _, _ = _prepare(self.qd[b:b + 1, h0 * G:h1 * G], self.kd[b:b + 1, h0:h1], self.vd[b:b + 1, h0:h1],
                                    causal, softmax_scale, "bhnd", False, self.od[b:b + 1, h0 * G:h1 * G], kernel, 0, 0)
-                n = _lib.lib.miniattn_fwd_balanced_scratch_bytes(C.byref(p))
+                n = _lib.lib.miniattn_fwd_scratch_bytes(C.byref(p), 0, 0)
                 if n < 0:
-                    _lib.check(int(n), "miniattn_fwd_balanced_scratch_bytes")
+                    _lib.check(int(n), "miniattn_fwd_scratch_bytes")
                 need = max(need, int(n))
                 blocks.append(p)
             entry = self._launches[key] = (blocks, need)

@@ -151,3 +151,65 @@ def test_plan_entry_rejects_bad_arguments():
     assert _lib.lib.miniattn_plan_fwd(C.byref(p), 148, None, None, 0) == _lib.EINVAL
     p.Nq = -1
     assert _lib.lib.miniattn_plan_fwd(C.byref(p), 148, C.byref(info), None, 0) == _lib.EINVAL
+
+
+def _fwd_params(B, Hq, Hkv, Nq, Nk, D, causal=True):
+    from miniattn import _lib
+    p = _lib.FwdParams()
+    p.B, p.Hq, p.Hkv, p.Nq, p.Nk, p.D, p.causal = B, Hq, Hkv, Nq, Nk, D, int(causal)
+    p.q_pos0 = Nk - Nq if causal else 0
+    return p
+
+
+def _scratch(p, int8qk=0):
+    import ctypes as C
+    from miniattn import _lib
+    need = _lib.lib.miniattn_fwd_scratch_bytes(C.byref(p), int8qk, SMS)
+    assert need >= 0
+    return need
+
+
+def test_a_growing_context_is_not_planned_for_at_every_token():
+    """Sizing the scratch of a decode call makes no plan of the general kernel; sizing an INT8-QK one, or a general
+    call of a few hundred rows, makes one for each new count of K/V tiles.  A plan takes 0.5 to 4 ms: two thousand
+    of them take seconds, and the bound is a tenth of one."""
+    import time
+    t0 = time.perf_counter()
+    needs = {_scratch(_fwd_params(16, 32, 8, 1, 4001 + i, 128)) for i in range(2000)}
+    assert max(needs) > 0 and time.perf_counter() - t0 < 0.1
+    t0 = time.perf_counter()
+    for i in range(2000):                       # 16 counts of tiles
+        _scratch(_fwd_params(2, 8, 8, 600, 4001 + i, 64, causal=False), i % 2)
+    assert time.perf_counter() - t0 < 0.5
+
+
+def test_plans_of_the_same_tiles_are_the_same():
+    """Key counts inside one 128-key tile visit the same tiles; across the boundary they do not."""
+    a, b, c = (plan_info(1, 6, 1024, nk, 128, sm_count=SMS) for nk in (4001, 4096, 4097))
+    assert a[0].split and a[1] == b[1] and a[0].scratch_bytes == b[0].scratch_bytes
+    assert a[1] != c[1]
+    d, e = (plan_info(b_, h, 1024, 4096, 128, sm_count=SMS) for b_, h in ((2, 3), (1, 6)))
+    assert d[1] == e[1]                         # the items are the same, whatever B and H are one by one
+
+
+def test_scratch_of_either_launch():
+    """Decode: the pieces of the few-rows kernel.  INT8-QK: the general kernel's plan without packed heads."""
+    p = _fwd_params(2, 24, 8, 777, 3333, 128)
+    assert _scratch(p, 1) == plan_info(2, 24, 777, 3333, 128, causal=True, q_pos0=3333 - 777, sm_count=SMS)[0].scratch_bytes
+    q = _fwd_params(1, 8, 1, 1, 8192, 128)
+    assert 16384 < _scratch(q) < 16384 + 2 * 2 * SMS * 16 * (8 + 4 * 128)
+    assert _scratch(q, 1) == plan_info(1, 8, 1, 8192, 128, causal=True, q_pos0=8191, sm_count=SMS)[0].scratch_bytes
+    q.carry_in = 1
+    assert _scratch(q) == 0
+
+
+def test_more_shapes_in_rotation_than_a_handful():
+    import time
+    shapes = [_fwd_params(1, 12, 4, 500 + 64 * i, 3000, 128) for i in range(40)]
+    t = []
+    for _ in range(2):
+        t0 = time.perf_counter()
+        for p in shapes:
+            _scratch(p)
+        t.append(time.perf_counter() - t0)
+    assert t[1] < t[0] / 4
