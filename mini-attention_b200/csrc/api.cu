@@ -292,6 +292,25 @@ static int head_group(const MiniAttnFwdParams* p, int pack) {
   return static_cast<int>(d * g);
 }
 
+// K/V tiles that the first n pairs of Q tiles visit together: the sum of kv_tiles_of, in at most 128 steps however
+// many pairs there are (one Q tile holds a single token where 128 heads share it).  Pair i ends at key end0 + step * i,
+// so pairs 128 apart differ by step tiles exactly.
+static long long kv_tiles_of_pairs(const ma::FwdArgs& a, long long n) {
+  const long long all = (static_cast<long long>(a.Nk) + ma::kTileN - 1) / ma::kTileN;
+  if (!a.causal) return n * all;
+  const long long step = 2 * a.tpt, end0 = a.q_pos0 - a.k_pos0 + step;
+  auto first_at = [&](long long key) {  // first pair that ends at `key` or later
+    return std::clamp<long long>(end0 >= key ? 0 : (key - end0 + step - 1) / step, 0, n);
+  };
+  const long long lo = first_at(1), hi = first_at(a.Nk);  // pairs before lo see nothing, those from hi on every key
+  long long sum = (n - hi) * all;
+  for (long long i = lo; i < std::min(lo + ma::kTileN, hi); ++i) {
+    const long long times = (hi - i + ma::kTileN - 1) / ma::kTileN;  // pairs i, i + 128, ... before hi
+    sum += times * ((end0 + step * i + ma::kTileN - 1) / ma::kTileN) + step * (times * (times - 1) / 2);
+  }
+  return sum;
+}
+
 // Query heads that share a Q tile: all G heads of a KV head, or 1.  Packed, a tile holds 128 / G tokens of
 // each head: the tail of a token count that is no multiple of 128 is padded once per KV head instead of once
 // per query head, and under a causal mask a pair of tiles spans 256 / G tokens, so that its rows share more
@@ -315,12 +334,10 @@ static int head_pack(const MiniAttnFwdParams* p) {
     a.k_pos0 = p->k_pos0;
     a.tpt = ma::kTileM / (packed ? g : 1);
     const int n_tiles = (p->Nq + a.tpt - 1) / a.tpt;
-    visits[packed] = 0;
-    for (int t = 0; t < n_tiles; t += 2) {
-      const int nt = t + 1 < n_tiles ? 2 : 1;
-      // a step of a tile alone takes two thirds of a pair's (2000 and 2950 clk)
-      visits[packed] += (nt == 2 ? 3 : 2) * static_cast<long long>(ma::kv_tiles_of(a, t * a.tpt, nt));
-    }
+    const int last = (n_tiles - 1) / 2, last_nt = n_tiles - 2 * last;
+    // a step of a tile alone takes two thirds of a pair's (2000 and 2950 clk)
+    visits[packed] = 3 * kv_tiles_of_pairs(a, last) +
+                     (last_nt == 2 ? 3 : 2) * static_cast<long long>(ma::kv_tiles_of(a, last * 2 * a.tpt, last_nt));
     if (!packed) visits[0] *= g;
   }
   return visits[1] * 100 <= visits[0] * 99 ? g : 1;

@@ -213,3 +213,62 @@ def test_more_shapes_in_rotation_than_a_handful():
             _scratch(p)
         t.append(time.perf_counter() - t0)
     assert t[1] < t[0] / 4
+
+
+def _packs(B, Hkv, G, Nq, Nk, causal, q_pos0):
+    """Whether the rule packs the G heads, read off the number of work items (G = 1 or 0 pairs apart: unknown)."""
+    import ctypes as C
+    from miniattn import _lib
+    p = _fwd_params(B, Hkv * G, Hkv, Nq, Nk, 128, causal)
+    p.q_pos0, p.carry_in = q_pos0, 0
+    p.B = 65535                                  # too many items to plan: n_ctas is their number
+    info = _lib.PlanInfo()
+    _lib.check(_lib.lib.miniattn_plan_fwd(C.byref(p), SMS, C.byref(info), None, 0), "plan")
+    plain = (((Nq + 127) // 128 + 1) // 2) * Hkv * G
+    tpt = 128 // G
+    packed = (((Nq + tpt - 1) // tpt + 1) // 2) * Hkv
+    items = info.n_ctas // 65535
+    assert items in (plain, packed)
+    return None if plain == packed else items == packed
+
+
+def _rule(G, Nq, Nk, causal, pos):
+    """The rule stated pair by pair: packed where that saves at least 1 % of the weighted K/V tiles."""
+    def visits(tpt):
+        n, s = -(-Nq // tpt), 0
+        for t in range(0, n, 2):
+            nt = 2 if t + 1 < n else 1
+            end = Nk if not causal else max(0, min(Nk, pos + min((t + nt) * tpt, Nq)))
+            s += (3 if nt == 2 else 2) * -(-end // 128)
+        return s
+    return visits(128 // G) * 100 <= visits(128) * G * 99
+
+
+def test_head_packing_rule_in_closed_form():
+    import random
+    rng = random.Random(5)
+    seen = [0, 0]
+    for _ in range(3000):
+        G = rng.choice([2, 3, 4, 5, 7, 8, 16, 48, 64, 128])
+        Nq, Nk = (int(2 ** rng.uniform(0, 15)) for _ in range(2))
+        causal = rng.random() < 0.8
+        pos = rng.choice([0, Nk - Nq, rng.randrange(-Nq - 300, Nk + 300)]) if causal else 0
+        got = _packs(1, 1, G, Nq, Nk, causal, pos)
+        if got is not None:
+            assert got == _rule(G, Nq, Nk, causal, pos), (G, Nq, Nk, causal, pos)
+            seen[got] += 1
+    assert min(seen) > 200
+
+
+def test_head_packing_rule_takes_no_time_over_many_pairs():
+    """128 heads share a KV head: a Q tile holds one token and 131072 rows have 65536 pairs.  A walk over them took
+    150 us a call; the bound is a fifth of that."""
+    import ctypes as C
+    import time
+    from miniattn import _lib
+    p = _fwd_params(1, 128, 1, 131072, 131072, 128)
+    info = _lib.PlanInfo()
+    t0 = time.perf_counter()
+    for _ in range(1000):
+        _lib.lib.miniattn_plan_fwd(C.byref(p), SMS, C.byref(info), None, 0)
+    assert time.perf_counter() - t0 < 0.03
