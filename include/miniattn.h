@@ -125,8 +125,8 @@ int64_t miniattn_fwd_carry_bytes(const MiniAttnFwdParams* p);
  *
  * A call with few query rows per KV head (decode: see plan_decode, csrc/plan.cu) runs another
  * kernel under MINIATTN_KERNEL_AUTO, with and without scratch; with it, the key range of its items
- * is cut over CTAs by the same contract, and no CTA waits for another.  miniattn_plan_fwd below
- * describes the general kernel's launch.
+ * is cut over CTAs by the same contract, and no CTA waits for another.  Scratch that is too small
+ * for its pieces sends the call to the general kernel, whose launch miniattn_plan_fwd describes.
  *
  * scratch: device memory, 256-byte aligned, at least miniattn_fwd_balanced_scratch_bytes(p)
  * bytes.  Its first 16384 bytes (the arrival counters) must be zero before the first launch that

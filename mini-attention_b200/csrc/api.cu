@@ -481,8 +481,8 @@ static size_t decode_scratch_bytes(const ma::DecodePlan& d, int D) {
   return kCounterBytes + align256(rows * sizeof(float2)) + rows * kernel_head_dim(D) * sizeof(float);
 }
 
-static int fwd_decode(const MiniAttnFwdParams* p, const ma::DecodePlan& d, void* scratch, size_t scratch_bytes,
-                      cudaStream_t st) {
+// scratch: decode_scratch_bytes(d, p->D) bytes, 256-byte aligned; null where that is 0.
+static int fwd_decode(const MiniAttnFwdParams* p, const ma::DecodePlan& d, void* scratch, cudaStream_t st) {
   const CUtensorMapDataType dt =
       p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   CUtensorMap tm[2];
@@ -513,13 +513,7 @@ static int fwd_decode(const MiniAttnFwdParams* p, const ma::DecodePlan& d, void*
   a.n_rb = d.n_rb;
   a.tiles = d.tiles;
   a.scale_log2 = (p->softmax_scale > 0.f ? p->softmax_scale : 1.0f / sqrtf((float)p->D)) * 1.4426950408889634f;
-  const size_t need = decode_scratch_bytes(d, p->D);
-  if (need > 0) {
-    if (scratch_bytes < need)
-      return fail(MINIATTN_EINVAL, "scratch holds %zu bytes, this launch needs %zu "
-                  "(miniattn_fwd_balanced_scratch_bytes)", scratch_bytes, need);
-    if (reinterpret_cast<uintptr_t>(scratch) % 256 != 0)
-      return fail(MINIATTN_EINVAL, "scratch must be 256-byte aligned");
+  if (scratch != nullptr) {
     uint8_t* base = static_cast<uint8_t*>(scratch);
     const size_t rows = static_cast<size_t>(2 * d.n_ctas) * 16 * d.rg;
     a.counters = reinterpret_cast<int*>(base);
@@ -542,7 +536,11 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   if ((rc = check_device(&sms)) != 0) return rc;
   ma::DecodePlan dec;
   decode_plan_of(p, sms, scratch != nullptr, &dec);
-  if (dec.rg != 0) return fwd_decode(p, dec, scratch, scratch_bytes, reinterpret_cast<cudaStream_t>(stream));
+  // Scratch that does not hold the pieces of the few-rows kernel may still do for the general one, which often
+  // needs none (a caller may have sized it by miniattn_plan_fwd): the call runs there, or is refused there.
+  const size_t dec_need = decode_scratch_bytes(dec, p->D);
+  if (dec.rg != 0 && (dec_need == 0 || (scratch_bytes >= dec_need && reinterpret_cast<uintptr_t>(scratch) % 256 == 0)))
+    return fwd_decode(p, dec, dec_need > 0 ? scratch : nullptr, reinterpret_cast<cudaStream_t>(stream));
 
   const CUtensorMapDataType dt =
       p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;

@@ -101,3 +101,37 @@ def test_captured_calls_have_scratch_of_their_own():
     for o, w in zip(outs, want):
         assert (o.float() - w.float()).abs().max().item() <= 2.0 ** -10  # fp32 order of the folds, one rounding
     assert miniattn.device_status(DEV) == 0
+
+
+def test_scratch_too_small_for_the_pieces():
+    """A caller's scratch that does for the general kernel's launch does for the call, whichever kernel the call would
+    rather have: what needs no scratch there is taken with any, what needs some is refused below that."""
+    import ctypes as C
+
+    from miniattn import _lib
+    from miniattn.ops import _prepare
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    buf = torch.zeros(64 << 20, dtype=torch.uint8, device=DEV)
+    for B, Hq, Hkv, Nq, Nk, D in ((2, 8, 8, 1, 1200, 128), (1, 8, 1, 2, 16384, 128), (4, 16, 4, 4, 1500, 64)):
+        q, k, v = make_inputs(B, Hq, Hkv, Nq, Nk, D, torch.float16, seed=Nk)
+        qd, kd, vd = q.to(DEV), k.to(DEV), v.to(DEV)
+        ref = attention_reference(q, k, v, out_dtype=torch.float32)
+        p, out, _ = _prepare(qd, kd, vd, False, None, "bhnd", False, None, "auto", 0, 0)
+        info = _lib.PlanInfo()
+        _lib.check(_lib.lib.miniattn_plan_fwd(C.byref(p), sms, C.byref(info), None, 0), "plan")
+        need, general = _lib.lib.miniattn_fwd_scratch_bytes(C.byref(p), 0, 0), info.scratch_bytes
+        assert need > 0
+        sizes = {need, need - 1, general, 0 if general == 0 else general - 1}
+        for size in sorted(sizes):
+            out.zero_()
+            rc = _lib.lib.miniattn_fwd_balanced(C.byref(p), C.c_void_p(buf.data_ptr()), C.c_size_t(size), stream)
+            assert (rc == _lib.OK) == (size >= min(need, general)), (size, need, general)
+            if rc == _lib.OK:
+                torch.cuda.synchronize()
+                assert (out.float().cpu() - ref).abs().max().item() <= TOL[torch.float16]
+        # a misaligned pointer: the same
+        rc = _lib.lib.miniattn_fwd_balanced(C.byref(p), C.c_void_p(buf.data_ptr() + 16), C.c_size_t(32 << 20), stream)
+        assert (rc == _lib.OK) == (general == 0)
+    torch.cuda.synchronize()
+    assert int(buf[:16384].view(torch.int32).abs().sum()) == 0 and miniattn.device_status(DEV) == 0
