@@ -292,49 +292,69 @@ void plan_decode(int B, int Hq, int Hkv, int Nq, int Nk, int D, int causal, long
   const int tiles = static_cast<int>((kv_end + 63) / 64);
   const long long total = items * tiles;
   const long long slots = 2ll * sms;  // two CTAs per SM
-  // Which kernel.  Measured on B200 (us, fwd_ws / this one, bf16, causal, the last Nq of Nk positions):
-  //   up to 16 rows   bound by HBM here, never slower: 8x8 KV heads, D=128, Nk=4096: G=1 Nq=1 42 / 37,
-  //                   G=8 Nq=1 194 / 38; 1x2 KV heads, Nk=1024, G=1: 18.5 / 14.3
-  //   17 to 32 rows   a tile costs its warps about as long as HBM takes to deliver it: G=4 Nq=8, Nk=1024:
-  //                   1x2 KV heads 20.5 / 20.5, 8x8 36.9 / 24.6; but one query head (G=1 Nq=32, 8x8,
-  //                   Nk=4096) 42.0 / 45.1 at D=128, 33.8 / 30.8 at D=64
-  //   more            bound by mma.sync: a block of 64 rows takes as long as two tcgen05 tiles of fwd_ws,
-  //                   which needs one per query head (8x8, Nk=16384: G=2 Nq=32 189 / 150, G=8 Nq=32
-  //                   671 / 464, G=4 Nq=64 353 / 465), and only where there is work for every SM: fwd_ws cuts
-  //                   few long items better (1x2, G=8 Nq=8, Nk=4096: 27.8 / 43.0)
-  if (rg == 2 && G == 1 && D == 128) return;
-  if (rg == 4 && (G < 2 * n_rb || G * total < 16 * slots)) return;
-  d->rg = rg;
-  d->n_rb = static_cast<int>(n_rb);
-  d->tiles = tiles;
-  d->total = total;
-  if (!cut) {
-    d->n_ctas = static_cast<int>(items);
-    return;
-  }
-  // Pieces of an item: at least four tiles long, and no more than balances a tile's time against what the
-  // CTA that folds them spends on each (in us: a round trip to L2 shared by eight, and the piece's rows at
-  // what one SM reads).
+  // How the items are cut: pieces of at least four tiles, and no more of them than balances a tile's time against
+  // what the CTA that folds them spends on each (in us: a round trip to L2 shared by eight, and the piece's rows at
+  // what one SM reads).  An item of fewer than 12 tiles is left whole, of fewer than 10 where there are next to no
+  // rows to fold: a cut costs 1 to 2 us (128 items of 8 tiles, D = 128: 16 rows 12.7 us cut in two, 10.6 whole, 1 row
+  // 11.1 / 10.6; of 12 tiles 13.9 / 13.1 and 12.7 / 13.1; 36 items of 10 tiles, 1 row 10.5 / 11.3).
   const double t_tile = rg == 1 ? 0.5 : rg == 2 ? 0.8 : 1.5;
   const double t_fold = 0.02 + std::min<double>(rows, 16 * rg) * D * 4 / 55e3;
-  const long long most = std::max(1ll, std::min<long long>(tiles / 4, static_cast<long long>(std::sqrt(tiles * t_tile / t_fold))));
+  const bool too_short = tiles < (rows <= 4 ? 10 : 12);
+  const long long most =
+      too_short ? 1 : std::max(1ll, std::min<long long>(tiles / 4, static_cast<long long>(std::sqrt(tiles * t_tile / t_fold))));
   // A CTA works on one item only wherever that leaves enough of them: one that ends a piece of one item and
   // begins the next pays for two ends (about 5 us of syncs, publishing and folding) and so does the launch.
   // 16 items of 563 tiles, D = 64: 39.3 us in 292 CTAs that straddle, 31.9 in 288 of one piece each, 30.0 in
   // 256; 128 items of 63 tiles, D = 128: 49.0 in 296, 46.6 in 256; 512 items of 16 tiles: 49.5 in 296, 46.0 in
-  // 256 of two items each.  HBM is saturated by fewer CTAs than fit (208 to 272), and pieces cost; where the
-  // tiles are bound by mma.sync (rg > 1) every slot counts.
+  // 256 of two items each; 328 items of 2 tiles: 15.6 in 296, 11.9 in 328; 320 of 11 tiles, 32 rows: 33.5 in 296,
+  // 37.1 in 320.  HBM is saturated by fewer CTAs than fit (208 to 272), and pieces cost; where the tiles are bound by
+  // mma.sync (rg > 1) every slot counts: 400 items of 64 tiles, D = 64, 64 rows 138.8 in 200, 109.1 in 296.
   const long long room = rg == 1 ? slots * 7 / 8 : slots;
-  if (items <= room) {
-    d->n_ctas = static_cast<int>(items * std::max(1ll, std::min(most, room / items)));
-    return;
+  long long n_ctas = items;
+  if (cut && items <= room) {
+    n_ctas = items * std::max(1ll, std::min(most, room / items));
+  } else if (cut) {
+    const long long enough = rg == 1 ? slots * 2 / 3 : slots * 9 / 10;
+    long long j = (items + slots - 1) / slots;
+    while (items % j != 0 && items / j >= enough) ++j;
+    if (items / j >= enough) n_ctas = items / j;
+    else if (tiles >= 10 || items >= 4 * slots) n_ctas = slots;
   }
-  d->n_ctas = static_cast<int>(slots);
-  for (long long j = (items + slots - 1) / slots; items / j >= slots * 2 / 3; ++j)
-    if (items % j == 0) {
-      d->n_ctas = static_cast<int>(items / j);
-      return;
-    }
+  // Which kernel.  fwd_ws packs the query heads of a KV head into one Q tile (head_pack, api.cu), so that it too reads
+  // K/V once; its tile of 128 rows takes 1.05 us for 128 keys whatever part of the rows is real, on one CTA per SM.
+  // Measured on B200 (us, fwd_ws / this one, bf16, causal, the last Nq of Nk positions; balanced launches):
+  //   up to 16 rows   two CTAs an SM, bound by HBM: 1 KV head, Nk=16384 45 / 18; 32 of 4096 keys 23 / 16; 128 of 2048
+  //                   to 4096 within 5 % either way (27.4 / 28.2, 48.5 / 47.1), more items ahead (320 of 2048 69 / 58)
+  //   17 to 32 rows   at D=64 ahead wherever an item is cut (72 of 2048 18.7 / 14.7, 128 of 1024 14.3 / 13.5) and whole
+  //                   while it is short (512 keys 9.0 / 8.6, 16384 keys 137 / 143).  At D=128 a tile costs its warps
+  //                   about what HBM takes to deliver it.  Ahead: more items than SMs (fwd_ws goes another round: 320 of
+  //                   2048 71 / 67, of 512 whole 28 / 27); few items long enough to cut (1 of 4096 20.2 / 19.3, of 16384
+  //                   45 / 30; 32 of 2048 20.3 / 19.3); more than half an SM each and long (128 of 8192 91.6 / 89.3).
+  //                   Behind: 512 keys 9.4 / 12.3, 72 of 4096 34.5 / 35.6, 128 of 2048 27.9 / 32.4; all of them whole and
+  //                   long (1 of 16384 167 / 229).  One query head (G=1): fwd_ws.
+  //   more            bound by mma.sync, a block of 64 rows 1.5 us for 64 keys: behind where heads are packed (128 of
+  //                   4096, D=128: 64 rows 49.6 / 80.7, 256 rows 64.7 / 260; 32 of 4096, D=64 24 / 44), but for one block
+  //                   at D=64 in more items than SMs (320 of 1024 38.5 / 33.8, 192 of 300 16.4 / 12.3; 192 of 4096 whole
+  //                   67 / 78), and level for one or two items of 20000 keys and more (1 of 40000: D=64 60 / 54, D=128
+  //                   80 / 75; of 50000 50 / 57, 60 / 81).  More than 128 query heads to a KV head do not fit a Q
+  //                   tile: ahead where there is work for every SM (192 heads, 4 of 1671 128 / 26).
+  // A launch of one whole item per CTA needs no scratch, and a call without scratch can have no other: the line is the
+  // same for both.
+  const bool whole = n_ctas == items;
+  if (rg == 2 && D == 64 && whole && items <= sms && tiles > 16) return;
+  if (rg == 2 && D == 128) {
+    const bool few = 4 * items <= sms, half = 2 * items > sms;
+    if (G == 1) return;
+    if (items <= sms && (whole || tiles < 16 || !(few || (half && tiles >= 128)))) return;
+    if (items > slots && whole && !too_short) return;
+  }
+  if (rg == 4 && G <= kTileM && !(D == 64 && n_rb == 1 && items > sms && (tiles <= 16 || !whole))) return;
+  if (rg == 4 && G > kTileM && (G < 2 * n_rb || G * total < 16 * slots)) return;
+  d->rg = rg;
+  d->n_rb = static_cast<int>(n_rb);
+  d->tiles = tiles;
+  d->total = total;
+  d->n_ctas = static_cast<int>(n_ctas);
 }
 
 }  // namespace ma

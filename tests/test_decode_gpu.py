@@ -60,6 +60,22 @@ def test_matches_the_oracle_and_the_general_kernel(B, Hq, Hkv, Nq, Nk, D, causal
             assert (lse[finite] - ref_lse[finite]).abs().max().item() <= 1e-3
 
 
+# either side of the lines in plan_decode: whole and cut items (11 / 12 tiles of 64 keys), 32 rows of either head dim
+# (7 / 8 and 16 / 17 tiles whole, few / half / more items than SMs), query heads that fill a Q tile or more
+EDGES = [
+    (2, 2, 2, 1, 704, 128), (2, 2, 2, 1, 705, 128), (3, 8, 1, 4, 448, 64), (3, 8, 1, 4, 449, 64), (2, 24, 1, 1, 705, 64),
+    (1, 8, 2, 8, 960, 128), (1, 8, 2, 8, 961, 128), (4, 40, 10, 5, 1100, 128), (19, 16, 8, 9, 700, 128),
+    (1, 128, 1, 1, 9000, 128), (1, 129, 1, 1, 9500, 64), (2, 192, 1, 2, 2000, 128), (50, 129, 1, 1, 300, 64),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("balance", [True, False])
+@pytest.mark.parametrize("B,Hq,Hkv,Nq,Nk,D", EDGES)
+def test_either_side_of_a_line(B, Hq, Hkv, Nq, Nk, D, balance, dtype):
+    test_matches_the_oracle_and_the_general_kernel(B, Hq, Hkv, Nq, Nk, D, True, "bhnd", balance, dtype)
+
+
 def test_strided_views_and_output_views():
     """Heads and tokens picked out of wider tensors, the result into a view: no form is copied first."""
     g = torch.Generator().manual_seed(3)
