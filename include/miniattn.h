@@ -283,6 +283,11 @@ int miniattn_selftest_wait(int32_t* status, uint64_t limit_ns, void* stream);
  */
 int miniattn_check_status(int32_t status_word);
 
+/* Which capture the stream is part of: *id is the number CUDA gives it, different for every capture,
+ * and 0 when the stream is not being captured.  For callers that keep scratch by capture: a captured
+ * launch may be replayed beside anything, so it must not share the scratch of launches outside. */
+int miniattn_stream_capture_id(void* stream, uint64_t* id);
+
 /* Library / build identification: "miniattn-b200 <version> sm_100a". */
 const char* miniattn_version(void);
 

@@ -877,6 +877,18 @@ int miniattn_check_status(int32_t status_word) {
   return fail(MINIATTN_EDEVICE_WAIT, "bounded device waits ran out (status word 0x%x): %s", status_word, list);
 }
 
+int miniattn_stream_capture_id(void* stream, uint64_t* id) {
+  g_err[0] = 0;
+  if (id == nullptr) return fail(MINIATTN_EINVAL, "id is null");
+  *id = 0;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long n = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo(reinterpret_cast<cudaStream_t>(stream), &status, &n);
+  if (e != cudaSuccess) return fail(MINIATTN_ECUDA, "cudaStreamGetCaptureInfo: %s", cudaGetErrorString(e));
+  if (status != cudaStreamCaptureStatusNone) *id = n;
+  return MINIATTN_OK;
+}
+
 int miniattn_selftest_wait(int32_t* status, uint64_t limit_ns, void* stream) {
   g_err[0] = 0;
   if (status == nullptr) return fail(MINIATTN_EINVAL, "status is null");

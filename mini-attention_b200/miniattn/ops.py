@@ -20,6 +20,7 @@ _DTYPES = {torch.float16: _lib.FP16, torch.bfloat16: _lib.BF16}
 _status_words: dict = {}
 _COUNTER_BYTES = 16384        # arrival counters at the start of a balanced launch's scratch
 _balance_scratch: dict = {}   # (device index, stream) -> zero-initialised uint8 scratch tensor
+_capture_scratch: dict = {}   # the same for the last capture on that stream: (capture id, scratch of the graph)
 # Parameter blocks of recent calls, keyed by everything that goes into one (pointers, shapes, strides,
 # dtype, flags).  A training or serving loop calls the operator with the same tensors again and again;
 # validating and filling the block costs more host time than a short-sequence kernel runs for.
@@ -67,13 +68,19 @@ def check_device_status(device: Union[torch.device, str, None] = None) -> None:
 def _scratch_for(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
     """Scratch of a balanced launch: one buffer per (device, stream), zeroed when created (the
     kernels leave the arrival counters at its start zero again), grown on demand.  A call that is being
-    captured gets a buffer of its own from the graph's memory, its counters cleared by the graph: a
-    captured launch may be replayed on any stream."""
-    if torch.cuda.is_current_stream_capturing():
-        t = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        t[:_COUNTER_BYTES].zero_()
-        return t
+    captured gets one of the graph's own memory, since the graph may be replayed on any stream: one buffer
+    for all calls that one capture makes on a stream, its counters cleared by the graph before the first."""
     key = (device.index if device.index is not None else torch.cuda.current_device(), stream)
+    if torch.cuda.is_current_stream_capturing():
+        capture = C.c_uint64(0)
+        _lib.check(_lib.lib.miniattn_stream_capture_id(stream, C.byref(capture)), "miniattn_stream_capture_id")
+        held = _capture_scratch.get(key)
+        if held is not None and held[0] == capture.value and held[1].numel() >= nbytes:
+            return held[1]
+        t = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+        t[:_COUNTER_BYTES].zero_()
+        _capture_scratch[key] = (capture.value, t)
+        return t
     t = _balance_scratch.get(key)
     if t is None or t.numel() < nbytes:
         t = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)

@@ -151,3 +151,44 @@ def test_scratch_too_small_for_the_pieces():
         assert (rc == _lib.OK) == (general == 0)
     torch.cuda.synchronize()
     assert int(buf[:16384].view(torch.int32).abs().sum()) == 0 and miniattn.device_status(DEV) == 0
+
+
+def test_one_capture_keeps_one_scratch():
+    """The calls of one capture share a buffer that the graph clears once, and on another stream of the same capture
+    have another; a later capture has its own; none of them is the one that eager calls use."""
+    from miniattn import ops
+    q, k, v = (t.to(DEV) for t in make_inputs(2, 8, 2, 1, 6000, 128, torch.float16, seed=4))
+    want = miniattn.flash_attn_fwd(q, k, v)
+    dev, seen, outs = torch.device(DEV), [], []
+    side = torch.cuda.Stream()
+
+    def scratch():
+        return ops._scratch_for(dev, torch.cuda.current_stream().cuda_stream, 1 << 20).data_ptr()
+
+    graphs = []
+    for _ in range(2):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            ptrs = []
+            for _ in range(3):
+                outs.append(miniattn.flash_attn_fwd(q, k, v))
+                ptrs.append(scratch())
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                outs.append(miniattn.flash_attn_fwd(q, k, v))
+                other = scratch()
+            outs.append(miniattn.flash_attn_fwd(q, k, v))     # beside the one on the other stream
+            torch.cuda.current_stream().wait_stream(side)
+        assert len(set(ptrs)) == 1 and other != ptrs[0]
+        seen += [ptrs[0], other]
+        graphs.append(g)
+    assert len(set(seen + [scratch()])) == 5
+    for _ in range(20):
+        for o in outs:
+            o.zero_()
+        for g in graphs:
+            g.replay()
+        torch.cuda.synchronize()
+        for o in outs:
+            assert torch.equal(o, want)      # pieces are folded in order
+    assert miniattn.device_status(DEV) == 0
