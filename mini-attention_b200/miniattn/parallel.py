@@ -183,7 +183,7 @@ def ring_forward(
     bufs = [(torch.empty_like(k_cur), torch.empty_like(v_cur)) for _ in range(2 if world > 1 else 0)]
     q_blocks = (q_local[:, :, :L], q_local[:, :, L:])
     out = torch.empty_like(q_local)
-    if fused and world == 1 and L2 == 2 * L:
+    if fused and world == 1 and L2 == 2 * L == k_cur.shape[2]:
         # the two blocks of a ring of one are neighbours: one causal launch, no state to carry (three launches
         # otherwise, each with the tail of its own)
         from .ops import flash_attn_fwd

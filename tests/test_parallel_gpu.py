@@ -145,3 +145,14 @@ def test_ring_emulated_block_lengths(N, world):
     ref = attention_reference(q, k, v, causal=True, out_dtype=torch.float32)
     assert miniattn.device_status(DEV) == 0
     assert (out.float() - ref).abs().max().item() <= TOL[torch.float16]
+
+
+@pytest.mark.parametrize("causal", [False, True])
+def test_ring_of_one_takes_its_own_rows_of_a_longer_kv(causal):
+    """One rank whose K/V tensors go on behind its 2 L tokens: the rows see the two blocks and nothing after them,
+    as on any rank."""
+    q, k, v = make_inputs(1, 2, 2, 300, 364, 128, torch.float16, seed=7)
+    out = par.ring_forward(q.to(DEV), k.to(DEV), v.to(DEV), causal=causal).cpu()
+    ref = attention_reference(q, k[:, :, :300], v[:, :, :300], causal=causal, out_dtype=torch.float32)
+    assert (out.float() - ref).abs().max().item() <= TOL[torch.float16]
+    assert miniattn.device_status(DEV) == 0
