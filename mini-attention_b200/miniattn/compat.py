@@ -75,6 +75,11 @@ ext = _Ext()
 def forward(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor) -> torch.Tensor:
     """Flash attention forward. q/k/v: (B, N, H, D) fp16 or bf16 CUDA tensors; non-causal,
     softmax scale 1/sqrt(D) (the reference operator's fixed behaviour)."""
+    dt, shape = q.dtype, q.shape
+    if (q.is_cuda and k.is_cuda and v.is_cuda and (dt is torch.float16 or dt is torch.bfloat16)
+            and k.dtype is dt and v.dtype is dt and k.shape == shape and v.shape == shape and len(shape) == 4
+            and q.is_contiguous() and k.is_contiguous() and v.is_contiguous()):
+        return flash_attn_fwd(q, k, v, layout="bnhd")   # the usual call; the others are told below what is wrong
     out = torch.empty_like(q)
     # the default configuration's own checks (fp16, its head dim, lengths that are multiples of its 64 x 64
     # blocks) hold wherever it applies; elsewhere the operator takes the call without one

@@ -223,13 +223,19 @@ def flash_attn_fwd(
     if use_carry and carry is None:
         raise RuntimeError("carry_in / carry_out need a carry buffer (carry_state)")
     # Fast path: the same tensors and flags as an earlier call.  Only a caller-provided `out` can be
-    # part of the key; a fresh output (and lse) is allocated per call and patched into the block.
+    # part of the key; a fresh output (and lse) is allocated per call and patched into the block.  What the key
+    # leaves out must follow from it in every call that validation accepts; a call where it does not goes there.
     try:
-        key = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if out is not None else 0,
-               q.shape, q.stride(), k.shape, k.stride(), v.stride(), out.stride() if out is not None else None,
-               q.dtype, q.device.index, causal, softmax_scale, layout, return_lse, kernel, q_pos0, k_pos0, balance,
-               carry.data_ptr() if carry is not None else 0, carry_in, carry_out, carry_rows)
-        hit = _param_cache.get(key)
+        dt = q.dtype
+        if (k.dtype is dt and v.dtype is dt and v.shape == k.shape
+                and (out is None or (out.dtype is dt and out.shape == q.shape))):
+            key = (q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr() if out is not None else 0,
+                   q.shape, q.stride(), k.shape, k.stride(), v.stride(), out.stride() if out is not None else None,
+                   dt, q.get_device(), causal, softmax_scale, layout, return_lse, kernel, q_pos0, k_pos0, balance,
+                   (carry.data_ptr(), carry.nbytes) if carry is not None else 0, carry_in, carry_out, carry_rows)
+            hit = _param_cache.get(key)
+        else:
+            key, hit = None, None
     except (AttributeError, TypeError):   # not tensors: let the validation below say so
         key, hit = None, None
     if hit is not None:
@@ -275,13 +281,12 @@ def flash_attn_fwd(
                 _param_cache.clear()
             _param_cache[key] = (p, need)
     if p is not None:
-        dev = q.device
-        dev_index = dev.index
+        dev_index = q.get_device()
         if _current_device() == dev_index:
-            rc = _launch_fwd(p, need, dev, _current_raw_stream(dev_index))
+            rc = _launch_fwd(p, need, q, _current_raw_stream(dev_index))
         else:
-            with torch.cuda.device(dev):
-                rc = _launch_fwd(p, need, dev, _current_raw_stream(dev_index))
+            with torch.cuda.device(dev_index):
+                rc = _launch_fwd(p, need, q, _current_raw_stream(dev_index))
         if rc != _lib.OK:
             _lib.check(rc, "miniattn_fwd")
     if carry_out:
@@ -296,9 +301,9 @@ _current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
 _current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
 
 
-def _launch_fwd(p, need: int, device: torch.device, stream: int) -> int:
+def _launch_fwd(p, need: int, q: torch.Tensor, stream: int) -> int:
     if need > 0:
-        scratch = _scratch_for(device, stream, need)
+        scratch = _scratch_for(q.device, stream, need)
         return _lib.lib.miniattn_fwd_balanced(_byref(p), scratch.data_ptr(), scratch.numel(), stream)
     return _lib.lib.miniattn_fwd(_byref(p), stream)
 
