@@ -863,7 +863,7 @@ int miniattn_check_status(int32_t status_word) {
   g_err[0] = 0;
   if (status_word == 0) return MINIATTN_OK;
   static const char* const names[] = {"K/V or Q tile load", "S = QK^T", "O += PV", "P hand-off", "ring slot release",
-                                      "correction hand-off", "partial of another CTA of a cut item"};
+                                      "(bit 5, not in use)", "partial of another CTA of a cut item"};
   char list[256] = "";
   for (int bit = 0; bit < 7; ++bit)
     if (status_word & (1 << bit)) {

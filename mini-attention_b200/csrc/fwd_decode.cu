@@ -1,14 +1,14 @@
 // Forward attention for few query rows per KV head (decode, speculative and short chunked prefill).
 //
 // With a handful of query tokens the call reads K and V once and does almost nothing with them: it
-// is bound by HBM, and the 128-row Q tiles of fwd_ws.cu are the wrong shape for it -- every query
-// head of a KV head is a work item of its own there, each re-reading K/V (from L2) for a tile whose
-// rows are nearly all padding.  Here the G query heads that share a KV head and the Nq tokens form
-// the rows of ONE item (row = token * G + head), so K/V cross the SM once for all of them:
+// is bound by HBM, and the 128-row Q tiles of fwd_ws.cu are the wrong shape for it -- nearly all of
+// their rows are padding, and one CTA per SM has a K/V tile or two in flight.  Here the G query heads
+// that share a KV head and the Nq tokens form the rows of ONE item (row = token * G + head), so K/V
+// cross the SM once for all of them, in blocks of 16 rows, and two CTAs share an SM:
 //
 //   item      = (batch, KV head, block of 16*RG rows);  T tiles of 64 keys each
 //   CTA       = a contiguous range of the tiles of all items, the same length for every CTA of the
-//               launch (two CTAs per SM), so no SM idles whatever the batch and context are
+//               launch; plan_decode (plan.cu) says how many and which calls come here at all
 //   warp 4    TMA producer: K and V boxes (64 keys, 128-byte swizzle) through a ring, 96 KB deep,
 //             192 KB in flight per SM
 //   warps 0-3 16 rows x (16*RG keys of the tile) each: RG row groups x 4/RG key groups, each warp
@@ -22,7 +22,7 @@
 // itself in; the CTA that counts in last folds the pieces and writes the rows.  Nobody waits.
 //
 // Measured (B200, 16 requests, 32/8 heads, 1 token against 4001 keys, D=128 bf16, 262 MB of K/V): 183 us
-// through fwd_ws.cu, 51 us here = 5.2 TB/s, 0.79 of the measured copy bandwidth.
+// through fwd_ws.cu before that packed heads, 48 now, 46 us here = 5.7 TB/s, 0.87 of the measured copy bandwidth.
 #include <atomic>
 #include <type_traits>
 

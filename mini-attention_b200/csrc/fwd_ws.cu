@@ -40,7 +40,7 @@
 // and the next S.
 //
 // Softmax arithmetic runs two scores per issue slot (packed f32x2 FMA / ADD); a share of the
-// exponentials is evaluated by a cubic on the FMA pipe instead of the exp2 unit.
+// exponentials is evaluated by a polynomial on the FMA pipe instead of the exp2 unit.
 //
 // Template variants of the one kernel: QK8 (int8 Q K^T, accumulator pre-biased so that the scores
 // arrive as floats), PLAN (balanced launch: work items cut over several CTAs, merged by the last
@@ -213,7 +213,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     n_tiles = pe_t1 - pe_t0;
   }
 
-  // TMA loads (issued by lane 0 of warp 13 only): Q tile t; ring fill i = K (even) or V (odd) of
+  // TMA loads (issued by lane 0 of warp kWarpTma only): Q tile t; ring fill i = K (even) or V (odd) of
   // K/V tile kv_t0 + i/2 into slot i % kStages.
   auto load_q = [&](int t) {
     if constexpr (QK8) {  // one box of D bytes x 128 rows
@@ -747,7 +747,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     reg_dec<kRegOther>();
     if (warp == kWarpMma0 || warp == kWarpMma1) {
       // =========================== MMA issuers =====================================
-      // One issuing thread per Q tile (warp 12 -> tile 0, warp 14 -> tile 1).  Each walks its
+      // One issuing thread per Q tile (warp 8 -> tile 0, warp 10 -> tile 1).  Each walks its
       // tile's halves in the order the softmax group publishes them: PV_a(j) S_a(j+1) PV_b(j)
       // S_b(j+1).  The tensor pipe interleaves the two streams.
       const int t = (warp == kWarpMma0) ? 0 : 1;
@@ -795,10 +795,9 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         mbar_wait(bar(L::kBarQFull + t), 0, wc, kErrWaitKV);
         int cons = 0;  // ring consumption index: K_0, V_0, K_1, V_1, ...
         mbar_wait(bar(L::kBarKvFull + 0), 0, wc, kErrWaitKV);
-        // Start tile 1 about half a softmax step after tile 0 (when tile 0 has published its
-        // first row maxima): the two softmax groups then alternate between their max and exp2
-        // phases instead of competing for the exp2 unit at the same moments.  The barrier
-        // completes exactly once, so a late issuer can never mistake a later phase for it.
+        // Start tile 1 about half a softmax step after tile 0 (when tile 0 has its first row maxima): the
+        // two softmax groups then do not want the exp2 unit at the same moments.  The barrier completes
+        // exactly once, so a late issuer can never mistake a later phase for it.
         if (t == 1) mbar_wait(bar(L::kBarStagger), 0, wc, kErrWaitP);
         tc_fence_after();
         for (int hb = 0; hb < 2; ++hb) {

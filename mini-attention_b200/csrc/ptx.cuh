@@ -18,7 +18,7 @@ constexpr int kErrWaitS    = 1 << 1;   // S = QK^T MMA never completed
 constexpr int kErrWaitO    = 1 << 2;   // O += PV MMA never completed
 constexpr int kErrWaitP    = 1 << 3;   // P tile never published by the softmax role
 constexpr int kErrWaitFree = 1 << 4;   // a ring slot was never released
-constexpr int kErrWaitCorr = 1 << 5;   // correction / epilogue hand-off never happened
+// 1 << 5 was a hand-off between roles that no longer exist; nothing raises it
 constexpr int kErrWaitPeer = 1 << 6;   // another CTA of a cut work item never published its partial
 constexpr int kErrTest     = 1 << 30;  // raised only by the wait self-test kernel
 
