@@ -30,13 +30,14 @@
 // maximum is found, O and l are rescaled, and the half is taken again.  l is accumulated against the same
 // reference, which keeps O / l exact.
 //
-// What bounds it (clock stamps, N = 2048, D = 128, per 128-key step of a CTA, about 2950 clk): the MMAs
-// of a step need 2608 clk of the tensor pipe, and they and TMA 2560 clk of the 128 B/clk shared-memory
-// port (Q is re-read for each half).  Finding the maximum of a half first and handing the factor to four
-// correction warps made it 3140: 3956 us for 16 heads at N = 32768, 3743 with the maximum found beside the
-// exponentials, 3685 without one.  At D = 64 the softmax thread is the bound: N = 8192 (2 x 16 heads) 706 /
-// 694 / 654 us.  One MMA of 128 keys for S (2080 clk of tensor work) measured slower, 49 against 41 us at
-// N = 2048: TMEM has room for one S buffer per Q tile then, and the thread waits 1600 clk per step for PV
+// What bounds it (N = 2048, D = 128, per 128-key step of a CTA, about 2660 clk; 2950 while the issuing threads put
+// every descriptor together anew): the MMAs of a step need 2608 clk of the tensor pipe, and they and TMA 2560 clk of
+// the 128 B/clk shared-memory port (Q is re-read for each half).  With that slower issue, finding the maximum of a
+// half first and handing the factor to four correction warps took 3956 us for 16 heads at N = 32768, 3743 with the
+// maximum found beside the exponentials, 3685 without one.  At D = 64 the softmax thread is the bound: N = 8192
+// (2 x 16 heads) 706 / 694 / 654 us, 609 with the present issue.  One MMA of 128 keys for S (2080 clk of tensor work)
+// measured slower, 49 against 41 us at N = 2048: TMEM has room for one S buffer per Q tile then, and the thread waits
+// 1600 clk per step for PV
 // and the next S.
 //
 // Softmax arithmetic runs two scores per issue slot (packed f32x2 FMA / ADD); a share of the
@@ -750,8 +751,13 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // One issuing thread per Q tile (warp 8 -> tile 0, warp 10 -> tile 1).  Each walks its
       // tile's halves in the order the softmax group publishes them: PV_a(j) S_a(j+1) PV_b(j)
       // S_b(j+1).  The tensor pipe interleaves the two streams.
+      // The whole warp walks the halves and one elected thread issues, its descriptors a warp-uniform base plus
+      // constants: an MMA then costs the issuing thread less than the 32 to 64 clk it takes the pipe.  Put together by a
+      // single thread of a diverged warp they cost 45 to 112 clk each, 24 of them a step: 16 heads, N = 16384
+      // 1834 -> 1646 us, N = 2048 32.3 -> 30.5, N = 512 9.55 -> 8.02; D = 64, N = 8192 657 -> 609; INT8-QK 680 -> 656.
       const int t = (warp == kWarpMma0) ? 0 : 1;
-      if (lane == 0 && n_tiles > 0 && t < nt) {
+      if (n_tiles > 0 && t < nt) {
+        const bool issuer = elect_one();
         // kind::f16: D fmt f32, A/B f16 or bf16.  kind::i8: D fmt s32 (2), A/B signed int8 (1).
         constexpr uint32_t idesc_s =
             QK8 ? make_idesc(2, 1, 0, 0, kTileM, kHalfN) : make_idesc(1, BF16 ? 1 : 0, 0, 0, kTileM, kHalfN);
@@ -762,6 +768,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // S(half) = Q_t . K[64*half .. 64*half+64)^T  ->  TMEM columns [128t + 64half, +64)
         auto issue_s = [&](int hb, int slot) {
           const uint32_t d_tmem = tSt + kHalfN * hb;
+          if (!issuer) return;
           if constexpr (QK8) {
             // The accumulator starts at 1.5*2^23 in every element: one fp16 MMA of two constant
             // tiles (3072 * 4096 in the k = 0 term, zeros elsewhere) writes the fp32 bit pattern
@@ -774,21 +781,17 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             // one MMA consumes K = 32 bytes.
             constexpr uint32_t kLayout = (D == 64) ? 4u : 2u;
             constexpr uint32_t kSbo = (D == 64) ? 512u : 1024u;
-            const uint32_t kb = sRing + slot * L::kTileBytes + hb * kHalfN * D;
+            const uint64_t da = make_smem_desc(sQt, 16, kSbo, kLayout);
+            const uint64_t db = make_smem_desc(sRing, 16, kSbo, kLayout) + ((slot * L::kTileBytes + hb * kHalfN * D) >> 4);
 #pragma unroll
-            for (int k = 0; k < D / 32; ++k) {
-              const uint64_t da = make_smem_desc(sQt + k * 32, 16, kSbo, kLayout);
-              const uint64_t db = make_smem_desc(kb + k * 32, 16, kSbo, kLayout);
-              mma_i8_ss(d_tmem, da, db, idesc_s, 1u);
-            }
+            for (int k = 0; k < D / 32; ++k) mma_i8_ss(d_tmem, da + k * 2, db + k * 2, idesc_s, 1u);
           } else {
-            const uint32_t kb = sRing + slot * L::kTileBytes + hb * kHalfN * 128;
+            const uint64_t da = make_smem_desc(sQt, 16, 1024);
+            const uint64_t db = make_smem_desc(sRing, 16, 1024) + ((slot * L::kTileBytes + hb * kHalfN * 128) >> 4);
 #pragma unroll
             for (int k = 0; k < kCols / 16; ++k) {
-              const uint32_t off = (k / 4) * kBoxBytes + (k % 4) * 32;
-              const uint64_t da = make_smem_desc(sQt + off, 16, 1024);
-              const uint64_t db = make_smem_desc(kb + off, 16, 1024);
-              mma_f16_ss(d_tmem, da, db, idesc_s, k > 0);
+              const uint32_t off = ((k / 4) * kBoxBytes + (k % 4) * 32) >> 4;
+              mma_f16_ss(d_tmem, da + off, db + off, idesc_s, k > 0);
             }
           }
         };
@@ -802,9 +805,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
         for (int hb = 0; hb < 2; ++hb) {
           issue_s(hb, 0);
-          mma_commit(bar(L::kBarSFull + 2 * t + hb));
+          if (issuer) mma_commit(bar(L::kBarSFull + 2 * t + hb));
         }
-        mma_commit(bar(L::kBarKvEmpty + 0));
+        if (issuer) mma_commit(bar(L::kBarKvEmpty + 0));
+        __syncwarp();
         cons = 1;
         for (int j = 0; j < n_tiles; ++j) {
           const int vslot = cons % L::kStages;
@@ -818,28 +822,35 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             mbar_wait(bar(L::kBarPReady + 2 * t + hb), j & 1, wc, kErrWaitP);
             tc_fence_after();
             const uint32_t tP = tSt + kHalfN * hb;
+            if (issuer) {
+              const uint64_t db = make_smem_desc(sRing, kBoxBytes, 1024) + ((vslot * L::kTileBytes) >> 4);
 #pragma unroll
-            for (int kk = 0; kk < kHalfN / 16; ++kk) {
-              const int k = hb * (kHalfN / 16) + kk;  // 16-key slice of the V tile
-              const uint64_t db =
-                  make_smem_desc(sRing + vslot * L::kTileBytes + k * 2048, kBoxBytes, 1024);
-              mma_f16_ts(tO, tP + kk * 8, db, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+              for (int kk = 0; kk < kHalfN / 16; ++kk) {
+                const int k = hb * (kHalfN / 16) + kk;  // 16-key slice of the V tile
+                mma_f16_ts(tO, tP + kk * 8, db + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+              }
+              mma_commit(bar(L::kBarODone + 2 * t + hb));
+              if (hb == 1) mma_commit(bar(L::kBarKvEmpty + vslot));
             }
-            mma_commit(bar(L::kBarODone + 2 * t + hb));
-            if (hb == 1) mma_commit(bar(L::kBarKvEmpty + vslot));
+            __syncwarp();
             if (has_next) {  // S_h(j+1) after PV_h(j), whose operand P_h(j) lives in the S buffer
               if (hb == 0) {
                 mbar_wait(bar(L::kBarKvFull + kslot), kpar, wc, kErrWaitKV);
                 tc_fence_after();
               }
               issue_s(hb, kslot);
-              mma_commit(bar(L::kBarSFull + 2 * t + hb));
-              if (hb == 1) mma_commit(bar(L::kBarKvEmpty + kslot));
+              if (issuer) {
+                mma_commit(bar(L::kBarSFull + 2 * t + hb));
+                if (hb == 1) mma_commit(bar(L::kBarKvEmpty + kslot));
+              }
+              __syncwarp();
             }
           }
           if (has_next) ++cons;
         }
-        if constexpr (PLAN || CARRY) mma_commit(bar(L::kBarTileDone + t));
+        if constexpr (PLAN || CARRY) {
+          if (issuer) mma_commit(bar(L::kBarTileDone + t));
+        }
       }
       __syncwarp();
     } else if (warp == kWarpTma) {
