@@ -862,6 +862,10 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         for (int i = n_early; i < n_fill; ++i) {
           const int slot = i % L::kStages;
           const int use = i / L::kStages;
+          // A warp that mbarrier.try_wait holds takes issue slots from the softmax warps beside it, a sleeping one takes
+          // none; the ring has slack for some of the half step until the next slot comes free (100 to 400 ns alike, 800
+          // starves it).  N = 8192 D = 64 625 -> 613 us, INT8-QK 618 -> 612, 4 x 32/8 heads N = 4096 causal 460 -> 456.
+          __nanosleep(200);
           mbar_wait(bar(L::kBarKvEmpty + slot), (use - 1) & 1, wc, kErrWaitFree);
           if (issuer) load_kv(i);
           __syncwarp();
