@@ -362,6 +362,7 @@ static void fill_args(const MiniAttnFwdParams* p, ma::FwdArgs* a, int pack) {
   a->n_q_tiles = (p->Nq + a->tpt - 1) / a->tpt;
   a->n_pair_items = 0;  // set by the warp-specialised launcher
   a->bh_group = head_group(p, pack);
+  ma::set_divisors(a);
   a->sq = nullptr;
   a->sk = nullptr;
   a->part_o = nullptr;

@@ -6,6 +6,26 @@
 
 namespace ma {
 
+// n / d for 0 <= n < 2^31 without a division: floor((m' * n) / 2^(32 + shift)) with m' = 2^32 + m the multiple of 1 / d
+// rounded up (Granlund and Montgomery, "Division by invariant integers using multiplication", 1994).
+struct FastDiv {
+  uint32_t d, m, shift;
+};
+inline FastDiv fast_div(uint32_t d) {
+  FastDiv f{d, 0, 0};
+  while ((1ull << f.shift) < d) ++f.shift;
+  f.m = static_cast<uint32_t>(((((1ull << f.shift) - d) << 32) / d) + 1);
+  return f;
+}
+__host__ __device__ inline int div_by(int n, const FastDiv& f) {
+#ifdef __CUDA_ARCH__
+  const uint32_t high = __umulhi(static_cast<uint32_t>(n), f.m);
+#else
+  const uint32_t high = static_cast<uint32_t>((static_cast<uint64_t>(n) * f.m) >> 32);
+#endif
+  return static_cast<int>((high + static_cast<uint32_t>(n)) >> f.shift);
+}
+
 struct FwdArgs {
   float*   lse;        // [B, Hq, Nq] or null
   int32_t* status;     // device word for wait-timeout bits, or null
@@ -25,6 +45,8 @@ struct FwdArgs {
   int bh_group;        // work items are ordered in groups of this many consecutive (batch, head)
                        // indices: all Q-tile pairs of a group (latest first, heads fastest) before the
                        // next group.  B*Hq = one group, the default order.  Divides B*Hq.
+  // divisors a CTA finds its work with, in the order it needs them (set by set_divisors)
+  FastDiv by_group_items, by_group, by_heads, by_gqa, by_pack;
   const float* sq;     // INT8-QK: [B, Hq,  ceil(Nq/128)] Q scales (softmax scale * log2e folded in)
   const float* sk;     // INT8-QK: [B, Hkv, ceil(Nk/128)] K scales
   // Balanced launches only (null otherwise): where CTAs that cover part of an item's key range
@@ -99,10 +121,20 @@ constexpr int kBoxBytes = kTileN * 128;  // one [128 rows x 128 B] TMA box
 // heads fastest, so that the CTAs in flight share the K/V of few heads.  Shared by the kernels and
 // the host planner.
 __host__ __device__ inline void item_to_pair_bh(const FwdArgs& a, int n_pairs, int item, int* pair, int* bh) {
-  const int per_group = n_pairs * a.bh_group;
-  const int within = item % per_group;
-  *pair = n_pairs - 1 - within / a.bh_group;
-  *bh = (item / per_group) * a.bh_group + within % a.bh_group;
+  const int group = div_by(item, a.by_group_items);
+  const int within = item - group * static_cast<int>(a.by_group_items.d);
+  const int back = div_by(within, a.by_group);
+  *pair = n_pairs - 1 - back;
+  *bh = group * a.bh_group + within - back * a.bh_group;
+}
+// After Hq, Hkv, n_q_tiles, bh_group and pack are known.
+inline void set_divisors(FwdArgs* a) {
+  const long long group_items = static_cast<long long>((a->n_q_tiles + 1) / 2) * a->bh_group;
+  a->by_group_items = fast_div(group_items > 0 && group_items < 0x7fffffffll ? static_cast<uint32_t>(group_items) : 1u);
+  a->by_group = fast_div(a->bh_group > 0 ? a->bh_group : 1);
+  a->by_heads = fast_div(a->Hq > 0 ? a->Hq : 1);
+  a->by_gqa = fast_div(a->Hkv > 0 && a->Hq >= a->Hkv ? a->Hq / a->Hkv : 1);
+  a->by_pack = fast_div(a->pack > 0 ? a->pack : 1);
 }
 
 // Number of K/V tiles the Q tiles whose first token is q0 have to visit (all of them without a mask,

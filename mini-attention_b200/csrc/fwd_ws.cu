@@ -193,9 +193,9 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int tpt = PACK ? a.tpt : kTileM;  // query tokens per Q tile
   int pair, bh;
   item_to_pair_bh(a, n_pairs, item, &pair, &bh);
-  const int h = bh % a.Hq;
-  const int b = bh / a.Hq;
-  const int hk = h / (a.Hq / a.Hkv);
+  const int b = div_by(bh, a.by_heads);
+  const int h = bh - b * a.Hq;
+  const int hk = div_by(h, a.by_gqa);
   const int q0 = (pair * 2 + (single > 0 ? 1 : 0)) * tpt;  // first query token
   // Q tiles of this CTA that hold real rows
   const int nt = (single < 0 && q0 + tpt < a.Nq) ? 2 : 1;
@@ -322,7 +322,7 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int t = warp >> 2;
     if (t < nt) {
       const int r = tid & 127;
-      const int row = q0 + t * tpt + (PACK ? r / a.pack : r);  // query token of this thread
+      const int row = q0 + t * tpt + (PACK ? div_by(r, a.by_pack) : r);  // query token of this thread
       const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
       const uint32_t tS = tmem_base + L::kColS + 128 * t + lane_off;
       long long vis_ll = a.Nk;
