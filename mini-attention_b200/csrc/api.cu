@@ -549,11 +549,12 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   const bool simple = p->kernel == MINIATTN_KERNEL_SIMPLE;
   ma::FwdArgs a;
   fill_args(p, &a, head_pack(p));
-  auto q_map = [&](CUtensorMap* out, const void* base, const int64_t stride[3], const char* what) {
-    return a.pack == 1 ? make_map(out, base, 2, dt, p->D, p->Nq, p->Hq, p->B, stride, ma::kBoxCols, ma::kTileM, what)
-                       : make_map_packed(out, base, dt, p->D, p->Nq, a.Hq, p->B, stride, a.pack, a.tpt, what);
+  // rows: of the box, a whole tile or what one warp stores of it
+  auto q_map = [&](CUtensorMap* out, const void* base, const int64_t stride[3], int rows, const char* what) {
+    return a.pack == 1 ? make_map(out, base, 2, dt, p->D, p->Nq, p->Hq, p->B, stride, ma::kBoxCols, rows, what)
+                       : make_map_packed(out, base, dt, p->D, p->Nq, a.Hq, p->B, stride, a.pack, rows / a.pack, what);
   };
-  if ((rc = q_map(&tm[0], p->q, p->q_stride, "q")) != 0) return rc;
+  if ((rc = q_map(&tm[0], p->q, p->q_stride, ma::kTileM, "q")) != 0) return rc;
   if (has_keys) {
     if ((rc = make_map(&tm[1], p->k, 2, dt, p->D, p->Nk, p->Hkv, p->B, p->k_stride, ma::kBoxCols,
                        ma::kTileN, "k")) != 0)
@@ -567,7 +568,8 @@ static int fwd_common(const MiniAttnFwdParams* p, void* scratch, size_t scratch_
   }
   if (p->o == nullptr) {
     tm[3] = tm[0];  // state-only call: the kernel never stores through the output map
-  } else if ((rc = q_map(&tm[3], p->o, p->o_stride, "o")) != 0) {
+  } else if ((rc = q_map(&tm[3], p->o, p->o_stride,
+                         simple || ma::kWarpRows % a.pack != 0 ? ma::kTileM : ma::kWarpRows, "o")) != 0) {
     return rc;
   }
 
@@ -793,7 +795,7 @@ static int int8_common(const MiniAttnInt8Params* p, void* scratch, size_t scratc
   if ((rc = make_map(&tm[2], f.v, 2, dt, f.D, f.Nk, f.Hkv, f.B, f.v_stride, ma::kBoxCols, ma::kTileN,
                      "v")) != 0)
     return rc;
-  if ((rc = make_map(&tm[3], f.o, 2, dt, f.D, f.Nq, f.Hq, f.B, f.o_stride, ma::kBoxCols, ma::kTileM,
+  if ((rc = make_map(&tm[3], f.o, 2, dt, f.D, f.Nq, f.Hq, f.B, f.o_stride, ma::kBoxCols, ma::kWarpRows,
                      "o")) != 0)
     return rc;
   ma::FwdArgs a;

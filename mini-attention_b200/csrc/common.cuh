@@ -113,6 +113,7 @@ struct DecodePlan {
 
 constexpr int kTileM = 128;   // query rows per MMA tile (TMEM lanes)
 constexpr int kTileN = 128;   // keys per K/V tile
+constexpr int kWarpRows = 32;  // rows of a Q tile that one warp stores
 constexpr int kBoxCols = 64;  // 16-bit elements per 128-byte swizzled row
 constexpr int kBoxBytes = kTileN * 128;  // one [128 rows x 128 B] TMA box
 
