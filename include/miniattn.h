@@ -266,6 +266,36 @@ typedef struct MiniAttnMergeParams {
 int miniattn_merge_partials(const MiniAttnMergeParams* p, void* stream);
 
 /*
+ * Linear layers that share their input, in one launch: y_i = x w_i^T + b_i, the projections around the
+ * attention call of the reference's modules (kernels/standard/pytorch/gqa.py:24-28, :50).  16-bit operands, fp32
+ * accumulation and bias, one rounding.  x is [M, K], w_i [N_i, K] and y_i [M, N_i], each with its last dimension
+ * contiguous and its rows ldx / ldw / ldy elements apart; K, N_i and the row strides are multiples of 8, the
+ * pointers (bias excepted) 16-byte aligned.  At most 3 weights.
+ */
+typedef struct MiniAttnLinearOut {
+  const void* w;
+  const void* bias;       /* [N] or null */
+  void*       y;
+  int64_t     ldw, ldy;
+  int32_t     N;
+  int32_t     reserved;   /* 0 */
+} MiniAttnLinearOut;
+
+typedef struct MiniAttnLinearParams {
+  const void* x;
+  int32_t*    status;     /* as in MiniAttnFwdParams */
+  int64_t     ldx;
+  int32_t     M, K;
+  int32_t     dtype;      /* MINIATTN_FP16 | MINIATTN_BF16 */
+  int32_t     n_out;
+  int32_t     only_if_faster;  /* 1: launch nothing and return 1 where one GEMM per weight is expected to be quicker */
+  int32_t     reserved;   /* 0 */
+  MiniAttnLinearOut out[3];
+} MiniAttnLinearParams;
+
+int miniattn_linear(const MiniAttnLinearParams* p, void* stream);
+
+/*
  * Failure-detection self-test (no reference counterpart; the reference never checks
  * its launches, flash_attention.cu:123).  Launches one CTA that waits on a barrier
  * nothing signals.  The wait gives up after `limit_ns` nanoseconds (0 < limit_ns <= 2e9),

@@ -16,6 +16,7 @@
 
 #include "../../include/miniattn.h"
 #include "common.cuh"
+#include "linear.cuh"
 
 namespace ma {
 cudaError_t launch_fwd_simple(int D, bool bf16, const CUtensorMap* tm, const FwdArgs& a,
@@ -41,6 +42,8 @@ cudaError_t launch_quant_qk_static(int D, bool bf16, const void* q, const long l
                                    const long long* ks, int B, int Hq, int Hkv, int Nq, int Nk,
                                    float q_fold, int8_t* q8, int8_t* k8, float* sq, float* sk,
                                    float* k_mean, cudaStream_t st);
+int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* pays);
+cudaError_t launch_linear(bool bf16, const LinearArgs& a, int pairs, cudaStream_t st);
 cudaError_t launch_wait_selftest(int32_t* status, unsigned long long limit_ns, cudaStream_t st);
 cudaError_t launch_merge_partials(float* acc_o, float* acc_lse, const void* part_o,
                                   const float* part_lse, void* out, long long rows, int D, bool bf16,
@@ -159,6 +162,34 @@ int make_map_packed(CUtensorMap* out, const void* base, CUtensorMapDataType dt, 
     if (dims[i + 1] == 1) strides[i] = (cuuint64_t)D * 2;
   CUresult r = enc(out, dt, 5, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return fail(MINIATTN_ECUDA, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r);
+  MapSlot& slot = cache[next_slot++ % kMapSlots];
+  slot.key = key;
+  slot.map = *out;
+  slot.valid = true;
+  return MINIATTN_OK;
+}
+
+// 2-D map over a row-major [rows, cols] matrix of 16-bit elements, for linear.cu.
+int make_map_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int rows, int cols, int64_t ld, int box_rows,
+                int box_cols, CUtensorMapSwizzle swizzle, const char* what) {
+  thread_local MapSlot cache[kMapSlots] = {};
+  thread_local unsigned next_slot = 0;
+  const MapKey key{base, {ld, 0, 0}, 2, static_cast<int>(dt), cols, rows, 1, 1, box_cols, box_rows, static_cast<int>(swizzle)};
+  for (int i = 0; i < kMapSlots; ++i)
+    if (cache[i].valid && cache[i].key == key) {
+      *out = cache[i].map;
+      return MINIATTN_OK;
+    }
+  EncodeTiledFn enc = encode_fn();
+  if (!enc) return fail(MINIATTN_ECUDA, "cuTensorMapEncodeTiled entry point not found");
+  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)(rows == 1 ? cols : ld) * 2};  // a size-1 dim may carry any stride
+  cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(MINIATTN_ECUDA, "cuTensorMapEncodeTiled(%s) failed with CUresult %d", what, (int)r);
   MapSlot& slot = cache[next_slot++ % kMapSlots];
@@ -859,6 +890,71 @@ int miniattn_merge_partials(const MiniAttnMergeParams* p, void* stream) {
                                             reinterpret_cast<cudaStream_t>(stream));
   if (e != cudaSuccess)
     return fail(MINIATTN_ECUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+  return MINIATTN_OK;
+}
+
+static int check_rows(const void* p, int64_t ld, int cols, const char* name) {
+  if (p == nullptr) return fail(MINIATTN_EINVAL, "%s is null", name);
+  if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return fail(MINIATTN_EINVAL, "%s must be 16-byte aligned", name);
+  if (ld % 8 != 0 || ld < cols)
+    return fail(MINIATTN_EINVAL, "row stride of %s (%lld) must be a multiple of 8 and cover its %d columns", name,
+                (long long)ld, cols);
+  return MINIATTN_OK;
+}
+
+int miniattn_linear(const MiniAttnLinearParams* p, void* stream) {
+  g_err[0] = 0;
+  if (p == nullptr) return fail(MINIATTN_EINVAL, "params is null");
+  if (p->dtype != MINIATTN_FP16 && p->dtype != MINIATTN_BF16)
+    return fail(MINIATTN_EUNSUPPORTED, "dtype must be fp16 (0) or bf16 (1), got %d", p->dtype);
+  if (p->n_out < 1 || p->n_out > ma::kLinearMax)
+    return fail(MINIATTN_EINVAL, "1 to %d weights, got %d", ma::kLinearMax, p->n_out);
+  if (p->M < 0 || p->K <= 0 || p->K % 8 != 0)
+    return fail(MINIATTN_EINVAL, "M (%d) must not be negative, K (%d) a positive multiple of 8", p->M, p->K);
+  if (p->M == 0) return MINIATTN_OK;
+  int rc, N[ma::kLinearMax];
+  if ((rc = check_rows(p->x, p->ldx, p->K, "x")) != 0) return rc;
+  for (int i = 0; i < p->n_out; ++i) {
+    const MiniAttnLinearOut& o = p->out[i];
+    if (o.N <= 0 || o.N % 8 != 0) return fail(MINIATTN_EINVAL, "N (%d) must be a positive multiple of 8", o.N);
+    if ((rc = check_rows(o.w, o.ldw, p->K, "w")) != 0 || (rc = check_rows(o.y, o.ldy, o.N, "y")) != 0) return rc;
+    if (o.bias != nullptr && reinterpret_cast<uintptr_t>(o.bias) % 2 != 0)
+      return fail(MINIATTN_EINVAL, "bias must be 2-byte aligned");
+    N[i] = o.N;
+  }
+  int sms = 0;
+  if ((rc = check_device(&sms)) != 0) return rc;
+  const CUtensorMapDataType dt =
+      p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  ma::LinearArgs a{};
+  bool pays = false;
+  a.bn = ma::linear_tile(p->M, p->K, p->n_out, N, sms / 2, &pays);
+  if (p->only_if_faster && !pays) return 1;
+  a.status = p->status;
+  a.M = p->M;
+  a.K = p->K;
+  a.n_seg = p->n_out;
+  if ((rc = make_map_2d(&a.tm_x, p->x, dt, p->M, p->K, p->ldx, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B, "x")) != 0) return rc;
+  int tiles = 0;
+  for (int i = 0; i < p->n_out; ++i) {
+    const MiniAttnLinearOut& o = p->out[i];
+    ma::LinearSeg& s = a.seg[i];
+    if ((rc = make_map_2d(&s.tm_w, o.w, dt, o.N, p->K, o.ldw, a.bn / 2, 64, CU_TENSOR_MAP_SWIZZLE_128B, "w")) != 0 ||
+        (rc = make_map_2d(&s.tm_y, o.y, dt, p->M, o.N, o.ldy, 32, 16, CU_TENSOR_MAP_SWIZZLE_NONE, "y")) != 0)
+      return rc;
+    s.bias = static_cast<const uint16_t*>(o.bias);
+    s.N = o.N;
+    s.bias_16 = reinterpret_cast<uintptr_t>(o.bias) % 16 == 0;
+    a.first_tile[i] = tiles;
+    tiles += (o.N + a.bn - 1) / a.bn;
+  }
+  const long long m_tiles = (p->M + 255ll) / 256;
+  if (tiles * m_tiles > 0x3fffffffll) return fail(MINIATTN_EUNSUPPORTED, "too many tiles");
+  a.by_m_tiles = ma::fast_div(static_cast<uint32_t>(m_tiles));
+  a.n_tiles = static_cast<int>(tiles * m_tiles);
+  const cudaError_t e =
+      ma::launch_linear(p->dtype == MINIATTN_BF16, a, sms / 2, reinterpret_cast<cudaStream_t>(stream));
+  if (e != cudaSuccess) return fail(MINIATTN_ECUDA, "kernel launch failed: %s", cudaGetErrorString(e));
   return MINIATTN_OK;
 }
 

@@ -74,6 +74,25 @@ class PlanPiece(C.Structure):
     ]
 
 
+class LinearOut(C.Structure):
+    """Mirror of ``MiniAttnLinearOut``."""
+
+    _fields_ = [
+        ("w", C.c_void_p), ("bias", C.c_void_p), ("y", C.c_void_p), ("ldw", C.c_int64), ("ldy", C.c_int64),
+        ("N", C.c_int32), ("reserved", C.c_int32),
+    ]
+
+
+class LinearParams(C.Structure):
+    """Mirror of ``MiniAttnLinearParams``."""
+
+    _fields_ = [
+        ("x", C.c_void_p), ("status", C.c_void_p), ("ldx", C.c_int64), ("M", C.c_int32), ("K", C.c_int32),
+        ("dtype", C.c_int32), ("n_out", C.c_int32), ("only_if_faster", C.c_int32), ("reserved", C.c_int32),
+        ("out", LinearOut * 3),
+    ]
+
+
 def _load() -> C.CDLL:
     if not _LIB_PATH.exists():
         raise ImportError(
@@ -99,6 +118,8 @@ def _load() -> C.CDLL:
     for name in ("miniattn_quant_qk_int8", "miniattn_quant_qk_int8_static", "miniattn_fwd_int8qk"):
         getattr(lib, name).argtypes = [C.POINTER(Int8Params), C.c_void_p]
         getattr(lib, name).restype = C.c_int
+    lib.miniattn_linear.argtypes = [C.POINTER(LinearParams), C.c_void_p]
+    lib.miniattn_linear.restype = C.c_int
     lib.miniattn_merge_partials.argtypes = [C.POINTER(MergeParams), C.c_void_p]
     lib.miniattn_merge_partials.restype = C.c_int
     lib.miniattn_selftest_wait.argtypes = [C.c_void_p, C.c_uint64, C.c_void_p]

@@ -552,3 +552,70 @@ def selftest_wait(limit_ms: float = 50.0, device: Union[torch.device, str, None]
                                              C.c_void_p(stream))
     _lib.check(rc, "miniattn_selftest_wait")
     return int(status.item())
+
+
+_Linear, _Parameter = torch.nn.Linear, torch.nn.Parameter
+_nn_module = torch.nn.modules.module
+_forward_ad = torch.autograd.forward_ad
+
+
+def _nobody_watches() -> bool:
+    """No trace, mode, global hook, tangent or autocast that a call of an ``nn.Linear`` would take part in."""
+    c = torch._C
+    return not (c._len_torch_dispatch_stack() or c._len_torch_function_stack() or c._functorch.peek_interpreter_stack()
+                or _forward_ad._current_level >= 0 or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing()
+                or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
+                or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
+                or _nn_module._global_backward_pre_hooks)
+
+
+def linear(x: torch.Tensor, *layers: torch.nn.Linear):
+    """``[layer(x) for layer in layers]`` for up to three linear layers that share their input.
+
+    One launch of ``miniattn_linear`` where that is the quicker form, every layer is a plain ``nn.Linear`` (no hooks, no replaced forward) of
+    16-bit operands on the GPU and nothing watches the call (gradients, tangents, autocast, tracing, modes); the
+    layers' own calls otherwise."""
+    p = None
+    if (type(x) is torch.Tensor and x.is_cuda and x.dtype in _DTYPES and x.is_contiguous() and x.dim() >= 2
+            and len(layers) <= 3 and _nobody_watches()):
+        shape, dt, dev, grad = x.shape, x.dtype, x.get_device(), torch.is_grad_enabled()
+        k, xp = shape[-1], x.data_ptr()
+        m = x.numel() // k if k else 0
+        if m > 0 and k % 8 == 0 and xp % 16 == 0 and not (grad and x.requires_grad):
+            p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
+            out = []
+            for i, layer in enumerate(layers):
+                own = layer.__dict__
+                w, b = own["_parameters"].get("weight"), own["_parameters"].get("bias")
+                if (type(layer) is not _Linear or type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
+                        or "forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"]
+                        or own["_backward_hooks"] or own["_backward_pre_hooks"] or w.dim() != 2
+                        or not w.is_contiguous() or (grad and w.requires_grad)):
+                    p = None
+                    break
+                n, wk = w.shape
+                wp, bp = w.data_ptr(), None
+                if wk != k or n % 8 or n == 0 or wp % 16:
+                    p = None
+                    break
+                if b is not None:
+                    if (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.dim() != 1
+                            or b.numel() != n or not b.is_contiguous() or (grad and b.requires_grad)):
+                        p = None
+                        break
+                    bp = b.data_ptr()
+                y = x.new_empty((*shape[:-1], n))
+                p.out[i] = (wp, bp, y.data_ptr(), k, n, n)
+                out.append(y)
+    if p is None:
+        return [layer(x) for layer in layers]
+    if _current_device() == dev:
+        rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
+    if rc == 1:  # one GEMM per layer is quicker
+        return [layer(x) for layer in layers]
+    if rc != _lib.OK:
+        _lib.check(rc, "miniattn_linear")
+    return out

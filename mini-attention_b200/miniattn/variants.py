@@ -1,7 +1,7 @@
 """MHA / GQA / MQA attention variants of kernels/standard/pytorch with the core attention
-call replaced by the B200 kernel.  Projections stay ordinary ``nn.Linear`` layers (they are
-not on the hot path); parameter names match the reference modules so state dicts load
-unchanged.
+call replaced by the B200 kernel.  Projections stay ordinary ``nn.Linear`` layers, parameter names match the
+reference modules so state dicts load unchanged; where nothing watches their calls (``ops.linear`` says what), the
+ones that share their input run as one launch.
 
 * ``MHA``        kernels/standard/pytorch/mha.py:9-55   (returns ``(output, weights)`` like the
                  reference; ``mask`` = None or all ones runs the non-causal kernel, a
@@ -20,7 +20,7 @@ import torch.nn as nn
 
 import math
 
-from .ops import flash_attn_fwd
+from .ops import flash_attn_fwd, linear
 
 
 def _attend(q, k, v, causal, return_lse=False):
@@ -64,18 +64,16 @@ class MHA(nn.Module):
                     raise RuntimeError("only no mask, an all-ones mask or a lower-triangular (causal) mask is "
                                        "supported: there is no eager path behind the fused kernel")
                 causal = True
-        q = self.w_q(x).view(B, S, self.n_heads, self.d_h)
-        k = self.w_k(x).view(B, S, self.n_heads, self.d_h)
-        v = self.w_v(x).view(B, S, self.n_heads, self.d_h)
+        q, k, v = (y.view(B, S, self.n_heads, self.d_h) for y in linear(x, self.w_q, self.w_k, self.w_v))
         if not self.need_weights:
-            return self.w_o(_attend(q, k, v, causal)), None
+            return linear(_attend(q, k, v, causal), self.w_o)[0], None
         o, lse = _attend(q, k, v, causal, return_lse=True)
         # weights = softmax(q k^T / sqrt(d_h) [+ mask]) rebuilt from the kernel's log-sum-exp
         scores = torch.matmul(q.transpose(1, 2).float(), k.permute(0, 2, 3, 1).float()) / math.sqrt(self.d_h)
         weights = torch.exp(scores - lse.unsqueeze(-1))
         if causal:
             weights = weights.masked_fill(~torch.tril(torch.ones(S, S, device=x.device, dtype=torch.bool)), 0.0)
-        return self.w_o(o), weights.to(x.dtype)
+        return linear(o, self.w_o)[0], weights.to(x.dtype)
 
 
 class GQA_Flash(nn.Module):
@@ -91,9 +89,10 @@ class GQA_Flash(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         B, S, _ = x.shape
-        q = self.w_q(x).view(B, S, self.n_heads, self.head_dim)
-        kv = self.kv(x).view(B, S, 2, self.n_kv_heads, self.head_dim)
-        return self.w_o(_attend(q, kv[:, :, 0], kv[:, :, 1], True))
+        q, kv = linear(x, self.w_q, self.kv)
+        q = q.view(B, S, self.n_heads, self.head_dim)
+        kv = kv.view(B, S, 2, self.n_kv_heads, self.head_dim)
+        return linear(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o)[0]
 
 
 class MQA_Flash(nn.Module):
@@ -107,6 +106,7 @@ class MQA_Flash(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         B, S, _ = x.shape
-        q = self.w_q(x).view(B, S, self.n_heads, self.head_dim)
-        kv = self.k_v(x).view(B, S, 2, 1, self.head_dim)
-        return self.w_o(_attend(q, kv[:, :, 0], kv[:, :, 1], True))
+        q, kv = linear(x, self.w_q, self.k_v)
+        q = q.view(B, S, self.n_heads, self.head_dim)
+        kv = kv.view(B, S, 2, 1, self.head_dim)
+        return linear(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o)[0]

@@ -1,0 +1,50 @@
+"""miniattn_linear's blocks have the layout of their ctypes mirrors, bad calls are refused before the GPU is looked
+for, and ``ops.linear`` on CPU tensors is the layers' own calls."""
+import ctypes as C
+import subprocess
+from pathlib import Path
+
+import torch
+
+from miniattn import _lib, ops
+
+HEADER = Path(__file__).resolve().parent.parent / "include" / "miniattn.h"
+
+
+def test_struct_layouts_match_c(tmp_path):
+    pairs = [("MiniAttnLinearOut", _lib.LinearOut), ("MiniAttnLinearParams", _lib.LinearParams)]
+    lines = ['#include <stdio.h>', '#include <stddef.h>', f'#include "{HEADER}"', "int main(void){"]
+    for name, mirror in pairs:
+        lines.append(f'printf("%zu\\n", sizeof({name}));')
+        lines += [f'printf("%zu\\n", offsetof({name}, {f[0]}));' for f in mirror._fields_]
+    src = tmp_path / "layout.c"
+    src.write_text("\n".join(lines + ["return 0;}"]))
+    subprocess.run(["gcc", "-std=c99", "-Wall", "-Werror", str(src), "-o", str(tmp_path / "layout")], check=True)
+    out = iter(subprocess.run([str(tmp_path / "layout")], check=True, capture_output=True, text=True).stdout.split())
+    for name, mirror in pairs:
+        assert int(next(out)) == C.sizeof(mirror), name
+        for f in mirror._fields_:
+            assert int(next(out)) == getattr(mirror, f[0]).offset, (name, f[0])
+
+
+def _call(**kw):
+    p = _lib.LinearParams(0x1000, 0, 64, 32, 64, 1, 1)
+    p.out[0] = (0x1000, None, 0x1000, 64, 64, 64)
+    for k, v in kw.items():
+        setattr(p.out[0] if hasattr(p.out[0], k) else p, k, v)
+    return _lib.lib.miniattn_linear(C.byref(p), None)
+
+
+def test_bad_calls_are_refused():
+    for kw in (dict(K=60), dict(M=-1), dict(N=12), dict(N=0), dict(n_out=4), dict(n_out=0), dict(x=0x1008), dict(w=None),
+               dict(y=0x1004), dict(ldx=60), dict(ldx=56), dict(ldw=32), dict(ldy=63), dict(bias=0x1001)):
+        assert _call(**kw) == _lib.EINVAL, kw
+    assert _call(dtype=2) == _lib.EUNSUPPORTED
+    assert _call(M=0) == _lib.OK                      # nothing to do, no device asked for
+
+
+def test_cpu_tensors_go_through_the_layers():
+    layers = [torch.nn.Linear(16, n) for n in (8, 24)]
+    x = torch.randn(3, 5, 16)
+    for y, layer in zip(ops.linear(x, *layers), layers):
+        assert torch.equal(y, layer(x)) and y.requires_grad

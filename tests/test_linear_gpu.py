@@ -1,0 +1,121 @@
+"""Linear layers that share their input in one launch (csrc/linear.cu): against the same product in fp64, and the module
+path against the layers' own calls.  Both round once, from fp32 sums: a result is within half an ulp of its own size
+plus the fp32 sum's error, K * 2^-24 of the terms' size."""
+import ctypes as C
+
+import pytest
+import torch
+
+import miniattn
+from miniattn import _lib, ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _launch(x, ws, bs, ys, only_if_faster=0):
+    p = _lib.LinearParams()
+    p.x, p.status, p.ldx, p.M, p.K = x.data_ptr(), ops._status_word(x.device).data_ptr(), x.stride(0), x.shape[0], x.shape[1]
+    p.dtype, p.n_out, p.only_if_faster = ops._DTYPES[x.dtype], len(ws), only_if_faster
+    for o, w, b, y in zip(p.out, ws, bs, ys):
+        o.w, o.y, o.ldw, o.ldy, o.N = w.data_ptr(), y.data_ptr(), w.stride(0), y.stride(0), w.shape[0]
+        o.bias = b.data_ptr() if b is not None else None
+    return _lib.lib.miniattn_linear(C.byref(p), torch.cuda.current_stream().cuda_stream)
+
+
+# M, K, N...: one row to several row tiles, edges of 32, 128 and 256 rows; K below, at and past a stage of 64 and past
+# the ring; N of one box of 16 columns, not a multiple of 16, and several tiles; more tiles than pairs of SMs
+CASES = [
+    (1, 8, (8,)), (31, 64, (16,)), (33, 72, (24, 40)), (128, 256, (256, 64, 8)), (129, 520, (104, 264)), (255, 448, (48,)),
+    (256, 128, (512,)), (257, 1000, (72, 136)), (1000, 1024, (1024, 256)), (2300, 192, (1536, 1544)), (5000, 96, (512, 128)),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("M,K,N", CASES)
+def test_linear_against_fp64(M, K, N, dtype):
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    wide = torch.randn(M, K + 8, device=DEV, generator=g).to(dtype)
+    x = wide[:, :K]                                    # rows further apart than their length
+    ws = [torch.randn(n, K, device=DEV, generator=g).to(dtype) for n in N]
+    bs = [torch.randn(n + 1, device=DEV, generator=g).to(dtype)[1:] if i != 1 else None for i, n in enumerate(N)]  # odd base
+    around = [torch.full((M + 2, n + 16), 7.0, dtype=dtype, device=DEV) for n in N]
+    ys = [t[1:-1, 8:-8] for t in around]
+    assert _launch(x, ws, bs, ys) == _lib.OK
+    assert miniattn.device_status(DEV) == 0
+    ulp = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    for w, b, y, t in zip(ws, bs, ys, around):
+        ref = x.double() @ w.double().T + (b.double() if b is not None else 0.0)
+        size = x.double().abs() @ w.double().abs().T + 4.0
+        bound = ulp * ref.abs() + K * 2.0 ** -24 * size + 2.0 ** -24
+        assert bool(((y.double() - ref).abs() <= bound).all())
+        assert bool((t[0] == 7).all() and (t[-1] == 7).all() and (t[:, :8] == 7).all() and (t[:, -8:] == 7).all())
+
+
+def test_linear_with_a_strided_row_of_one():
+    x = torch.ones(1, 16, dtype=torch.float16, device=DEV)
+    w = torch.ones(8, 16, dtype=torch.float16, device=DEV)
+    y = torch.zeros(1, 8, dtype=torch.float16, device=DEV)
+    assert _launch(x, [w], [None], [y]) == _lib.OK
+    assert bool((y == 16).all())
+
+
+def test_linear_refusals():
+    x = torch.ones(4, 16, dtype=torch.float16, device=DEV)
+    w, y = torch.ones(8, 16, dtype=torch.float16, device=DEV), torch.zeros(4, 8, dtype=torch.float16, device=DEV)
+    assert _launch(x, [w[:7]], [None], [y[:, :7]]) == _lib.EINVAL           # N not a multiple of 8
+    assert _launch(x[:, :12], [w[:, :12]], [None], [y]) == _lib.EINVAL      # K not a multiple of 8
+    assert _launch(x[:, 4:12], [w[:, :8]], [None], [y]) == _lib.EINVAL      # not 16-byte aligned
+    assert _launch(x, [w] * 3, [None] * 3, [y.clone() for _ in range(3)]) == _lib.OK
+
+
+def _module(cls, *args):
+    torch.manual_seed(3)
+    return cls(*args).to(torch.bfloat16).to(DEV)
+
+
+@pytest.mark.parametrize("cls,args,S", [(miniattn.GQA_Flash, (512, 8, 2), 700), (miniattn.MQA_Flash, (512, 4), 300),
+                                        (miniattn.MHA, (256, 2, 0.0, False), 515)])
+def test_modules_against_their_layers_own_calls(cls, args, S, monkeypatch):
+    m = _module(cls, *args)
+    x = torch.randn(2, S, args[0], device=DEV, dtype=torch.bfloat16)
+    first = (lambda y: y[0] if isinstance(y, tuple) else y)
+    with torch.no_grad():
+        fused = first(m(x))
+        monkeypatch.setattr("miniattn.variants.linear", lambda t, *layers: [layer(t) for layer in layers])
+        plain = first(m(x))
+    assert miniattn.device_status(DEV) == 0
+    # the projections differ by their sums' order at most: an ulp of a few of the attention's inputs
+    assert (fused.float() - plain.float()).norm() <= 2.0 ** -8 * plain.float().norm()
+
+
+def test_calls_that_something_watches_go_through_the_layers():
+    """Gradients, hooks, autocast, forward-mode tangents and modes see the layers' own calls, with the same result."""
+    from torch.utils.flop_counter import FlopCounterMode
+    lin = torch.nn.Linear(64, 32).half().to(DEV)
+    x = torch.randn(256, 64, device=DEV, dtype=torch.float16)
+    want = lin(x)
+    y, = ops.linear(x, lin)
+    assert y.requires_grad and torch.equal(y, want)
+    y.sum().backward()
+    assert lin.weight.grad is not None
+    lin.requires_grad_(False)
+    got, = ops.linear(x, lin)
+    assert not got.requires_grad and (got - want).abs().max() <= 2.0 ** -9 * want.abs().max()
+    calls = []
+    handle = lin.register_forward_hook(lambda mod, args, out: calls.append(1))
+    ops.linear(x, lin)
+    handle.remove()
+    assert calls == [1]
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert ops.linear(x, lin)[0].dtype is torch.bfloat16
+    with FlopCounterMode(display=False) as counter:
+        ops.linear(x, lin)
+    assert counter.get_total_flops() == 2 * 256 * 64 * 32
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x, torch.ones_like(x))
+        assert torch.autograd.forward_ad.unpack_dual(ops.linear(dual, lin)[0]).tangent is not None
+    batched = torch.vmap(lambda t: ops.linear(t, lin)[0])(x.view(4, 64, 64))
+    assert batched.shape == (4, 64, 32)
+    assert ops.linear(x.t().contiguous().t(), lin)[0].shape == (256, 32)   # not contiguous
+    assert ops.linear(x[:0], lin)[0].shape == (0, 32)
