@@ -544,6 +544,13 @@ static int fwd_decode(const MiniAttnFwdParams* p, const ma::DecodePlan& d, void*
   a.rows = a.G * p->Nq;
   a.n_rb = d.n_rb;
   a.tiles = d.tiles;
+  a.small = (d.n_ctas + 1ll) <= 0x7fffffffll / d.total;
+  a.by_ctas = ma::fast_div(d.n_ctas);
+  a.by_tiles = ma::fast_div(d.tiles);
+  a.by_total = ma::fast_div(a.small ? static_cast<uint32_t>(d.total) : 1u);
+  a.by_rb = ma::fast_div(d.n_rb);
+  a.by_hkv = ma::fast_div(p->Hkv);
+  a.by_g = ma::fast_div(a.G);
   a.scale_log2 = (p->softmax_scale > 0.f ? p->softmax_scale : 1.0f / sqrtf((float)p->D)) * 1.4426950408889634f;
   if (scratch != nullptr) {
     uint8_t* base = static_cast<uint8_t*>(scratch);

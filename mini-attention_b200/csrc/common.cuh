@@ -100,6 +100,8 @@ struct DecodeArgs {
   int rows;                // G * Nq
   int n_rb;                // row blocks per (batch, KV head)
   int tiles;               // 64-key tiles of an item
+  int small;               // total * (CTAs + 1) < 2^31: tiles are found by the divisors below, in 32 bits
+  FastDiv by_ctas, by_tiles, by_total, by_rb, by_hkv, by_g;
   float scale_log2;
   float*  part_o;          // [2 * CTAs][rows of an item][D] fp32: pieces of cut items, un-normalised
   float2* part_ml;         // [2 * CTAs][rows of an item]: (row maximum in log2 units, row sum)

@@ -22,7 +22,10 @@
 // itself in; the CTA that counts in last folds the pieces and writes the rows.  Nobody waits.
 //
 // Measured (B200, 16 requests, 32/8 heads, 1 token against 4001 keys, D=128 bf16, 262 MB of K/V): 183 us
-// through fwd_ws.cu before that packed heads, 48 now, 46 us here = 5.7 TB/s, 0.87 of the measured copy bandwidth.
+// through fwd_ws.cu before that packed heads, 48 now, 45.6 us here = 5.7 TB/s, 0.88 of the measured copy bandwidth.  Short
+// calls are bound by their ends: with 64-bit divisions for a CTA's range and for every tile, and the first copies
+// after the CTA's first synchronisation, 8 KV heads of 500 keys took 7.2 us (5.25 now), 64 items of 9000 16.6 (13.4),
+// 4 x 32/8 heads of 1024 11.3 (10.2).
 #include <atomic>
 #include <type_traits>
 
@@ -44,7 +47,9 @@ template <int D>
 struct DecLayout {
   static constexpr int kBoxes = D / 64;
   static constexpr int kStageBytes = 2 * kBoxes * kDecBox;  // K then V
-  static constexpr int kStages = 96 * 1024 / kStageBytes;
+  // 64 KB of ring at D = 64 is enough, and more in flight wears on HBM: 64 items of 36002 keys 30.7 us in 96 KB, 29.5 in
+  // 64, 16 items of 30000 26.7 / 25.8.  At D = 128 a stage is 32 KB.
+  static constexpr int kStages = D == 64 ? 4 : 3;
   static constexpr int kOffMerge = kStages * kStageBytes;   // float[4 warps][16][kMergePitch]
   static constexpr int kOffMl = kOffMerge + 4 * 16 * kMergePitch * 4;  // float2[4 warps][16]
   static constexpr int kOffBar = kOffMl + 4 * 16 * 8;       // full[kStages], empty[kStages]
@@ -104,32 +109,48 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   const WaitCtx wc{abort_flag, a.status, MINIATTN_WAIT_LIMIT_NS};
   // this CTA's tiles [lo, hi) of the launch's total
   const long long n_ctas = gridDim.x;
-  const long long lo = blockIdx.x * a.total / n_ctas, hi = (blockIdx.x + 1) * a.total / n_ctas;
-
-  if (tid == 128) {
-    for (int s = 0; s < L::kStages; ++s) {
-      mbar_init(full(s), 1);
-      mbar_init(empty(s), 4);
-    }
-    *abort_flag = 0;
-    fence_mbar_init();
-    fence_proxy_async_smem();
-    prefetch_tmap(&tm_k);
-    prefetch_tmap(&tm_v);
-  }
-  __syncthreads();
-  grid_dep_wait();
+  auto first_tile = [&](long long cta) -> long long {
+    return a.small ? div_by(static_cast<int>(cta * a.total), a.by_ctas) : cta * a.total / n_ctas;
+  };
+  auto item_of = [&](long long x) -> int {
+    return a.small ? div_by(static_cast<int>(x), a.by_tiles) : static_cast<int>(x / a.tiles);
+  };
+  auto cta_of = [&](long long x) -> long long {  // that holds tile x
+    return a.small ? div_by(static_cast<int>((x + 1) * n_ctas - 1), a.by_total) : ((x + 1) * n_ctas - 1) / a.total;
+  };
+  const long long lo = first_tile(blockIdx.x), hi = first_tile(blockIdx.x + 1ll);
 
   if (warp == 4) {
-    if (lane == 0) {
-      int i = 0;
-      for (long long x = lo; x < hi; ++x, ++i) {
-        const int item = static_cast<int>(x / a.tiles);
-        const int t = static_cast<int>(x - static_cast<long long>(item) * a.tiles);
-        const int kvh = item / a.n_rb;
-        const int hk = kvh % a.Hkv, b = kvh / a.Hkv;
-        const int slot = i % L::kStages;
-        if (i >= L::kStages) mbar_wait(empty(slot), (i / L::kStages - 1) & 1, wc, kErrWaitFree);
+    // =========================== TMA producer ====================================
+    // The whole warp, one elected thread issues (a diverged thread takes several times as long), and it starts as
+    // soon as its barriers are there: the first stages are on their way while the workers fetch Q.
+    const bool issuer = elect_one();
+    if (issuer) {
+      for (int s = 0; s < L::kStages; ++s) {
+        mbar_init(full(s), 1);
+        mbar_init(empty(s), 4);
+      }
+      *abort_flag = 0;
+      fence_mbar_init();
+      fence_proxy_async_smem();
+      prefetch_tmap(&tm_k);
+      prefetch_tmap(&tm_v);
+    }
+    __syncwarp();
+    asm volatile("bar.arrive 2, 160;" ::: "memory");  // the workers look at the barriers from here on
+    grid_dep_wait();
+    int item = item_of(lo), t = static_cast<int>(lo - static_cast<long long>(item) * a.tiles);
+    int b, hk;
+    auto locate = [&]() {
+      const int kvh = div_by(item, a.by_rb);
+      b = div_by(kvh, a.by_hkv);
+      hk = kvh - b * a.Hkv;
+    };
+    locate();
+    int slot = 0, par = 1, i = 0;
+    for (long long x = lo; x < hi; ++x, ++i) {
+      if (i >= L::kStages) mbar_wait(empty(slot), par, wc, kErrWaitFree);
+      if (issuer) {
         mbar_expect_tx(full(slot), L::kStageBytes);
         const uint32_t dst = sbase + slot * L::kStageBytes;
 #pragma unroll
@@ -139,16 +160,28 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
         for (int bx = 0; bx < L::kBoxes; ++bx)
           tma_load_4d(dst + (L::kBoxes + bx) * kDecBox, &tm_v, full(slot), bx * 64, t * kDecKeys, hk, b);
       }
-      // give-up path: let the copies in flight land (bounded) before the shared memory is released
-      if (*abort_flag) {
-        const uint64_t t0 = global_timer_ns();
-        while (global_timer_ns() - t0 < 2000000ull) {
-        }
+      __syncwarp();
+      if (++slot == L::kStages) {
+        slot = 0;
+        par ^= 1;
+      }
+      if (++t == a.tiles) {
+        t = 0;
+        ++item;
+        locate();
+      }
+    }
+    // give-up path: let the copies in flight land (bounded) before the shared memory is released
+    if (*abort_flag) {
+      const uint64_t t0 = global_timer_ns();
+      while (global_timer_ns() - t0 < 2000000ull) {
       }
     }
     __syncwarp();
     return;
   }
+  grid_dep_wait();
+  bool barriers_there = false;
 
   // ---------------------------------------------------------------- workers
   const int rg = warp % RG, kg = warp / RG;
@@ -162,12 +195,12 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
   int i = 0;  // ring index
 
   for (long long x = lo; x < hi;) {
-    const int item = static_cast<int>(x / a.tiles);
+    const int item = item_of(x);
     const long long item0 = static_cast<long long>(item) * a.tiles;
     const int t0 = static_cast<int>(x - item0);
     const int t1 = static_cast<int>(min(static_cast<long long>(a.tiles), hi - item0));
-    const int rb = item % a.n_rb, kvh = item / a.n_rb;
-    const int hk = kvh % a.Hkv, b = kvh / a.Hkv;
+    const int kvh = div_by(item, a.by_rb), rb = item - kvh * a.n_rb;
+    const int b = div_by(kvh, a.by_hkv), hk = kvh - b * a.Hkv;
     const int row0 = rb * kRows;
 
     // Q fragments of this warp's 16 rows, and how many keys its two rows of this lane may see.  Ordinary
@@ -178,7 +211,7 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int r = row0 + rg * 16 + g + 8 * e;
-      const int tok = r / a.G;
+      const int tok = div_by(r, a.by_g);
       long long v = a.Nk;
       if (a.causal) v = min(v, a.diag + tok + 1);
       const bool ok = r < a.rows;
@@ -199,6 +232,8 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    if (!barriers_there) asm volatile("bar.sync 2, 160;" ::: "memory");
+    barriers_there = true;
 
     for (int t = t0; t < t1; ++t, ++i) {
       const int slot = i % L::kStages;
@@ -332,7 +367,7 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       f[e] = part_weight(m_run[e], mt);
       if (whole) f[e] *= lt > 0.f ? 1.f / lt : 0.f;
     }
-    const long long c_first = ((item0 + 1) * n_ctas - 1) / a.total;  // CTA that holds the item's tile 0
+    const long long c_first = whole ? 0 : cta_of(item0);  // CTA that holds the item's tile 0
     const long long my_slot = 2ll * blockIdx.x + (t0 == 0 ? 1 : 0);
     if (tid < kRows && row0 + tid < a.rows) {
       const int rgi = tid >> 4, rr = tid & 15;
@@ -345,13 +380,13 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
       if (!whole) {
         a.part_ml[my_slot * kRows + tid] = make_float2(mt, lt);
       } else if (a.lse != nullptr) {
-        const int r = row0 + tid, tok = r / a.G, h = hk * a.G + (r - tok * a.G);
+        const int r = row0 + tid, tok = div_by(r, a.by_g), h = hk * a.G + (r - tok * a.G);
         a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Nq + tok] =
             lt > 0.f ? mt * 0.6931471805599453f + __logf(lt) : -INFINITY;
       }
     }
     auto store_row = [&](int r_in, int col, const float4& o) {  // four columns of a finished row
-      const int r = row0 + r_in, tok = r / a.G, h = hk * a.G + (r - tok * a.G);
+      const int r = row0 + r_in, tok = div_by(r, a.by_g), h = hk * a.G + (r - tok * a.G);
       uint2 w;
       w.x = pack2<BF16>(o.x, o.y);
       w.y = pack2<BF16>(o.z, o.w);
@@ -392,7 +427,7 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
     if (!whole) {
       __threadfence();  // release: the piece before the count
       workers_sync();
-      const long long c_last = ((item0 + a.tiles) * n_ctas - 1) / a.total;
+      const long long c_last = cta_of(item0 + a.tiles - 1);
       const int n_parts = static_cast<int>(c_last - c_first + 1);
       if (tid == 0) {
         __threadfence();
@@ -460,7 +495,7 @@ fwd_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constan
               o[u].w *= inv;
               if (col < a.D) store_row(r_in, col, o[u]);
               if (col == 0 && a.lse != nullptr) {
-                const int r = row0 + r_in, tok = r / a.G, h = hk * a.G + (r - tok * a.G);
+                const int r = row0 + r_in, tok = div_by(r, a.by_g), h = hk * a.G + (r - tok * a.G);
                 a.lse[(static_cast<long long>(b) * a.Hq + h) * a.Nq + tok] =
                     lt[u] > 0.f ? mt[u] * 0.6931471805599453f + __logf(lt[u]) : -INFINITY;
               }
