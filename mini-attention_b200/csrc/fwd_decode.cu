@@ -9,7 +9,7 @@
 //   item      = (batch, KV head, block of 16*RG rows);  T tiles of 64 keys each
 //   CTA       = a contiguous range of the tiles of all items, the same length for every CTA of the
 //               launch; plan_decode (plan.cu) says how many and which calls come here at all
-//   warp 4    TMA producer: K and V boxes (64 keys, 128-byte swizzle) through a ring, 96 KB deep,
+//   warp 4    TMA producer: K and V boxes (64 keys, 128-byte swizzle) through a ring, 96 KB deep (64 KB at D = 64),
 //             192 KB in flight per SM
 //   warps 0-3 16 rows x (16*RG keys of the tile) each: RG row groups x 4/RG key groups, each warp
 //             with its own running (m, l, O) in registers -- no CTA-wide step inside the loop

@@ -8,7 +8,7 @@
 //               epilogue (O / l -> 16 bit -> swizzled smem -> TMA store); they also rescale the
 //               tile's O accumulator in TMEM where a row maximum moved (rare)
 //   warps 4-7   the same for Q tile 1
-//   warp 8      MMA issuer of Q tile 0 (one thread issues its tcgen05.mma stream)
+//   warp 8      MMA issuer of Q tile 0 (the converged warp walks the stream, an elected thread issues)
 //   warp 10     MMA issuer of Q tile 1
 //   warp 9      TMA producer: Q tiles once, then K_0, V_0, K_1, V_1, ... through a ring
 //   warp 11     idle (donates its registers)
@@ -23,22 +23,21 @@
 //   S0a [0,64) S0b [64,128) S1a [128,192) S1b [192,256)   O0 [256,256+D)  O1 [256+D,256+2D)
 //
 // MMA order per Q tile and K/V tile j:  PV_a(j) S_a(j+1) PV_b(j) S_b(j+1); the two tiles have
-// one issuing thread each and the tensor pipe interleaves their streams.
+// one issuing warp each and the tensor pipe interleaves their streams.
 //
 // The reference that a row's exponentials are taken against is updated lazily: it stays what it is, and
 // no maximum is searched for, until the sum of a half's exponentials exceeds 2^8; only then the row's
 // maximum is found, O and l are rescaled, and the half is taken again.  l is accumulated against the same
 // reference, which keeps O / l exact.
 //
-// What bounds it (N = 2048, D = 128, per 128-key step of a CTA, about 2660 clk; 2950 while the issuing threads put
-// every descriptor together anew): the MMAs of a step need 2608 clk of the tensor pipe, and they and TMA 2560 clk of
+// What bounds it (N = 2048, D = 128, per 128-key step of a CTA, 2615 to 2640 clk; 2950 while the issuing threads put
+// every descriptor together anew): the MMAs of a step need 2577 clk of the tensor pipe, and they and TMA 2560 clk of
 // the 128 B/clk shared-memory port (Q is re-read for each half).  With that slower issue, finding the maximum of a
 // half first and handing the factor to four correction warps took 3956 us for 16 heads at N = 32768, 3743 with the
 // maximum found beside the exponentials, 3685 without one.  At D = 64 the softmax thread is the bound: N = 8192
 // (2 x 16 heads) 706 / 694 / 654 us, 609 with the present issue.  One MMA of 128 keys for S (2080 clk of tensor work)
 // measured slower, 49 against 41 us at N = 2048: TMEM has room for one S buffer per Q tile then, and the thread waits
-// 1600 clk per step for PV
-// and the next S.
+// 1600 clk per step for PV and the next S.
 //
 // Softmax arithmetic runs two scores per issue slot (packed f32x2 FMA / ADD); a share of the
 // exponentials is evaluated by a polynomial on the FMA pipe instead of the exp2 unit.
