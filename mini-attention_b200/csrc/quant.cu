@@ -10,7 +10,11 @@
 // become resident while stage 1 drains and load their K slabs before they wait for stage 1's
 // column sums, so the second launch's ramp and first loads hide under the first one's tail; stage 1 stands in
 // the same relation to the kernel before it, and the attention kernel to stage 2.
-// HBM-bound byte movers: 16-byte loads, 8-byte int8 stores, one CTA per
+// What bounds them: HBM and the loads of a CTA that waits for its own slab, after the instructions were the bound.  With
+// one score at a time, a branch for each, a margin around a tie that sent 6 % of the warps' elements through a division, and (bf16)
+// the unpacked slab held in registers, the pre-pass took, us fp16 / bf16: 2 x 16 heads, 8192 tokens, D = 64 37.0 / 39.4, now
+// 30.7 / 32.6 (134 MB, 4.4 TB/s); 2 x 64/16 heads, 8265, D = 128 144.9 / 214.6, now 117.9 / 132.5 (576 MB, 4.9).
+// 16-byte loads, 8-byte int8 stores, one CTA per
 // (128-token block, head, batch) or per 1024-token column-sum chunk.  Algorithmic traffic per element: K 2 B (mean pass) + 2 B + 1 B,
 // Q 2 B + 1 B, plus 4 B per 128 x D slab for the scale.
 // What these kernels read is not declared __restrict__: the compiler would take it for read-only over the whole
@@ -51,7 +55,42 @@ __device__ __forceinline__ void unpack8(const uint4& w, float (&f)[8]) {
   }
 }
 
+// Pairs of fp32 in 64-bit registers, low word first: one issue slot for two.  Subnormal numbers are kept, as in the
+// scalar operations of the same rounding.
+__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 halves_of(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_mul(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 constexpr int kSumRows = 1024;  // tokens per partial column sum
+constexpr float kNearTie = 1e-4f;
+// CTAs of an SM that the registers are made to allow.  Free choice takes 58 (D = 64) and 78 registers, 4 and 3 CTAs; one
+// more (48 and 64, a few spilled around the rare division) measured, us for both launches of the pre-pass, fp16 / bf16:
+// 2 x 16 heads, 8192 tokens, D = 64 32.2 / 34.5 -> 30.7 / 32.6; 2 x 64/16 heads, 8265, D = 128 122.4 / 138.5 -> 117.9 / 132.5.
+// Two more at D = 64 (40 registers) 33.3 / 35.4.
+template <int D>
+constexpr int kCtasPerSm = D == 64 ? 5 : 4;
 
 }  // namespace
 
@@ -64,18 +103,18 @@ __device__ __forceinline__ void colsum_body(const uint16_t* k, long long sb, lon
   constexpr int RPP = 256 / CPR;      // rows per pass
   const int col8 = threadIdx.x % CPR, r0 = threadIdx.x / CPR;
   const uint16_t* base = k + b * sb + h * sh;
-  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  uint64_t acc2[4] = {0, 0, 0, 0};
   const int row_end = min(N, (chunk + 1) * kSumRows);
   for (int row = chunk * kSumRows + r0; row < row_end; row += RPP) {
     const uint4 w = *reinterpret_cast<const uint4*>(base + row * sn + col8 * 8);
     float f[8];
     unpack8<BF16>(w, f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += f[i];
+    for (int i = 0; i < 4; ++i) acc2[i] = pair_add(acc2[i], pair_of(f[2 * i], f[2 * i + 1]));
   }
-  __shared__ float red[RPP][D];
+  __shared__ __align__(16) float red[RPP][D];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) red[r0][col8 * 8 + i] = acc[i];
+  for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(&red[r0][col8 * 8 + 2 * i]) = halves_of(acc2[i]);
   __syncthreads();
   if (threadIdx.x < D) {
     float s = 0.f;
@@ -95,7 +134,7 @@ __device__ __forceinline__ void quant_body(const uint16_t* x, long long sb, long
                                            int n_blocks) {
   constexpr int CPR = D / 8;
   constexpr int PER = 16 * D / 256;  // chunks per thread (128 rows * D/8 chunks / 256 threads)
-  __shared__ float mean[D];
+  __shared__ __align__(16) float minus_mean[D];
   __shared__ float wmax[8];
   const uint16_t* base = x + b * sb + h * sh;
   // The slab stays in registers as loaded (16-bit pairs) and is unpacked twice, once for the
@@ -119,23 +158,35 @@ __device__ __forceinline__ void quant_body(const uint16_t* x, long long sb, long
       const float* p = partial + (static_cast<long long>(b) * H + h) * n_chunks * D + threadIdx.x;
       for (int c = 0; c < n_chunks; ++c) s += p[c * D];
       const float m = s / static_cast<float>(N);
-      mean[threadIdx.x] = m;
+      minus_mean[threadIdx.x] = -m;
       if (blk == 0 && mean_out != nullptr) mean_out[(static_cast<long long>(b) * H + h) * D + threadIdx.x] = m;
     }
     __syncthreads();
   }
+  auto load = [&](int i, int col8, uint64_t (&x2)[4]) {  // chunk i of this thread, smoothed
+    float f[8];
+    unpack8<BF16>(raw[i], f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      x2[e] = pair_of(f[2 * e], f[2 * e + 1]);
+      if (SMOOTH) {
+        const float2 m = *reinterpret_cast<const float2*>(minus_mean + col8 * 8 + 2 * e);
+        x2[e] = pair_add(x2[e], pair_of(m.x, m.y));
+      }
+    }
+  };
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int id = threadIdx.x + i * 256;
     const int row = blk * 128 + id / CPR, col8 = id % CPR;
     if (row < N) {
-      float f[8];
-      unpack8<BF16>(raw[i], f);
+      uint64_t x2[4];
+      load(i, col8, x2);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (SMOOTH) f[e] -= mean[col8 * 8 + e];
-        amax = fmaxf(amax, fabsf(f[e]));
+      for (int e = 0; e < 4; ++e) {
+        const float2 f = halves_of(x2[e]);
+        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
       }
     }
   }
@@ -156,29 +207,43 @@ __device__ __forceinline__ void quant_body(const uint16_t* x, long long sb, long
     const int id = threadIdx.x + i * 256;
     const int row = blk * 128 + id / CPR, col8 = id % CPR;
     if (row < N) {
-      float f[8];
-      unpack8<BF16>(raw[i], f);
-      uint32_t lo = 0, hi = 0;
+      // round-half-even(x / scale), bit for bit, without a division per element: y = x * (1/scale) and the rounded
+      // quotient are each within 1.6e-5 of the true one, and adding 1.5*2^23 rounds y to the nearest integer (ties to
+      // even), whose low byte is then the sum's.  Only where y lies within kNearTie of a tie can the two differ: one
+      // element in 5000, one look at the largest distance for eight.
+      uint64_t x2[4], sum[4];
+      // or the compiler keeps the first pass's fp32 values: 106 instead of 78 registers at D = 128 bf16
+      asm volatile("" : "+r"(raw[i].x), "+r"(raw[i].y), "+r"(raw[i].z), "+r"(raw[i].w));
+      load(i, col8, x2);
+      const uint64_t inv2 = pair_of(inv, inv), big = pair_of(12582912.f, 12582912.f);
+      const uint64_t minus_big = pair_of(-12582912.f, -12582912.f), minus_one = pair_of(-1.f, -1.f);
+      uint64_t d2[4];
+      float far = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (SMOOTH) f[e] -= mean[col8 * 8 + e];
-        // round-half-even(x / scale), bit for bit, without a division per element: y = x * (1/scale)
-        // is within 2e-5 of the true quotient, and adding 1.5*2^23 rounds it to the nearest integer
-        // (ties to even) in the low mantissa bits.  Only when y lies within 1e-3 of a tie can the
-        // two roundings differ; those elements (about 0.2 %) take the exact division.
-        const float y = f[e] * inv;
-        const float t = y + 12582912.f;
-        const float d = y - (t - 12582912.f);
-        int qv;
-        if (fabsf(d) > 0.499f) {
-          qv = __float2int_rn(__fdiv_rn(f[e], scale));
-          qv = max(-127, min(127, qv));
-        } else {
-          qv = __float_as_int(t) - 0x4B400000;
-        }
-        if (e < 4) lo |= (static_cast<uint32_t>(qv) & 0xFFu) << (8 * e);
-        else hi |= (static_cast<uint32_t>(qv) & 0xFFu) << (8 * (e - 4));
+      for (int e = 0; e < 4; ++e) {
+        const uint64_t y = pair_mul(x2[e], inv2);
+        sum[e] = pair_add(y, big);
+        d2[e] = pair_fma(pair_add(sum[e], minus_big), minus_one, y);
+        const float2 d = halves_of(d2[e]);
+        far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
       }
+      uint32_t t[8];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 w = halves_of(sum[e]);
+        t[2 * e] = __float_as_uint(w.x);
+        t[2 * e + 1] = __float_as_uint(w.y);
+      }
+      if (far > 0.5f - kNearTie) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float2 d = halves_of(d2[e >> 1]), f = halves_of(x2[e >> 1]);
+          if (fabsf((e & 1) ? d.y : d.x) > 0.5f - kNearTie)
+            t[e] = static_cast<uint32_t>(max(-127, min(127, __float2int_rn(__fdiv_rn((e & 1) ? f.y : f.x, scale)))));
+        }
+      }
+      const uint32_t lo = __byte_perm(__byte_perm(t[0], t[1], 0x0040), __byte_perm(t[2], t[3], 0x0040), 0x5410);
+      const uint32_t hi = __byte_perm(__byte_perm(t[4], t[5], 0x0040), __byte_perm(t[6], t[7], 0x0040), 0x5410);
       *reinterpret_cast<uint2*>(obase + static_cast<long long>(row) * D + col8 * 8) = make_uint2(lo, hi);
     }
   }
@@ -187,7 +252,7 @@ __device__ __forceinline__ void quant_body(const uint16_t* x, long long sb, long
 // Stage 1, one launch: the Q quantiser (nothing depends on it but the attention kernel) and the
 // partial column sums of K.  The first gridDim.x - q_blocks blocks sum K, the rest quantise Q.
 template <int D, bool BF16>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kCtasPerSm<D>)
 prepass_stage1_kernel(const uint16_t* q, long long qsb, long long qsh, long long qsn, int Nq,
                       int Hq, int nqb, int8_t* __restrict__ q8, float* __restrict__ sq, float fold,
                       const uint16_t* k, long long ksb, long long ksh, long long ksn, int Nk,
@@ -212,7 +277,7 @@ prepass_stage1_kernel(const uint16_t* q, long long qsb, long long qsh, long long
 
 // Stage 2: smooth and quantise K (needs every column sum of stage 1).
 template <int D, bool BF16>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kCtasPerSm<D>)
 quant_k_kernel(const uint16_t* k, long long sb, long long sh, long long sn, int N,
                const float* partial, int n_chunks, int8_t* __restrict__ k8,
                float* __restrict__ scale_out, float* __restrict__ mean_out) {
