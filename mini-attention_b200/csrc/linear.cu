@@ -32,7 +32,6 @@ constexpr int kBBytes = kLinearMaxBn / 2 * kK * 2;
 constexpr int kStageBytes = kABytes + kBBytes;
 constexpr int kStoreCols = 16;        // columns of a store box: 32 rows x 32 bytes
 constexpr int kStoreBytes = 32 * kStoreCols * 2;
-constexpr int kStoreBufs = 4;         // boxes of a warp in flight
 constexpr int kOffStore = kStages * kStageBytes;
 constexpr int kOffBar = kOffStore + 8 * kStoreBufs * kStoreBytes;
 constexpr int kBarFull = 0, kBarEmpty = kStages, kBarAccFull = 2 * kStages, kBarAccFree = kBarAccFull + 2;
@@ -96,6 +95,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
     const uint32_t acc_free = mapa(bar(kBarAccFree), 0);
     const int n_box = a.bn / kStoreCols;
     int done = 0;  // tiles of this pair so far
+    StoreTurn turn;
     for (int tile = first; tile < a.n_tiles; tile += step, ++done) {
       int m0, seg, n0;
       locate(tile, &m0, &seg, &n0);
@@ -134,7 +134,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
 #pragma unroll
         for (int i = 0; i < 8; ++i)
           w[i] = pack2<BF16>(__uint_as_float(u[2 * i]) + bv[2 * i], __uint_as_float(u[2 * i + 1]) + bv[2 * i + 1]);
-        const uint32_t box = stage + ((bx >> 1) % kStoreBufs) * kStoreBytes;
+        const uint32_t box = stage + turn.take() * kStoreBytes;
         if (lane == 0) tma_store_wait_read<kStoreBufs - 1>();
         __syncwarp();
         const uint32_t at = box + lane * (kStoreCols * 2);

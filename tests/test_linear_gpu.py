@@ -24,7 +24,8 @@ def _launch(x, ws, bs, ys, only_if_faster=0):
 
 
 # M, K, N...: one row to several row tiles, edges of 32, 128 and 256 rows; K below, at and past a stage of 64 and past
-# the ring; N of one box of 16 columns, not a multiple of 16, and several tiles; more tiles than pairs of SMs
+# the ring; N of one box of 16 columns, not a multiple of 16, and several tiles; two tiles for a pair of SMs in the last
+# but one
 CASES = [
     (1, 8, (8,)), (31, 64, (16,)), (33, 72, (24, 40)), (128, 256, (256, 64, 8)), (129, 520, (104, 264)), (255, 448, (48,)),
     (256, 128, (512,)), (257, 1000, (72, 136)), (1000, 1024, (1024, 256)), (2300, 192, (1536, 1544)), (5000, 96, (512, 128)),
@@ -50,6 +51,37 @@ def test_linear_against_fp64(M, K, N, dtype):
         bound = ulp * ref.abs() + K * 2.0 ** -24 * size + 2.0 ** -24
         assert bool(((y.double() - ref).abs() <= bound).all())
         assert bool((t[0] == 7).all() and (t[-1] == 7).all() and (t[:, :8] == 7).all() and (t[:, -8:] == 7).all())
+
+
+# Three and more tiles for a pair of SMs and few stages of K, so that the next accumulator is there before the copies of
+# the tile before have read their buffers; boxes of a warp and tile that the buffers do not divide (1, 3, 5, 6, 7)
+# and tiles cut short by the last column.  The sums' order is fixed: every launch gives the first one's result.
+MANY_TILES = [
+    (16384, 64, (64, 64, 64)), (32768, 64, (64, 64, 64)), (40000, 64, (64, 128)), (16384, 320, (320, 128)),
+    (40000, 320, (320, 640)), (60001, 8, (16,)), (20000, 24, (352, 184)), (9000, 128, (1000, 520, 264)),
+]
+
+
+@pytest.mark.parametrize("M,K,N", MANY_TILES)
+def test_many_tiles_of_a_pair(M, K, N):
+    dtype = torch.bfloat16
+    g = torch.Generator(device=DEV).manual_seed(M + K)
+    x = torch.randn(M, K, device=DEV, generator=g).to(dtype)
+    ws = [torch.randn(n, K, device=DEV, generator=g).to(dtype) for n in N]
+    bs = [torch.randn(n, device=DEV, generator=g).to(dtype) for n in N]
+    first = [torch.empty(M, n, dtype=dtype, device=DEV) for n in N]
+    assert _launch(x, ws, bs, first) == _lib.OK
+    for w, b, y in zip(ws, bs, first):
+        ref = x.double() @ w.double().T + b.double()
+        size = x.double().abs() @ w.double().abs().T + 4.0
+        assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + K * 2.0 ** -24 * size + 2.0 ** -24).all())
+    differ = torch.zeros((), dtype=torch.int64, device=DEV)
+    for _ in range(100):
+        ys = [torch.full_like(y, 7.0) for y in first]
+        assert _launch(x, ws, bs, ys) == _lib.OK
+        for y, want in zip(ys, first):
+            differ += (y.view(torch.int16) != want.view(torch.int16)).sum()
+    assert int(differ) == 0 and miniattn.device_status(DEV) == 0
 
 
 def test_linear_with_a_strided_row_of_one():
