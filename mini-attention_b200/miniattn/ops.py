@@ -569,6 +569,25 @@ def _nobody_watches() -> bool:
                 or _nn_module._global_backward_pre_hooks)
 
 
+def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: bool):
+    """(weight, bias or None) of a layer whose own call is x weight^T + bias and nothing else, over `k` inputs of dtype
+    `dt` on device `dev`, in the form ``miniattn_linear`` takes; None for any other layer."""
+    own = layer.__dict__
+    w, b = own["_parameters"].get("weight"), own["_parameters"].get("bias", False)  # False: not a parameter, or not there
+    if (type(layer) is not _Linear or type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
+            or "forward" in own or "weight" in own or "bias" in own or own["_forward_hooks"] or own["_forward_pre_hooks"]
+            or own["_backward_hooks"] or own["_backward_pre_hooks"] or w.dim() != 2
+            or not w.is_contiguous() or (grad and w.requires_grad)):
+        return None
+    n, wk = w.shape
+    if wk != k or n % 8 or n == 0 or w.data_ptr() % 16:
+        return None
+    if b is not None and (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.dim() != 1
+                          or b.numel() != n or not b.is_contiguous() or (grad and b.requires_grad)):
+        return None
+    return w, b
+
+
 def linear(x: torch.Tensor, *layers: torch.nn.Linear):
     """``[layer(x) for layer in layers]`` for up to three linear layers that share their input.
 
@@ -585,27 +604,14 @@ def linear(x: torch.Tensor, *layers: torch.nn.Linear):
             p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
             out = []
             for i, layer in enumerate(layers):
-                own = layer.__dict__
-                w, b = own["_parameters"].get("weight"), own["_parameters"].get("bias")
-                if (type(layer) is not _Linear or type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
-                        or "forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"]
-                        or own["_backward_hooks"] or own["_backward_pre_hooks"] or w.dim() != 2
-                        or not w.is_contiguous() or (grad and w.requires_grad)):
+                wb = _operands(layer, k, dt, dev, grad)
+                if wb is None:
                     p = None
                     break
-                n, wk = w.shape
-                wp, bp = w.data_ptr(), None
-                if wk != k or n % 8 or n == 0 or wp % 16:
-                    p = None
-                    break
-                if b is not None:
-                    if (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.dim() != 1
-                            or b.numel() != n or not b.is_contiguous() or (grad and b.requires_grad)):
-                        p = None
-                        break
-                    bp = b.data_ptr()
+                w, b = wb
+                n = w.shape[0]
                 y = x.new_empty((*shape[:-1], n))
-                p.out[i] = (wp, bp, y.data_ptr(), k, n, n)
+                p.out[i] = (w.data_ptr(), None if b is None else b.data_ptr(), y.data_ptr(), k, n, n)
                 out.append(y)
     if p is None:
         return [layer(x) for layer in layers]

@@ -4,6 +4,7 @@ import ctypes as C
 import subprocess
 from pathlib import Path
 
+import pytest
 import torch
 
 from miniattn import _lib, ops
@@ -48,3 +49,37 @@ def test_cpu_tensors_go_through_the_layers():
     x = torch.randn(3, 5, 16)
     for y, layer in zip(ops.linear(x, *layers), layers):
         assert torch.equal(y, layer(x)) and y.requires_grad
+
+
+def _layer(bias=True):
+    return torch.nn.Linear(16, 8, bias=bias).half().requires_grad_(False)
+
+
+def _taken(layer):
+    return ops._operands(layer, 16, torch.float16, -1, True) is not None   # -1: the CPU's device index
+
+
+def _bias_as(kind):
+    layer = _layer()
+    bias = layer.bias.detach().clone()
+    if kind == "shadowed":
+        layer.__dict__["bias"] = bias
+        return layer
+    del layer.bias
+    if kind == "buffer":
+        layer.register_buffer("bias", bias)
+    elif kind == "attribute":
+        layer.bias = bias
+    return layer
+
+
+def test_plain_layers_are_taken():
+    layer = _layer()
+    assert _taken(layer) and _taken(_layer(bias=False))
+    w, b = ops._operands(layer, 16, torch.float16, -1, True)
+    assert w is layer.weight and b is layer.bias
+
+
+@pytest.mark.parametrize("kind", ["buffer", "attribute", "missing", "shadowed"])
+def test_a_bias_that_is_no_parameter_is_left_to_the_layer(kind):
+    assert not _taken(_bias_as(kind))

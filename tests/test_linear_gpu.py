@@ -151,3 +151,16 @@ def test_calls_that_something_watches_go_through_the_layers():
     assert batched.shape == (4, 64, 32)
     assert ops.linear(x.t().contiguous().t(), lin)[0].shape == (256, 32)   # not contiguous
     assert ops.linear(x[:0], lin)[0].shape == (0, 32)
+
+
+@pytest.mark.parametrize("register", [True, False])
+def test_a_bias_that_is_no_parameter_is_added(register):
+    lin = torch.nn.Linear(64, 32).half().to(DEV).requires_grad_(False)
+    bias = torch.full((32,), 100.0, dtype=torch.float16, device=DEV)
+    del lin.bias
+    if register:
+        lin.register_buffer("bias", bias)
+    else:
+        lin.bias = bias
+    x = torch.randn(256, 64, device=DEV, dtype=torch.float16)
+    assert torch.equal(ops.linear(x, lin)[0], lin(x))
