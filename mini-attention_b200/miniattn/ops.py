@@ -572,9 +572,11 @@ def _nobody_watches() -> bool:
 def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: bool):
     """(weight, bias or None) of a layer whose own call is x weight^T + bias and nothing else, over `k` inputs of dtype
     `dt` on device `dev`, in the form ``miniattn_linear`` takes; None for any other layer."""
+    if type(layer) is not _Linear:   # a scripted or traced layer keeps its parameters elsewhere
+        return None
     own = layer.__dict__
     w, b = own["_parameters"].get("weight"), own["_parameters"].get("bias", False)  # False: not a parameter, or not there
-    if (type(layer) is not _Linear or type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
+    if (type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
             or "forward" in own or "weight" in own or "bias" in own or own["_forward_hooks"] or own["_forward_pre_hooks"]
             or own["_backward_hooks"] or own["_backward_pre_hooks"] or w.dim() != 2
             or not w.is_contiguous() or (grad and w.requires_grad)):

@@ -83,3 +83,11 @@ def test_plain_layers_are_taken():
 @pytest.mark.parametrize("kind", ["buffer", "attribute", "missing", "shadowed"])
 def test_a_bias_that_is_no_parameter_is_left_to_the_layer(kind):
     assert not _taken(_bias_as(kind))
+
+
+@pytest.mark.parametrize("make", [
+    torch.jit.script, lambda layer: torch.jit.trace(layer, torch.randn(2, 16).half()), torch.nn.Sequential,
+    lambda layer: type("Own", (torch.nn.Linear,), {})(16, 8).half().requires_grad_(False), lambda layer: layer.forward,
+], ids=["scripted", "traced", "wrapped", "subclass", "function"])
+def test_other_callables_are_left_to_themselves(make):
+    assert not _taken(make(_layer()))
