@@ -557,16 +557,20 @@ def selftest_wait(limit_ms: float = 50.0, device: Union[torch.device, str, None]
 _Linear, _Parameter = torch.nn.Linear, torch.nn.Parameter
 _nn_module = torch.nn.modules.module
 _forward_ad = torch.autograd.forward_ad
+_functional = torch.nn.functional
+_linear_call, _linear_forward, _aten_linear = _Linear.__call__, _Linear.forward, torch._C._nn.linear
 
 
 def _nobody_watches() -> bool:
-    """No trace, mode, global hook, tangent or autocast that a call of an ``nn.Linear`` would take part in."""
+    """No trace, mode, global hook, tangent or autocast that a call of an ``nn.Linear`` would take part in, and nobody
+    has put a call, forward or ``F.linear`` of their own in the place of torch's."""
     c = torch._C
     return not (c._len_torch_dispatch_stack() or c._len_torch_function_stack() or c._functorch.peek_interpreter_stack()
                 or _forward_ad._current_level >= 0 or torch.is_autocast_enabled("cuda") or torch.jit.is_tracing()
                 or torch.compiler.is_compiling() or _nn_module._global_forward_hooks
                 or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
-                or _nn_module._global_backward_pre_hooks)
+                or _nn_module._global_backward_pre_hooks or _Linear.__call__ is not _linear_call
+                or _Linear.forward is not _linear_forward or _functional.linear is not _aten_linear)
 
 
 def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: bool):

@@ -91,3 +91,12 @@ def test_a_bias_that_is_no_parameter_is_left_to_the_layer(kind):
 ], ids=["scripted", "traced", "wrapped", "subclass", "function"])
 def test_other_callables_are_left_to_themselves(make):
     assert not _taken(make(_layer()))
+
+
+@pytest.mark.parametrize("owner,name", [(torch.nn.Linear, "forward"), (torch.nn.Linear, "__call__"),
+                                        (torch.nn.Module, "__call__"), (torch.nn.functional, "linear")])
+def test_a_replaced_call_of_every_linear_layer_is_seen(owner, name, monkeypatch):
+    assert ops._nobody_watches()
+    was = getattr(owner, name)
+    monkeypatch.setattr(owner, name, lambda *args, **kw: was(*args, **kw))
+    assert not ops._nobody_watches()
