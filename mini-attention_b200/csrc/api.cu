@@ -42,7 +42,6 @@ cudaError_t launch_quant_qk_static(int D, bool bf16, const void* q, const long l
                                    const long long* ks, int B, int Hq, int Hkv, int Nq, int Nk,
                                    float q_fold, int8_t* q8, int8_t* k8, float* sq, float* sk,
                                    float* k_mean, cudaStream_t st);
-int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* pays);
 cudaError_t launch_linear(bool bf16, const LinearArgs& a, int pairs, cudaStream_t st);
 cudaError_t launch_wait_selftest(int32_t* status, unsigned long long limit_ns, cudaStream_t st);
 cudaError_t launch_merge_partials(float* acc_o, float* acc_lse, const void* part_o,
@@ -942,7 +941,7 @@ int miniattn_linear(const MiniAttnLinearParams* p, void* stream) {
   a.K = p->K;
   a.n_seg = p->n_out;
   if ((rc = make_map_2d(&a.tm_x, p->x, dt, p->M, p->K, p->ldx, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B, "x")) != 0) return rc;
-  int tiles = 0;
+  long long tiles = 0;
   for (int i = 0; i < p->n_out; ++i) {
     const MiniAttnLinearOut& o = p->out[i];
     ma::LinearSeg& s = a.seg[i];
@@ -952,8 +951,8 @@ int miniattn_linear(const MiniAttnLinearParams* p, void* stream) {
     s.bias = static_cast<const uint16_t*>(o.bias);
     s.N = o.N;
     s.bias_16 = reinterpret_cast<uintptr_t>(o.bias) % 16 == 0;
-    a.first_tile[i] = tiles;
-    tiles += (o.N + a.bn - 1) / a.bn;
+    a.first_tile[i] = static_cast<int>(tiles);
+    tiles += (o.N + (a.bn - 1ll)) / a.bn;
   }
   const long long m_tiles = (p->M + 255ll) / 256;
   if (tiles * m_tiles > 0x3fffffffll) return fail(MINIATTN_EUNSUPPORTED, "too many tiles");

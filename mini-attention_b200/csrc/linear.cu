@@ -59,7 +59,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
   const int lane = tid & 31;
   const int rank = static_cast<int>(cluster_rank());
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
-  const int n_k = (a.K + kK - 1) / kK;
+  const int n_k = (a.K - 1) / kK + 1;
 
   if (warp == kWarpTma) {
     for (int i = lane; i < kNumBars; i += 32) mbar_init(bar(i), i >= kBarAccFree ? 16 : 1);
@@ -102,12 +102,12 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
       const int buf = done & 1;
       const CUtensorMap* tm = &a.seg[seg].tm_y;
       const uint16_t* bias = a.seg[seg].bias;
-      const int n = a.seg[seg].N;
+      const uint32_t n = a.seg[seg].N;
       mbar_wait(bar(kBarAccFull + buf), (done >> 1) & 1, wc, kErrWaitS);
       tc_fence_after();
       const uint32_t tA = tmem_base + buf * 256 + (static_cast<uint32_t>(quad * 32) << 16);
       for (int bx = half; bx < n_box; bx += 2) {
-        const int col = n0 + bx * kStoreCols;
+        const uint32_t col = static_cast<uint32_t>(n0) + bx * kStoreCols;  // may pass 2^31 in the last tile
         if (col >= n) break;
         uint32_t u[16];
         tmem_ld16(tA + bx * kStoreCols, u);
@@ -144,7 +144,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
         __syncwarp();
         if (lane == 0) {
           const int row = m0 + rank * kRows + quad * 32;
-          if (row < a.M) tma_store_2d(tm, box, col, row);
+          if (row < a.M) tma_store_2d(tm, box, static_cast<int>(col), row);
           tma_store_commit();
         }
       }
@@ -197,7 +197,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
           const uint32_t dst = sbase + stage * kStageBytes;
           if (rank == 0) mbar_expect_tx(bar(kBarFull + stage), 2 * (kABytes + b_rows * kK * 2));
           tma_load_2d_pair(dst, &a.tm_x, full + 8 * stage, k * kK, m0 + rank * kRows);
-          tma_load_2d_pair(dst + kABytes, &a.seg[seg].tm_w, full + 8 * stage, k * kK, n0 + rank * b_rows);
+          tma_load_2d_pair(dst + kABytes, &a.seg[seg].tm_w, full + 8 * stage, k * kK, static_cast<int>(static_cast<uint32_t>(n0) + rank * b_rows));
         }
         __syncwarp();
         if (++stage == kStages) {
@@ -226,37 +226,6 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
 }
 
 }  // namespace
-
-// Width of a tile: fewest clocks over the rounds of tiles, at bn / 2 clk for 16 columns of K and about 1500 a tile.
-// pays: whether that is expected to be no slower than a library GEMM for each weight, which reaches 0.92 of the tensor
-// rate at these sizes; either takes about 2 us a launch beside its work.  Measured, us of device time for the whole of
-// GQA_Flash in bf16, the layers' own calls / x's projections in one launch / the output's too: 2 x 1024 tokens, 16/4
-// heads of 128 52.6 / 49.9 / 50.4 (host-bound without a graph: 90.8 / 81.8 / 56.3); 1 x 4096, 32/8 heads 398 / 377 / 374;
-// 4 x 4096, 32/8 1766 / 1581 / 1570; 2 x 777, 24/8, where 1554 rows leave a seventh of the last row tiles 76.0 / 78.6 /
-// 83.2: not taken.  A launch of up to 13 us is taken in any case: the calls of the layers then take the host longer
-// than the GPU (1 x 512 tokens, 8/2 heads of 64: 66.5 us a call with them, 56.4 without, 16 on the device either way).
-int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* pays) {
-  const long long m_tiles = (M + 2 * kRows - 1) / (2 * kRows);
-  long long best = -1;
-  int bn = kLinearMaxBn;
-  for (int w = kLinearMaxBn; w >= 64; w -= 16) {
-    long long tiles = 0;
-    for (int i = 0; i < n_seg; ++i) tiles += (N[i] + w - 1) / w;
-    tiles *= m_tiles;
-    const long long rounds = (tiles + pairs - 1) / pairs;
-    const long long per_mma = w / 2 > 48 ? w / 2 : 48;  // narrower ones wait for shared memory
-    const long long clk = rounds * (per_mma * ((K + 15) / 16) + 1500);
-    if (best < 0 || clk < best) {
-      best = clk;
-      bn = w;
-    }
-  }
-  double macs = 0.;
-  for (int i = 0; i < n_seg; ++i) macs += static_cast<double>(M) * N[i] * K;
-  const double launch = 3700.;
-  *pays = best + launch <= 1.08 * (macs / (2. * pairs * 4096. * 0.92) + n_seg * launch) || best + launch <= 24000.;
-  return bn;
-}
 
 cudaError_t launch_linear(bool bf16, const LinearArgs& a, int pairs, cudaStream_t st) {
   static std::atomic<unsigned long long> smem_set[2] = {};

@@ -554,6 +554,7 @@ def selftest_wait(limit_ms: float = 50.0, device: Union[torch.device, str, None]
     return int(status.item())
 
 
+_INT32_MAX = 2 ** 31 - 1
 _Linear, _Parameter = torch.nn.Linear, torch.nn.Parameter
 _nn_module = torch.nn.modules.module
 _forward_ad = torch.autograd.forward_ad
@@ -586,7 +587,7 @@ def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: b
             or not w.is_contiguous() or (grad and w.requires_grad)):
         return None
     n, wk = w.shape
-    if wk != k or n % 8 or n == 0 or w.data_ptr() % 16:
+    if wk != k or n % 8 or not 0 < n <= _INT32_MAX or w.data_ptr() % 16:
         return None
     if b is not None and (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.dim() != 1
                           or b.numel() != n or not b.is_contiguous() or (grad and b.requires_grad)):
@@ -606,7 +607,7 @@ def linear(x: torch.Tensor, *layers: torch.nn.Linear):
         shape, dt, dev, grad = x.shape, x.dtype, x.get_device(), torch.is_grad_enabled()
         k, xp = shape[-1], x.data_ptr()
         m = x.numel() // k if k else 0
-        if m > 0 and k % 8 == 0 and xp % 16 == 0 and not (grad and x.requires_grad):
+        if 0 < m <= _INT32_MAX and k <= _INT32_MAX and k % 8 == 0 and xp % 16 == 0 and not (grad and x.requires_grad):
             p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
             out = []
             for i, layer in enumerate(layers):

@@ -100,3 +100,46 @@ def test_a_replaced_call_of_every_linear_layer_is_seen(owner, name, monkeypatch)
     was = getattr(owner, name)
     monkeypatch.setattr(owner, name, lambda *args, **kw: was(*args, **kw))
     assert not ops._nobody_watches()
+
+
+def test_a_weight_of_more_rows_than_the_kernel_counts_is_left_to_the_layer():
+    layer = torch.nn.Linear(16, 8, bias=False, device="meta", dtype=torch.float16).requires_grad_(False)
+    assert _taken(layer)
+    layer.weight = torch.nn.Parameter(torch.empty(2 ** 32 + 8, 16, device="meta", dtype=torch.float16), requires_grad=False)
+    assert not _taken(layer)
+
+
+# Sizes at the ends of the ranges, where sums of them do not fit 32 bits.
+TOP = 2 ** 31 - 1
+ENDS = [(TOP, 64, 64), (8, 64, TOP - 7), (64, TOP - 7, 8), (1, 8, 8)]
+WIDTHS = r"""
+#include <cuda_runtime.h>
+#include "linear.cuh"
+#include <cstdio>
+int main() {
+  const int shapes[][3] = {%s};
+  for (auto& s : shapes) {
+    bool pays = false;
+    std::printf("%%d %%d ", ma::linear_tile(s[0], s[1], 1, &s[2], 74, &pays), pays ? 1 : 0);
+  }
+  return 0;
+}
+""" % ", ".join("{%d, %d, %d}" % s for s in ENDS)
+
+
+def _width(m, k, n):
+    """The same rule in whole numbers of any size."""
+    clk = {w: -(-(-(-m // 256) * -(-n // w)) // 74) * (max(w // 2, 48) * -(-k // 16) + 1500) for w in range(256, 63, -16)}
+    return min(clk, key=clk.get)
+
+
+@pytest.mark.skipif(not Path("/usr/local/cuda/include/cuda.h").exists(), reason="no CUDA headers")
+def test_tile_width_at_the_ends_of_the_ranges(tmp_path):
+    src = tmp_path / "widths.cpp"
+    src.write_text(WIDTHS)
+    csrc = HEADER.parent.parent / "mini-attention_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "-I/usr/local/cuda/include", str(src), "-o", str(tmp_path / "widths")],
+                   check=True)
+    got = [int(t) for t in subprocess.run([str(tmp_path / "widths")], check=True, capture_output=True, text=True).stdout.split()]
+    assert got[::2] == [_width(*s) for s in ENDS]
+    assert got[5] == 0     # a tile of 2^31 columns of K would outlast the bounded waits

@@ -164,3 +164,11 @@ def test_a_bias_that_is_no_parameter_is_added(register):
         lin.bias = bias
     x = torch.randn(256, 64, device=DEV, dtype=torch.float16)
     assert torch.equal(ops.linear(x, lin)[0], lin(x))
+
+
+def test_more_rows_than_the_kernel_counts_go_through_the_layers(monkeypatch):
+    if torch.cuda.mem_get_info()[0] < 50 << 30:
+        pytest.skip("needs 34 GB of free memory")
+    monkeypatch.setattr(ops, "_operands", lambda *args: pytest.fail("taken"))
+    x = torch.empty(2 ** 31 + 8, 8, dtype=torch.float16, device=DEV)
+    assert ops.linear(x, lambda t: t.shape) == [x.shape]
