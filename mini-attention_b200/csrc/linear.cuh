@@ -37,16 +37,30 @@ struct LinearArgs {
   FastDiv by_m_tiles;
 };
 
+// Where the one launch pays.
+enum class LinearPays {
+  kNo,          // one library GEMM for each weight is expected to be quicker
+  kIssuedOnly,  // quicker to issue, not to run: not in a call that is captured, where the host's time is not paid again
+  kYes,
+};
+
 // Width of a tile: fewest clocks over the rounds of tiles, at bn / 2 clk for 16 columns of K and about 1500 a tile.
-// pays: whether that is expected to be no slower than a library GEMM for each weight, which reaches 0.92 of the tensor
-// rate at these sizes; either takes about 2 us a launch beside its work.  Measured, us of device time for the whole of
-// GQA_Flash in bf16, the layers' own calls / x's projections in one launch / the output's too: 2 x 1024 tokens, 16/4
-// heads of 128 52.6 / 49.9 / 50.4 (host-bound without a graph: 90.8 / 81.8 / 56.3); 1 x 4096, 32/8 heads 398 / 377 / 374;
-// 4 x 4096, 32/8 1766 / 1581 / 1570; 2 x 777, 24/8, where 1554 rows leave a seventh of the last row tiles 76.0 / 78.6 /
-// 83.2: not taken.  A launch of up to 13 us is taken in any case: the calls of the layers then take the host longer
-// than the GPU (1 x 512 tokens, 8/2 heads of 64: 66.5 us a call with them, 56.4 without, 16 on the device either way).
+//
+// pays: against a library GEMM for each weight, which reaches 0.92 of the tensor rate and, like this launch, takes about
+// 3700 clk beside its work.  q = this estimate / that.  Measured on 98 shapes of GQA_Flash and MHA (bf16, 128 to 16384
+// tokens, 64 to 4096 wide), chains of six modules replayed as a graph in bursts / for 0.1 s at the power cap, x's projections in
+// one launch over the layers' own calls, the whole module's time:
+//   q up to 1             0.84 to 1.02 / 0.82 to 1.02, mean 0.93: taken
+//   q up to 1.06          0.90 to 1.02 / 0.90 to 1.08, mean 0.98: taken, but with more than 32 MB of weights
+//                         1.01 to 1.03 / 1.06 to 1.11 (4096 wide: every pair fetches its operands itself through L2): not taken
+//   q above               0.94 to 1.17 / 0.94 to 1.32, mean 1.01: not taken
+// One weight alone saves no launch, and the library's tiles are the better ones: the output projection in this form
+// 0.97 to 1.12 of the module, mean 1.03.  It is quicker to issue, though, by 5 to 10 us of a call's 65 (a module of up to about 60 us on
+// the GPU is bound by that): 2 x 1024 tokens, 16/4 heads of 128 66 us with the layers' calls, 62 with x's projections in one
+// launch, 57 with the output's as well, 52 to 57 on the GPU.  So launches of up to 24000 clk (13 us), which are those of
+// such modules, are taken where they are issued anew each time.
 // Never with so many columns of K that a tile would come near the bounded waits' limit (about 8 clk a column, 1 s).
-inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* pays) {
+inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, LinearPays* pays) {
   const long long m_tiles = (M + 255ll) / 256;
   long long best = -1;
   int bn = kLinearMaxBn;
@@ -62,12 +76,12 @@ inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* p
       bn = w;
     }
   }
-  double macs = 0.;
-  for (int i = 0; i < n_seg; ++i) macs += static_cast<double>(M) * N[i] * K;
+  double weights = 0.;
+  for (int i = 0; i < n_seg; ++i) weights += static_cast<double>(N[i]) * K;
   const double launch = 3700.;
-  *pays = K <= 1 << 24 &&
-          (best + launch <= 1.08 * (macs / (2. * pairs * 4096. * 0.92) + n_seg * launch) ||
-           best + launch <= 24000.);
+  const double own = best + launch, library = M * weights / (2. * pairs * 4096. * 0.92) + n_seg * launch;
+  const bool quicker = n_seg > 1 && (own <= library || (own <= 1.06 * library && 2. * weights <= 32e6));
+  *pays = K > 1 << 24 ? LinearPays::kNo : quicker ? LinearPays::kYes : own <= 24000. ? LinearPays::kIssuedOnly : LinearPays::kNo;
   return bn;
 }
 

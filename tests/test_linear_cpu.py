@@ -109,22 +109,46 @@ def test_a_weight_of_more_rows_than_the_kernel_counts_is_left_to_the_layer():
     assert not _taken(layer)
 
 
-# Sizes at the ends of the ranges, where sums of them do not fit 32 bits.
+# Sizes at the ends of the ranges, where sums of them do not fit 32 bits, and where the one launch pays: 0 no, 1 where it
+# is issued anew each time, 2 yes.
 TOP = 2 ** 31 - 1
 ENDS = [(TOP, 64, 64), (8, 64, TOP - 7), (64, TOP - 7, 8), (1, 8, 8)]
-WIDTHS = r"""
+PAYS = [
+    ((64, TOP - 7, 8), 0),                     # a tile of 2^31 columns of K would outlast the bounded waits
+    ((2048, 2048, 2048, 1024), 2), ((512, 512, 512, 256), 2), ((2277, 1536, 1536, 1536, 1536), 2), ((700, 3072, 3072, 3072, 3072), 2),
+    ((4768, 2048, 2048, 1024), 2),             # q = 1.03, 12 MB of weights
+    ((4096, 4096, 4096, 2048), 0),             # q = 1.02, 50 MB
+    ((1554, 3072, 3072, 2048), 0), ((804, 4096, 4096, 4096), 0),   # q = 1.09, 1.20
+    ((361, 4096, 4096, 1024), 1),              # q = 1.13, 20000 clk
+    ((2048, 2048, 2048), 1), ((512, 512, 512), 1), ((16384, 64, 64), 1),     # one weight: no launch saved
+    ((4096, 4096, 4096), 0), ((8192, 2048, 2048), 0), ((16384, 4096, 4096), 0),
+]
+RULE = r"""
 #include <cuda_runtime.h>
 #include "linear.cuh"
 #include <cstdio>
 int main() {
-  const int shapes[][3] = {%s};
+  const int shapes[][5] = {%s};
   for (auto& s : shapes) {
-    bool pays = false;
-    std::printf("%%d %%d ", ma::linear_tile(s[0], s[1], 1, &s[2], 74, &pays), pays ? 1 : 0);
+    int n = 1;
+    while (n < 3 && s[2 + n] > 0) ++n;
+    ma::LinearPays pays;
+    const int w = ma::linear_tile(s[0], s[1], n, &s[2], 74, &pays);
+    std::printf("%%d %%d ", w, static_cast<int>(pays));
   }
   return 0;
 }
-""" % ", ".join("{%d, %d, %d}" % s for s in ENDS)
+"""
+
+
+def _rule(tmp_path, shapes):
+    src = tmp_path / "rule.cpp"
+    src.write_text(RULE % ", ".join("{%s}" % ", ".join(map(str, s)) for s in shapes))
+    csrc = HEADER.parent.parent / "mini-attention_b200" / "csrc"
+    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "-I/usr/local/cuda/include", str(src), "-o", str(tmp_path / "rule")],
+                   check=True)
+    got = subprocess.run([str(tmp_path / "rule")], check=True, capture_output=True, text=True).stdout.split()
+    return [int(t) for t in got[::2]], [int(t) for t in got[1::2]]
 
 
 def _width(m, k, n):
@@ -133,13 +157,14 @@ def _width(m, k, n):
     return min(clk, key=clk.get)
 
 
-@pytest.mark.skipif(not Path("/usr/local/cuda/include/cuda.h").exists(), reason="no CUDA headers")
+needs_headers = pytest.mark.skipif(not Path("/usr/local/cuda/include/cuda.h").exists(), reason="no CUDA headers")
+
+
+@needs_headers
 def test_tile_width_at_the_ends_of_the_ranges(tmp_path):
-    src = tmp_path / "widths.cpp"
-    src.write_text(WIDTHS)
-    csrc = HEADER.parent.parent / "mini-attention_b200" / "csrc"
-    subprocess.run(["g++", "-std=c++17", f"-I{csrc}", "-I/usr/local/cuda/include", str(src), "-o", str(tmp_path / "widths")],
-                   check=True)
-    got = [int(t) for t in subprocess.run([str(tmp_path / "widths")], check=True, capture_output=True, text=True).stdout.split()]
-    assert got[::2] == [_width(*s) for s in ENDS]
-    assert got[5] == 0     # a tile of 2^31 columns of K would outlast the bounded waits
+    assert _rule(tmp_path, ENDS)[0] == [_width(*s) for s in ENDS]
+
+
+@needs_headers
+def test_where_one_launch_pays(tmp_path):
+    assert _rule(tmp_path, [s for s, _ in PAYS])[1] == [want for _, want in PAYS]

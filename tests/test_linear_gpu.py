@@ -172,3 +172,30 @@ def test_more_rows_than_the_kernel_counts_go_through_the_layers(monkeypatch):
     monkeypatch.setattr(ops, "_operands", lambda *args: pytest.fail("taken"))
     x = torch.empty(2 ** 31 + 8, 8, dtype=torch.float16, device=DEV)
     assert ops.linear(x, lambda t: t.shape) == [x.shape]
+
+
+def test_a_captured_call_is_judged_by_the_gpus_time():
+    """One weight is quicker to issue in this form and not to run: taken in an ordinary call, left to the layer in a
+    captured one; two weights that save a launch are taken in both."""
+    def launch(n_out):
+        x, ws = torch.ones(512, 512, dtype=torch.float16, device=DEV), [torch.ones(512, 512, dtype=torch.float16, device=DEV)] * n_out
+        ys = [torch.zeros(512, 512, dtype=torch.float16, device=DEV) for _ in ws]
+        return (x, ws, [None] * n_out, ys), ys
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for n_out in (1, 2):
+            args, ys = launch(n_out)
+            assert _launch(*args, only_if_faster=1) == _lib.OK
+            stream.synchronize()
+            for y in ys:
+                assert bool((y == 512).all())
+                y.zero_()
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                rc = _launch(*args, only_if_faster=1)
+                ys[0] += 1.0
+            assert rc == (1 if n_out == 1 else _lib.OK)
+            graph.replay()
+            stream.synchronize()
+            assert bool((ys[0] == (1 if n_out == 1 else 513)).all())
