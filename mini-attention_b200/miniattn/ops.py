@@ -595,40 +595,60 @@ def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: b
     return w, b
 
 
-def linear(x: torch.Tensor, *layers: torch.nn.Linear):
-    """``[layer(x) for layer in layers]`` for up to three linear layers that share their input.
+# Sizes (of x, rows of each weight) for which one GEMM per layer is the quicker form, called anew or replayed.  A size that is found
+# here is left to the layers before anything is looked at or allocated: finding that out again with each call took the host 12 us a
+# layer, 66 -> 113 us for a module none of whose projections is taken.
+_left_to_layers: set = set()
+_LEFT_MAX = 4096
 
-    One launch of ``miniattn_linear`` where that is the quicker form, every layer is a plain ``nn.Linear`` (no hooks, no replaced forward) of
-    16-bit operands on the GPU and nothing watches the call (gradients, tangents, autocast, tracing, modes); the
-    layers' own calls otherwise."""
-    p = None
-    if (type(x) is torch.Tensor and x.is_cuda and x.dtype in _DTYPES and x.is_contiguous() and x.dim() >= 2
-            and len(layers) <= 3 and _nobody_watches()):
-        shape, dt, dev, grad = x.shape, x.dtype, x.get_device(), torch.is_grad_enabled()
-        k, xp = shape[-1], x.data_ptr()
-        m = x.numel() // k if k else 0
-        if 0 < m <= _INT32_MAX and k <= _INT32_MAX and k % 8 == 0 and xp % 16 == 0 and not (grad and x.requires_grad):
-            p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
-            out = []
-            for i, layer in enumerate(layers):
-                wb = _operands(layer, k, dt, dev, grad)
-                if wb is None:
-                    p = None
-                    break
-                w, b = wb
-                n = w.shape[0]
-                y = x.new_empty((*shape[:-1], n))
-                p.out[i] = (w.data_ptr(), None if b is None else b.data_ptr(), y.data_ptr(), k, n, n)
-                out.append(y)
-    if p is None:
-        return [layer(x) for layer in layers]
+
+def _one_launch(x: torch.Tensor, layers, size):
+    """The layers' outputs out of one launch of ``miniattn_linear``; None where it takes no such layers or does not pay."""
+    shape, dt, dev, grad = x.shape, x.dtype, x.get_device(), torch.is_grad_enabled()
+    k, xp = shape[-1], x.data_ptr()
+    m = x.numel() // k if k else 0
+    if not 0 < m <= _INT32_MAX or k > _INT32_MAX or k % 8 or xp % 16 or (grad and x.requires_grad):
+        return None
+    operands = []
+    for layer in layers:
+        wb = _operands(layer, k, dt, dev, grad)
+        if wb is None:
+            return None
+        operands.append(wb)
+    p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
+    out = []
+    for i, (w, b) in enumerate(operands):
+        n = w.shape[0]
+        y = x.new_empty((*shape[:-1], n))
+        p.out[i] = (w.data_ptr(), None if b is None else b.data_ptr(), y.data_ptr(), k, n, n)
+        out.append(y)
     if _current_device() == dev:
         rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
     else:
         with torch.cuda.device(dev):
             rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
-    if rc == 1:  # one GEMM per layer is quicker
-        return [layer(x) for layer in layers]
+    if rc == 1:  # one GEMM per layer is quicker; a captured call is judged by another rule
+        if not torch.cuda.is_current_stream_capturing():
+            if len(_left_to_layers) >= _LEFT_MAX:
+                _left_to_layers.clear()
+            _left_to_layers.add(size)
+        return None
     if rc != _lib.OK:
         _lib.check(rc, "miniattn_linear")
     return out
+
+
+def linear(x: torch.Tensor, *layers: torch.nn.Linear):
+    """``[layer(x) for layer in layers]`` for up to three linear layers that share their input.
+
+    One launch of ``miniattn_linear`` where that is the quicker form, every layer is a plain ``nn.Linear`` (no hooks, no replaced
+    forward) of 16-bit operands on the GPU and nothing watches the call (gradients, tangents, autocast, tracing, modes); the
+    layers' own calls otherwise."""
+    if (type(x) is torch.Tensor and x.is_cuda and x.dtype in _DTYPES and x.is_contiguous() and x.dim() >= 2
+            and len(layers) <= 3):
+        size = (x.shape, *[getattr(layer, "out_features", None) for layer in layers])
+        if size not in _left_to_layers and _nobody_watches():
+            out = _one_launch(x, layers, size)
+            if out is not None:
+                return out
+    return [layer(x) for layer in layers]

@@ -169,7 +169,7 @@ def test_a_bias_that_is_no_parameter_is_added(register):
 def test_more_rows_than_the_kernel_counts_go_through_the_layers(monkeypatch):
     if torch.cuda.mem_get_info()[0] < 50 << 30:
         pytest.skip("needs 34 GB of free memory")
-    monkeypatch.setattr(ops, "_operands", lambda *args: pytest.fail("taken"))
+    monkeypatch.setattr(ops, "_operands", lambda *args: pytest.fail("taken"))   # nothing is looked at
     x = torch.empty(2 ** 31 + 8, 8, dtype=torch.float16, device=DEV)
     assert ops.linear(x, lambda t: t.shape) == [x.shape]
 
@@ -199,3 +199,28 @@ def test_a_captured_call_is_judged_by_the_gpus_time():
             graph.replay()
             stream.synchronize()
             assert bool((ys[0] == (1 if n_out == 1 else 513)).all())
+
+
+def test_sizes_that_are_left_to_the_layers_are_known_the_second_time(monkeypatch):
+    """What is looked at for a size that does not pay: the layer once, nothing after that.  A captured call's answer is
+    not kept for calls that are issued."""
+    seen, was = [], ops._operands
+    monkeypatch.setattr(ops, "_operands", lambda *args: seen.append(1) or was(*args))
+    monkeypatch.setattr(ops, "_left_to_layers", set())
+    lin = torch.nn.Linear(3072, 3072).half().to(DEV).requires_grad_(False)
+    x = torch.randn(1554, 3072, device=DEV, dtype=torch.float16)
+    for _ in range(3):
+        assert torch.equal(ops.linear(x, lin)[0], lin(x))
+    assert len(seen) == 1 and len(ops._left_to_layers) == 1
+    small, sx = torch.nn.Linear(512, 512).half().to(DEV).requires_grad_(False), x[:, :512].contiguous()
+    small(sx)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.linear(sx, small)
+    assert len(ops._left_to_layers) == 1
+    launches, fn = [], _lib.lib.miniattn_linear
+    monkeypatch.setattr(ops._lib, "lib", type("Lib", (), {"miniattn_linear": staticmethod(
+        lambda *args: launches.append(fn(*args)) or launches[-1])}))
+    ops.linear(sx, small)
+    assert launches == [_lib.OK]
