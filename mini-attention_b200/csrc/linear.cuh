@@ -55,10 +55,10 @@ enum class LinearPays {
 //                         1.01 to 1.03 / 1.06 to 1.11 (4096 wide: every pair fetches its operands itself through L2): not taken
 //   q above               0.94 to 1.17 / 0.94 to 1.32, mean 1.01: not taken
 // One weight alone saves no launch, and the library's tiles are the better ones: the output projection in this form
-// 0.97 to 1.12 of the module, mean 1.03.  It is quicker to issue, though, by 5 to 10 us of a call's 65 (a module of up to about 60 us on
-// the GPU is bound by that): 2 x 1024 tokens, 16/4 heads of 128 66 us with the layers' calls, 62 with x's projections in one
-// launch, 57 with the output's as well, 52 to 57 on the GPU.  So launches of up to 24000 clk (13 us), which are those of
-// such modules, are taken where they are issued anew each time.
+// 0.97 to 1.12 of the module, mean 1.03.  It is quicker to issue, though, and a module of up to about 60 us on the GPU is bound by
+// that: 2 x 1024 tokens, 16/4 heads of 128 65 us with the layers' calls, 61 with x's projections in one launch, 54 with the
+// output's as well, 52 to 57 on the GPU.  So launches of up to 24000 clk (13 us), which are those of such modules, are taken
+// where they are issued anew each time.  (Only after x's: one of this form between library calls takes the host 3 us more.)
 // Never with so many columns of K that a tile would come near the bounded waits' limit (about 8 clk a column, 1 s).
 inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, LinearPays* pays) {
   const long long m_tiles = (M + 255ll) / 256;

@@ -118,7 +118,7 @@ def _load() -> C.CDLL:
     for name in ("miniattn_quant_qk_int8", "miniattn_quant_qk_int8_static", "miniattn_fwd_int8qk"):
         getattr(lib, name).argtypes = [C.POINTER(Int8Params), C.c_void_p]
         getattr(lib, name).restype = C.c_int
-    lib.miniattn_linear.argtypes = [C.POINTER(LinearParams), C.c_void_p]
+    lib.miniattn_linear.argtypes = [C.c_void_p, C.c_void_p]   # a LinearParams by reference, or its bytes
     lib.miniattn_linear.restype = C.c_int
     lib.miniattn_merge_partials.argtypes = [C.POINTER(MergeParams), C.c_void_p]
     lib.miniattn_merge_partials.restype = C.c_int

@@ -10,6 +10,7 @@ device memory and streams only; the arithmetic runs in libminiattn.so.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Optional, Tuple, Union
 
 import torch
@@ -575,24 +576,30 @@ def _nobody_watches() -> bool:
 
 
 def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: bool):
-    """(weight, bias or None) of a layer whose own call is x weight^T + bias and nothing else, over `k` inputs of dtype
-    `dt` on device `dev`, in the form ``miniattn_linear`` takes; None for any other layer."""
+    """(address of the weight, address of the bias or 0, rows of the weight) of a layer whose own call is x weight^T + bias and
+    nothing else, over `k` inputs of dtype `dt` on device `dev`, in the form ``miniattn_linear`` takes; None for any other."""
     if type(layer) is not _Linear:   # a scripted or traced layer keeps its parameters elsewhere
         return None
     own = layer.__dict__
-    w, b = own["_parameters"].get("weight"), own["_parameters"].get("bias", False)  # False: not a parameter, or not there
+    parameters = own["_parameters"]
+    w, b = parameters.get("weight"), parameters.get("bias", False)  # False: not a parameter, or not there
     if (type(w) is not _Parameter or w.dtype is not dt or w.get_device() != dev
             or "forward" in own or "weight" in own or "bias" in own or own["_forward_hooks"] or own["_forward_pre_hooks"]
-            or own["_backward_hooks"] or own["_backward_pre_hooks"] or w.dim() != 2
+            or own["_backward_hooks"] or own["_backward_pre_hooks"]
             or not w.is_contiguous() or (grad and w.requires_grad)):
         return None
-    n, wk = w.shape
-    if wk != k or n % 8 or not 0 < n <= _INT32_MAX or w.data_ptr() % 16:
+    shape = w.shape
+    if len(shape) != 2 or shape[1] != k:
         return None
-    if b is not None and (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.dim() != 1
-                          or b.numel() != n or not b.is_contiguous() or (grad and b.requires_grad)):
+    n, wp = shape[0], w.data_ptr()
+    if n % 8 or not 0 < n <= _INT32_MAX or wp % 16:
         return None
-    return w, b
+    if b is None:
+        return wp, 0, n
+    if (type(b) is not _Parameter or b.dtype is not dt or b.get_device() != dev or b.shape != (n,) or not b.is_contiguous()
+            or (grad and b.requires_grad)):
+        return None
+    return wp, b.data_ptr(), n
 
 
 # Sizes (of x, rows of each weight) for which one GEMM per layer is the quicker form, called anew or replayed.  A size that is found
@@ -602,10 +609,16 @@ _left_to_layers: set = set()
 _LEFT_MAX = 4096
 
 
+# MiniAttnLinearParams in one go: its fields set one by one through ctypes take the host 5 us.
+_pack_linear = struct.Struct("@PPqiiiiii" + 3 * "PPPqqii").pack
+_no_output = (0, 0, 0, 0, 0, 0, 0)
+
+
 def _one_launch(x: torch.Tensor, layers, size):
     """The layers' outputs out of one launch of ``miniattn_linear``; None where it takes no such layers or does not pay."""
-    shape, dt, dev, grad = x.shape, x.dtype, x.get_device(), torch.is_grad_enabled()
-    k, xp = shape[-1], x.data_ptr()
+    dt, dev, grad = x.dtype, x.get_device(), torch.is_grad_enabled()
+    *rows, k = x.shape
+    xp = x.data_ptr()
     m = x.numel() // k if k else 0
     if not 0 < m <= _INT32_MAX or k > _INT32_MAX or k % 8 or xp % 16 or (grad and x.requires_grad):
         return None
@@ -615,18 +628,21 @@ def _one_launch(x: torch.Tensor, layers, size):
         if wb is None:
             return None
         operands.append(wb)
-    p = _lib.LinearParams(xp, _status_word(x.device).data_ptr(), k, m, k, _DTYPES[dt], len(layers), 1)
-    out = []
-    for i, (w, b) in enumerate(operands):
-        n = w.shape[0]
-        y = x.new_empty((*shape[:-1], n))
-        p.out[i] = (w.data_ptr(), None if b is None else b.data_ptr(), y.data_ptr(), k, n, n)
+    out, fields = [], []
+    for w, b, n in operands:
+        y = x.new_empty((*rows, n))
+        fields += (w, b, y.data_ptr(), k, n, n, 0)
         out.append(y)
+    for _ in range(len(layers), 3):
+        fields += _no_output
+    status = _status_words.get(("cuda", dev))
+    block = _pack_linear(xp, (_status_word(x.device) if status is None else status).data_ptr(), k, m, k, _DTYPES[dt],
+                         len(layers), 1, 0, *fields)
     if _current_device() == dev:
-        rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
+        rc = _lib.lib.miniattn_linear(block, _current_raw_stream(dev))
     else:
         with torch.cuda.device(dev):
-            rc = _lib.lib.miniattn_linear(_byref(p), _current_raw_stream(dev))
+            rc = _lib.lib.miniattn_linear(block, _current_raw_stream(dev))
     if rc == 1:  # one GEMM per layer is quicker; a captured call is judged by another rule
         if not torch.cuda.is_current_stream_capturing():
             if len(_left_to_layers) >= _LEFT_MAX:
@@ -641,14 +657,14 @@ def _one_launch(x: torch.Tensor, layers, size):
 def linear(x: torch.Tensor, *layers: torch.nn.Linear):
     """``[layer(x) for layer in layers]`` for up to three linear layers that share their input.
 
-    One launch of ``miniattn_linear`` where that is the quicker form, every layer is a plain ``nn.Linear`` (no hooks, no replaced
-    forward) of 16-bit operands on the GPU and nothing watches the call (gradients, tangents, autocast, tracing, modes); the
-    layers' own calls otherwise."""
+    One launch of ``miniattn_linear`` (the result is a tuple then) where that is the quicker form, every layer is a plain
+    ``nn.Linear`` (no hooks, no replaced forward) of 16-bit operands on the GPU and nothing watches the call (gradients, tangents,
+    autocast, tracing, modes); the layers' own calls (a list) otherwise."""
     if (type(x) is torch.Tensor and x.is_cuda and x.dtype in _DTYPES and x.is_contiguous() and x.dim() >= 2
-            and len(layers) <= 3):
+            and 1 <= len(layers) <= 3):
         size = (x.shape, *[getattr(layer, "out_features", None) for layer in layers])
         if size not in _left_to_layers and _nobody_watches():
             out = _one_launch(x, layers, size)
             if out is not None:
-                return out
+                return tuple(out)
     return [layer(x) for layer in layers]

@@ -34,6 +34,12 @@ def _attend(q, k, v, causal, return_lse=False):
     return (o, res[1]) if return_lse else o
 
 
+def _project(o, layer, projected):
+    """The output projection: in one launch of the same kernel where the projections before it (`projected`) were, a call of
+    the layer where they were the layers' calls (one of each takes the host longer than two of either)."""
+    return linear(o, layer)[0] if type(projected) is tuple else layer(o)
+
+
 class MHA(nn.Module):
     def __init__(self, d_model: int, n_heads: int, dropout: float = 0.0, need_weights: bool = True):
         super().__init__()
@@ -64,16 +70,17 @@ class MHA(nn.Module):
                     raise RuntimeError("only no mask, an all-ones mask or a lower-triangular (causal) mask is "
                                        "supported: there is no eager path behind the fused kernel")
                 causal = True
-        q, k, v = (y.view(B, S, self.n_heads, self.d_h) for y in linear(x, self.w_q, self.w_k, self.w_v))
+        projected = linear(x, self.w_q, self.w_k, self.w_v)
+        q, k, v = (y.view(B, S, self.n_heads, self.d_h) for y in projected)
         if not self.need_weights:
-            return linear(_attend(q, k, v, causal), self.w_o)[0], None
+            return _project(_attend(q, k, v, causal), self.w_o, projected), None
         o, lse = _attend(q, k, v, causal, return_lse=True)
         # weights = softmax(q k^T / sqrt(d_h) [+ mask]) rebuilt from the kernel's log-sum-exp
         scores = torch.matmul(q.transpose(1, 2).float(), k.permute(0, 2, 3, 1).float()) / math.sqrt(self.d_h)
         weights = torch.exp(scores - lse.unsqueeze(-1))
         if causal:
             weights = weights.masked_fill(~torch.tril(torch.ones(S, S, device=x.device, dtype=torch.bool)), 0.0)
-        return linear(o, self.w_o)[0], weights.to(x.dtype)
+        return _project(o, self.w_o, projected), weights.to(x.dtype)
 
 
 class GQA_Flash(nn.Module):
@@ -89,10 +96,10 @@ class GQA_Flash(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         B, S, _ = x.shape
-        q, kv = linear(x, self.w_q, self.kv)
+        q, kv = projected = linear(x, self.w_q, self.kv)
         q = q.view(B, S, self.n_heads, self.head_dim)
         kv = kv.view(B, S, 2, self.n_kv_heads, self.head_dim)
-        return linear(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o)[0]
+        return _project(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o, projected)
 
 
 class MQA_Flash(nn.Module):
@@ -106,7 +113,7 @@ class MQA_Flash(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         B, S, _ = x.shape
-        q, kv = linear(x, self.w_q, self.k_v)
+        q, kv = projected = linear(x, self.w_q, self.k_v)
         q = q.view(B, S, self.n_heads, self.head_dim)
         kv = kv.view(B, S, 2, 1, self.head_dim)
-        return linear(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o)[0]
+        return _project(_attend(q, kv[:, :, 0], kv[:, :, 1], True), self.w_o, projected)

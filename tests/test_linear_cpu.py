@@ -76,8 +76,16 @@ def _bias_as(kind):
 def test_plain_layers_are_taken():
     layer = _layer()
     assert _taken(layer) and _taken(_layer(bias=False))
-    w, b = ops._operands(layer, 16, torch.float16, -1, True)
-    assert w is layer.weight and b is layer.bias
+    assert ops._operands(layer, 16, torch.float16, -1, True) == (layer.weight.data_ptr(), layer.bias.data_ptr(), 8)
+    assert ops._operands(_layer(bias=False), 16, torch.float16, -1, True)[1:] == (0, 8)
+
+
+def test_packed_block_has_the_layout_of_the_mirror():
+    one, two = (1, 2, 3, 4, 5, 6, 0), (11, 0, 13, 14, 15, 16, 0)
+    p = _lib.LinearParams.from_buffer_copy(ops._pack_linear(21, 22, 23, 24, 25, 1, 2, 1, 0, *one, *two, *ops._no_output))
+    assert (p.x, p.status, p.ldx, p.M, p.K, p.dtype, p.n_out, p.only_if_faster) == (21, 22, 23, 24, 25, 1, 2, 1)
+    assert [(o.w, o.bias, o.y, o.ldw, o.ldy, o.N) for o in p.out] == [(1, 2, 3, 4, 5, 6), (11, None, 13, 14, 15, 16),
+                                                                       (None, None, None, 0, 0, 0)]
 
 
 @pytest.mark.parametrize("kind", ["buffer", "attribute", "missing", "shadowed"])

@@ -224,3 +224,20 @@ def test_sizes_that_are_left_to_the_layers_are_known_the_second_time(monkeypatch
         lambda *args: launches.append(fn(*args)) or launches[-1])}))
     ops.linear(sx, small)
     assert launches == [_lib.OK]
+
+
+@pytest.mark.parametrize("S,heads,names", [(300, (12, 4), ["w_q+kv", "w_o"]), (1554, (24, 8), []), (4768, (16, 4), ["w_q+kv"])])
+def test_which_projections_of_a_module_are_launches(S, heads, names, monkeypatch):
+    """Short ones all, ones that the library does quicker none (the output's alone neither), long ones x's."""
+    m = _module(miniattn.variants.GQA_Flash, heads[0] * 128, *heads).requires_grad_(False)
+    which = {(layer,): name for name, layer in m.named_children()} | {(m.w_q, m.kv): "w_q+kv"}
+    was, seen = ops._one_launch, []
+    def spy(x, layers, size):
+        out = was(x, layers, size)
+        if out is not None:
+            seen.append(which[tuple(layers)])
+        return out
+    monkeypatch.setattr(ops, "_left_to_layers", set())
+    monkeypatch.setattr(ops, "_one_launch", spy)
+    m(torch.randn(1, S, heads[0] * 128, device=DEV, dtype=torch.bfloat16))
+    assert seen == names
