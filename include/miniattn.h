@@ -269,7 +269,7 @@ int miniattn_merge_partials(const MiniAttnMergeParams* p, void* stream);
  * Linear layers that share their input, in one launch: y_i = x w_i^T + b_i, the projections around the
  * attention call of the reference's modules (kernels/standard/pytorch/gqa.py:24-28, :50).  16-bit operands, fp32
  * accumulation and bias, one rounding.  x is [M, K], w_i [N_i, K] and y_i [M, N_i], each with its last dimension
- * contiguous and its rows ldx / ldw / ldy elements apart; K, N_i and the row strides are multiples of 8, the
+ * contiguous and its rows ldx / ldw / ldy elements apart; K, N_i (at most 2^31 - 257) and the row strides are multiples of 8, the
  * pointers (bias excepted) 16-byte aligned.  At most 3 weights.
  */
 typedef struct MiniAttnLinearOut {

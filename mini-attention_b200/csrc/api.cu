@@ -931,6 +931,7 @@ int miniattn_linear(const MiniAttnLinearParams* p, void* stream) {
   for (int i = 0; i < p->n_out; ++i) {
     const MiniAttnLinearOut& o = p->out[i];
     if (o.N <= 0 || o.N % 8 != 0) return fail(MINIATTN_EINVAL, "N (%d) must be a positive multiple of 8", o.N);
+    if (o.N > ma::kLinearMaxN) return fail(MINIATTN_EUNSUPPORTED, "N (%d) must be at most %d", o.N, ma::kLinearMaxN);
     if ((rc = check_rows(o.w, o.ldw, p->K, "w")) != 0 || (rc = check_rows(o.y, o.ldy, o.N, "y")) != 0) return rc;
     if (o.bias != nullptr && reinterpret_cast<uintptr_t>(o.bias) % 2 != 0)
       return fail(MINIATTN_EINVAL, "bias must be 2-byte aligned");

@@ -102,12 +102,12 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
       const int buf = done & 1;
       const CUtensorMap* tm = &a.seg[seg].tm_y;
       const uint16_t* bias = a.seg[seg].bias;
-      const uint32_t n = a.seg[seg].N;
+      const int n = a.seg[seg].N;
       mbar_wait(bar(kBarAccFull + buf), (done >> 1) & 1, wc, kErrWaitS);
       tc_fence_after();
       const uint32_t tA = tmem_base + buf * 256 + (static_cast<uint32_t>(quad * 32) << 16);
       for (int bx = half; bx < n_box; bx += 2) {
-        const uint32_t col = static_cast<uint32_t>(n0) + bx * kStoreCols;  // may pass 2^31 in the last tile
+        const int col = n0 + bx * kStoreCols;
         if (col >= n) break;
         uint32_t u[16];
         tmem_ld16(tA + bx * kStoreCols, u);
@@ -144,7 +144,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
         __syncwarp();
         if (lane == 0) {
           const int row = m0 + rank * kRows + quad * 32;
-          if (row < a.M) tma_store_2d(tm, box, static_cast<int>(col), row);
+          if (row < a.M) tma_store_2d(tm, box, col, row);
           tma_store_commit();
         }
       }
@@ -197,7 +197,7 @@ linear_kernel(const __grid_constant__ LinearArgs a) {
           const uint32_t dst = sbase + stage * kStageBytes;
           if (rank == 0) mbar_expect_tx(bar(kBarFull + stage), 2 * (kABytes + b_rows * kK * 2));
           tma_load_2d_pair(dst, &a.tm_x, full + 8 * stage, k * kK, m0 + rank * kRows);
-          tma_load_2d_pair(dst + kABytes, &a.seg[seg].tm_w, full + 8 * stage, k * kK, static_cast<int>(static_cast<uint32_t>(n0) + rank * b_rows));
+          tma_load_2d_pair(dst + kABytes, &a.seg[seg].tm_w, full + 8 * stage, k * kK, n0 + rank * b_rows);
         }
         __syncwarp();
         if (++stage == kStages) {

@@ -6,6 +6,7 @@ namespace ma {
 
 constexpr int kLinearMax = 3;      // weights of one launch
 constexpr int kLinearMaxBn = 256;  // columns of a tile (two accumulators fill TMEM)
+constexpr int kLinearMaxN = 0x7fffffff - kLinearMaxBn;  // a tile's last column fits 32 bits
 constexpr int kStoreBufs = 4;      // boxes of an epilogue warp in flight
 
 // The buffer an epilogue warp stages its next box in.  Strictly in turn over all tiles of the warp: before it writes

@@ -592,7 +592,7 @@ def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: b
     if len(shape) != 2 or shape[1] != k:
         return None
     n, wp = shape[0], w.data_ptr()
-    if n % 8 or not 0 < n <= _INT32_MAX or wp % 16:
+    if n % 8 or not 0 < n < _INT32_MAX - 256 or wp % 16:
         return None
     if b is None:
         return wp, 0, n

@@ -41,6 +41,8 @@ def test_bad_calls_are_refused():
                dict(y=0x1004), dict(ldx=60), dict(ldx=56), dict(ldw=32), dict(ldy=63), dict(bias=0x1001)):
         assert _call(**kw) == _lib.EINVAL, kw
     assert _call(dtype=2) == _lib.EUNSUPPORTED
+    top = 2 ** 31 - 8
+    assert _call(N=top, ldy=top) == _lib.EUNSUPPORTED  # a tile's last columns would pass 2^31
     assert _call(M=0) == _lib.OK                      # nothing to do, no device asked for
 
 
@@ -113,8 +115,9 @@ def test_a_replaced_call_of_every_linear_layer_is_seen(owner, name, monkeypatch)
 def test_a_weight_of_more_rows_than_the_kernel_counts_is_left_to_the_layer():
     layer = torch.nn.Linear(16, 8, bias=False, device="meta", dtype=torch.float16).requires_grad_(False)
     assert _taken(layer)
-    layer.weight = torch.nn.Parameter(torch.empty(2 ** 32 + 8, 16, device="meta", dtype=torch.float16), requires_grad=False)
-    assert not _taken(layer)
+    for rows in (2 ** 31 - 8, 2 ** 32 + 8):
+        layer.weight = torch.nn.Parameter(torch.empty(rows, 16, device="meta", dtype=torch.float16), requires_grad=False)
+        assert not _taken(layer)
 
 
 # Sizes at the ends of the ranges, where sums of them do not fit 32 bits, and where the one launch pays: 0 no, 1 where it
