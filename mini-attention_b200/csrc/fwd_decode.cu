@@ -10,7 +10,7 @@
 //   CTA       = a contiguous range of the tiles of all items, the same length for every CTA of the
 //               launch; plan_decode (plan.cu) says how many and which calls come here at all
 //   warp 4    TMA producer: K and V boxes (64 keys, 128-byte swizzle) through a ring, 96 KB deep (64 KB at D = 64),
-//             192 KB in flight per SM
+//             192 KB (128 KB) in flight per SM
 //   warps 0-3 16 rows x (16*RG keys of the tile) each: RG row groups x 4/RG key groups, each warp
 //             with its own running (m, l, O) in registers -- no CTA-wide step inside the loop
 //
@@ -24,8 +24,8 @@
 // Measured (B200, 16 requests, 32/8 heads, 1 token against 4001 keys, D=128 bf16, 262 MB of K/V): 183 us
 // through fwd_ws.cu before that packed heads, 48 now, 45.6 us here = 5.7 TB/s, 0.88 of the measured copy bandwidth.  Short
 // calls are bound by their ends: with 64-bit divisions for a CTA's range and for every tile, and the first copies
-// after the CTA's first synchronisation, 8 KV heads of 500 keys took 7.2 us (5.25 now), 64 items of 9000 16.6 (13.4),
-// 4 x 32/8 heads of 1024 11.3 (10.2).
+// after the CTA's first synchronisation, 32/8 heads of 500 keys took 8.1 us (6.1 now; D = 64 6.6 and 4.7), 4 x 32/8 heads of
+// 1024 9.4 (8.5), 64 items of 9000 at D = 64 27.6 (27.2), all with K and V in L2; calls of 40 us and more are as they were.
 #include <atomic>
 #include <type_traits>
 

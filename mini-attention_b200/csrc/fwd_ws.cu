@@ -213,8 +213,8 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     n_tiles = pe_t1 - pe_t0;
   }
 
-  // TMA loads (issued by lane 0 of warp kWarpTma only): Q tile t; ring fill i = K (even) or V (odd) of
-  // K/V tile kv_t0 + i/2 into slot i % kStages.
+  // TMA loads (one thread of warp kWarpTma: lane 0 for the first fill, an elected one from then on): Q tile t; ring fill
+  // i = K (even) or V (odd) of K/V tile kv_t0 + i/2 into slot i % kStages.
   auto load_q = [&](int t) {
     if constexpr (QK8) {  // one box of D bytes x 128 rows
       mbar_expect_tx(bar(L::kBarQFull + t), kTileM * D);
@@ -703,7 +703,8 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tmem_wait_ld();
         // A warp's 32 rows of a box go as soon as they are there: the copies overlap the rest of the conversion, and no
         // warp waits for the others of its tile (the CTA cannot leave before they have read the buffer, 1100 clk when
-        // the whole tile went at the end; N = 512 8.02 -> 7.76 us, D = 64 N = 1024 17.3 -> 17.1, INT8-QK 613 -> 593).
+        // the whole tile went at the end; N = 512 8.02 -> 7.76 us of the GPU's time, D = 64
+        // N = 1024 17.3 -> 17.1, INT8-QK 613 -> 593).
         // Packed heads that do not divide 32 make no box of 32 rows: their tile goes as one.
         const bool by_warp = !PACK || kWarpRows % a.pack == 0;
         auto store_box = [&](int bx) {
@@ -770,13 +771,14 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     reg_dec<kRegOther>();
     if (warp == kWarpMma0 || warp == kWarpMma1) {
       // =========================== MMA issuers =====================================
-      // One issuing thread per Q tile (warp 8 -> tile 0, warp 10 -> tile 1).  Each walks its
+      // One issuing warp per Q tile (warp 8 -> tile 0, warp 10 -> tile 1).  Each walks its
       // tile's halves in the order the softmax group publishes them: PV_a(j) S_a(j+1) PV_b(j)
       // S_b(j+1).  The tensor pipe interleaves the two streams.
       // The whole warp walks the halves and one elected thread issues, its descriptors a warp-uniform base plus
       // constants: an MMA then costs the issuing thread less than the 32 to 64 clk it takes the pipe.  Put together by a
       // single thread of a diverged warp they cost 45 to 112 clk each, 24 of them a step: 16 heads, N = 16384
-      // 1834 -> 1646 us, N = 2048 32.3 -> 30.5, N = 512 9.55 -> 8.02; D = 64, N = 8192 657 -> 609; INT8-QK 680 -> 656.
+      // 1834 -> 1646 us, N = 2048 32.3 -> 30.5, N = 512 9.55 -> 8.02 (the GPU's time; called from Python, where the host is the
+      // bound, 9.4 -> 9.0 with the per-warp stores); D = 64, N = 8192 657 -> 609; INT8-QK 680 -> 656.
       const int t = (warp == kWarpMma0) ? 0 : 1;
       if (n_tiles > 0 && t < nt) {
         const bool issuer = elect_one();
@@ -886,7 +888,8 @@ fwd_ws_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const int use = i / L::kStages;
           // A warp that mbarrier.try_wait holds takes issue slots from the softmax warps beside it, a sleeping one takes
           // none; the ring has slack for some of the half step until the next slot comes free (100 to 400 ns alike, 800
-          // starves it).  N = 8192 D = 64 625 -> 613 us, INT8-QK 618 -> 612, 4 x 32/8 heads N = 4096 causal 460 -> 456.
+          // starves it).  N = 8192 D = 64 625 -> 613 us, INT8-QK 618 -> 612, 4 x 32/8 heads N = 4096 causal 460 -> 456.  The shortest
+          // steps there are, those of a lone Q tile at D = 64 (0.9 us for 128 keys, 0.45 for a slot), are not starved either.
           __nanosleep(200);
           mbar_wait(bar(L::kBarKvEmpty + slot), (use - 1) & 1, wc, kErrWaitFree);
           if (issuer) load_kv(i);

@@ -68,9 +68,10 @@ float list_schedule(const std::vector<float>& cost, int sms, std::vector<float>*
 int min_piece(float plain_steps) { return plain_steps >= 24.f ? 4 : 6; }
 constexpr int kMaxParts = 64;      // pieces per item
 
-// Cost model, in steps (one K/V tile of a two-Q-tile CTA, about 2 us at D = 128): fixed cost of
+// Cost model, in steps (one K/V tile of a two-Q-tile CTA, about 1.6 us at D = 128): fixed cost of
 // a CTA, and what a piece of a cut item adds on average (publishing its partial takes about 0.6
-// steps; the last piece to arrive also reads the others', about 2 steps).
+// steps; the last piece to arrive also reads the others', about 2 steps).  The constants are from when a step took 2 us
+// and have not been measured anew since.
 float cta_cost(int D) { return D == 128 ? 2.0f : 3.0f; }
 float grade_frac() { return 0.015f; }  // spread of the per-SM targets, as a fraction of T
 float piece_cost() { return 1.3f; }

@@ -12,7 +12,7 @@ DEV = "cuda:0"
 
 
 @pytest.mark.parametrize("B,Hkv,G,Nk,balance", [
-    (2500, 8, 1, 512, False),    # 20000 items of 8 tiles, one CTA each: 3.6e9 tiles x CTAs
+    (2500, 8, 1, 512, False),    # 20000 items of 8 tiles, one CTA each: 3.2e9 tiles x CTAs
     (2000, 8, 1, 512, False),    # 16000: 2.05e9, just inside
     (37, 3, 2, 777, True),       # items that do not divide over the CTAs
     (1, 1, 4, 20000, True),      # one item in many pieces
