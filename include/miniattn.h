@@ -288,8 +288,7 @@ typedef struct MiniAttnLinearParams {
   int32_t     M, K;
   int32_t     dtype;      /* MINIATTN_FP16 | MINIATTN_BF16 */
   int32_t     n_out;
-  int32_t     only_if_faster;  /* 1: launch nothing and return 1 where one GEMM per weight is expected to be quicker (by the GPU's
-                                * time alone in a stream that is being captured) */
+  int32_t     only_if_faster;  /* 1: launch nothing and return 1 where one GEMM per weight is expected to be quicker */
   int32_t     reserved;   /* 0 */
   MiniAttnLinearOut out[3];
 } MiniAttnLinearParams;

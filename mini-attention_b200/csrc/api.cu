@@ -900,14 +900,6 @@ int miniattn_merge_partials(const MiniAttnMergeParams* p, void* stream) {
   return MINIATTN_OK;
 }
 
-// Whether work on the stream is being recorded into a graph (which the legacy stream cannot be).
-static bool captured(void* stream) {
-  if (stream == nullptr) return false;
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(reinterpret_cast<cudaStream_t>(stream), &status) == cudaSuccess &&
-         status != cudaStreamCaptureStatusNone;
-}
-
 static int check_rows(const void* p, int64_t ld, int cols, const char* name) {
   if (p == nullptr) return fail(MINIATTN_EINVAL, "%s is null", name);
   if (reinterpret_cast<uintptr_t>(p) % 16 != 0) return fail(MINIATTN_EINVAL, "%s must be 16-byte aligned", name);
@@ -943,10 +935,9 @@ int miniattn_linear(const MiniAttnLinearParams* p, void* stream) {
   const CUtensorMapDataType dt =
       p->dtype == MINIATTN_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   ma::LinearArgs a{};
-  ma::LinearPays pays;
+  bool pays = false;
   a.bn = ma::linear_tile(p->M, p->K, p->n_out, N, sms / 2, &pays);
-  if (p->only_if_faster && (pays == ma::LinearPays::kNo || (pays == ma::LinearPays::kIssuedOnly && captured(stream))))
-    return 1;
+  if (p->only_if_faster && !pays) return 1;
   a.status = p->status;
   a.M = p->M;
   a.K = p->K;

@@ -38,13 +38,6 @@ struct LinearArgs {
   FastDiv by_m_tiles;
 };
 
-// Where the one launch pays.
-enum class LinearPays {
-  kNo,          // one library GEMM for each weight is expected to be quicker
-  kIssuedOnly,  // quicker to issue, not to run: not in a call that is captured, where the host's time is not paid again
-  kYes,
-};
-
 // Width of a tile: fewest clocks over the rounds of tiles, at bn / 2 clk for 16 columns of K and about 1500 a tile.
 //
 // pays: against a library GEMM for each weight, which reaches 0.92 of the tensor rate and, like this launch, takes about
@@ -54,14 +47,17 @@ enum class LinearPays {
 //   q up to 1             0.84 to 1.02 / 0.82 to 1.02, mean 0.93: taken
 //   q up to 1.06          0.90 to 1.02 / 0.90 to 1.08, mean 0.98: taken, but with more than 32 MB of weights
 //                         1.01 to 1.03 / 1.06 to 1.11 (4096 wide: every pair fetches its operands itself through L2): not taken
-//   q above               0.94 to 1.17 / 0.94 to 1.32, mean 1.01: not taken
+//   q above               0.94 to 1.17 / 0.94 to 1.32, mean 1.01: not taken, but for launches of up to 24000 clk (13 us), 0.94 to
+//                         1.02: a module of such launches is bound by the host
 // One weight alone saves no launch, and the library's tiles are the better ones: the output projection in this form
 // 0.97 to 1.12 of the module, mean 1.03.  It is quicker to issue, though, and a module of up to about 60 us on the GPU is bound by
 // that: 2 x 1024 tokens, 16/4 heads of 128 65 us with the layers' calls, 61 with x's projections in one launch, 54 with the
-// output's as well, 52 to 57 on the GPU.  So launches of up to 24000 clk (13 us), which are those of such modules, are taken
-// where they are issued anew each time.  (Only after x's: one of this form between library calls takes the host 3 us more.)
+// output's as well, 52 to 57 on the GPU.  So launches of up to 24000 clk, which are those of such modules, are taken.  (Only
+// after x's: one of this form between library calls takes the host 3 us more.)
+// The answer is the same in a stream that is being captured, although a replay pays no host time: a library that the calls before
+// the capture never reached cannot be set up in one.
 // Never with so many columns of K that a tile would come near the bounded waits' limit (about 8 clk a column, 1 s).
-inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, LinearPays* pays) {
+inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, bool* pays) {
   const long long m_tiles = (M + 255ll) / 256;
   long long best = -1;
   int bn = kLinearMaxBn;
@@ -82,7 +78,7 @@ inline int linear_tile(int M, int K, int n_seg, const int* N, int pairs, LinearP
   const double launch = 3700.;
   const double own = best + launch, library = M * weights / (2. * pairs * 4096. * 0.92) + n_seg * launch;
   const bool quicker = n_seg > 1 && (own <= library || (own <= 1.06 * library && 2. * weights <= 32e6));
-  *pays = K > 1 << 24 ? LinearPays::kNo : quicker ? LinearPays::kYes : own <= 24000. ? LinearPays::kIssuedOnly : LinearPays::kNo;
+  *pays = K <= 1 << 24 && (quicker || own <= 24000.);
   return bn;
 }
 

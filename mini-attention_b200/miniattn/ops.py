@@ -602,7 +602,7 @@ def _operands(layer: torch.nn.Module, k: int, dt: torch.dtype, dev: int, grad: b
     return wp, b.data_ptr(), n
 
 
-# Sizes (of x, rows of each weight) for which one GEMM per layer is the quicker form, called anew or replayed.  A size that is found
+# Sizes (of x, rows of each weight) for which one GEMM per layer is the quicker form.  A size that is found
 # here is left to the layers before anything is looked at or allocated: finding that out again with each call took the host 12 us a
 # layer, 66 -> 113 us for a module none of whose projections is taken.
 _left_to_layers: set = set()
@@ -643,11 +643,10 @@ def _one_launch(x: torch.Tensor, layers, size):
     else:
         with torch.cuda.device(dev):
             rc = _lib.lib.miniattn_linear(block, _current_raw_stream(dev))
-    if rc == 1:  # one GEMM per layer is quicker; a captured call is judged by another rule
-        if not torch.cuda.is_current_stream_capturing():
-            if len(_left_to_layers) >= _LEFT_MAX:
-                _left_to_layers.clear()
-            _left_to_layers.add(size)
+    if rc == 1:  # one GEMM per layer is quicker
+        if len(_left_to_layers) >= _LEFT_MAX:
+            _left_to_layers.clear()
+        _left_to_layers.add(size)
         return None
     if rc != _lib.OK:
         _lib.check(rc, "miniattn_linear")

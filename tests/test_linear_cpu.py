@@ -120,18 +120,17 @@ def test_a_weight_of_more_rows_than_the_kernel_counts_is_left_to_the_layer():
         assert not _taken(layer)
 
 
-# Sizes at the ends of the ranges, where sums of them do not fit 32 bits, and where the one launch pays: 0 no, 1 where it
-# is issued anew each time, 2 yes.
+# Sizes at the ends of the ranges, where sums of them do not fit 32 bits, and where the one launch pays.
 TOP = 2 ** 31 - 1
 ENDS = [(TOP, 64, 64), (8, 64, TOP - 7), (64, TOP - 7, 8), (1, 8, 8)]
 PAYS = [
-    ((64, TOP - 7, 8), 0),                     # a tile of 2^31 columns of K would outlast the bounded waits
-    ((2048, 2048, 2048, 1024), 2), ((512, 512, 512, 256), 2), ((2277, 1536, 1536, 1536, 1536), 2), ((700, 3072, 3072, 3072, 3072), 2),
-    ((4768, 2048, 2048, 1024), 2),             # q = 1.03, 12 MB of weights
+    ((64, TOP - 7, 8), 0), ((64, TOP - 7, 8, 8), 0),    # a tile of 2^31 columns of K would outlast the bounded waits
+    ((2048, 2048, 2048, 1024), 1), ((512, 512, 512, 256), 1), ((2277, 1536, 1536, 1536, 1536), 1), ((700, 3072, 3072, 3072, 3072), 1),
+    ((4768, 2048, 2048, 1024), 1),             # q = 1.03, 12 MB of weights
     ((4096, 4096, 4096, 2048), 0),             # q = 1.02, 50 MB
     ((1554, 3072, 3072, 2048), 0), ((804, 4096, 4096, 4096), 0),   # q = 1.09, 1.20
     ((361, 4096, 4096, 1024), 1),              # q = 1.13, 20000 clk
-    ((2048, 2048, 2048), 1), ((512, 512, 512), 1), ((16384, 64, 64), 1),     # one weight: no launch saved
+    ((2048, 2048, 2048), 1), ((512, 512, 512), 1), ((16384, 64, 64), 1),     # one weight: where it is short
     ((4096, 4096, 4096), 0), ((8192, 2048, 2048), 0), ((16384, 4096, 4096), 0),
 ]
 RULE = r"""
@@ -143,9 +142,9 @@ int main() {
   for (auto& s : shapes) {
     int n = 1;
     while (n < 3 && s[2 + n] > 0) ++n;
-    ma::LinearPays pays;
+    bool pays = false;
     const int w = ma::linear_tile(s[0], s[1], n, &s[2], 74, &pays);
-    std::printf("%%d %%d ", w, static_cast<int>(pays));
+    std::printf("%%d %%d ", w, pays ? 1 : 0);
   }
   return 0;
 }

@@ -2,6 +2,10 @@
 path against the layers' own calls.  Both round once, from fp32 sums: a result is within half an ulp of its own size
 plus the fp32 sum's error, K * 2^-24 of the terms' size."""
 import ctypes as C
+import os
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 import torch
@@ -174,36 +178,31 @@ def test_more_rows_than_the_kernel_counts_go_through_the_layers(monkeypatch):
     assert ops.linear(x, lambda t: t.shape) == [x.shape]
 
 
-def test_a_captured_call_is_judged_by_the_gpus_time():
-    """One weight is quicker to issue in this form and not to run: taken in an ordinary call, left to the layer in a
-    captured one; two weights that save a launch are taken in both."""
-    def launch(n_out):
-        x, ws = torch.ones(512, 512, dtype=torch.float16, device=DEV), [torch.ones(512, 512, dtype=torch.float16, device=DEV)] * n_out
-        ys = [torch.zeros(512, 512, dtype=torch.float16, device=DEV) for _ in ws]
-        return (x, ws, [None] * n_out, ys), ys
-    stream = torch.cuda.Stream()
-    with torch.cuda.stream(stream):
-        for n_out in (1, 2):
-            args, ys = launch(n_out)
-            assert _launch(*args, only_if_faster=1) == _lib.OK
-            stream.synchronize()
-            for y in ys:
-                assert bool((y == 512).all())
-                y.zero_()
-            stream.synchronize()
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph, stream=stream):
-                rc = _launch(*args, only_if_faster=1)
-                ys[0] += 1.0
-            assert rc == (1 if n_out == 1 else _lib.OK)
-            graph.replay()
-            stream.synchronize()
-            assert bool((ys[0] == (1 if n_out == 1 else 513)).all())
+CAPTURE = """
+import torch
+from miniattn import GQA_Flash
+m = GQA_Flash(512, 8, 2).to(torch.bfloat16).to("cuda").requires_grad_(False)
+x = torch.randn(2, 300, 512, device="cuda", dtype=torch.bfloat16)
+want = m(x)
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = m(x)
+graph.replay()
+torch.cuda.synchronize()
+print(torch.equal(y, want))
+"""
+
+
+def test_a_captured_module_goes_the_way_of_the_calls_before_it():
+    """In a process of its own, whose other calls have not set up cuBLAS: that is not possible inside a capture."""
+    r = subprocess.run([sys.executable, "-c", CAPTURE], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=str(Path(miniattn.__file__).parents[1])))
+    assert r.returncode == 0 and r.stdout.strip() == "True", r.stderr[-2000:]
 
 
 def test_sizes_that_are_left_to_the_layers_are_known_the_second_time(monkeypatch):
-    """What is looked at for a size that does not pay: the layer once, nothing after that.  A captured call's answer is
-    not kept for calls that are issued."""
+    """What is looked at for a size that does not pay: the layer once, nothing after that."""
     seen, was = [], ops._operands
     monkeypatch.setattr(ops, "_operands", lambda *args: seen.append(1) or was(*args))
     monkeypatch.setattr(ops, "_left_to_layers", set())
@@ -213,17 +212,9 @@ def test_sizes_that_are_left_to_the_layers_are_known_the_second_time(monkeypatch
         assert torch.equal(ops.linear(x, lin)[0], lin(x))
     assert len(seen) == 1 and len(ops._left_to_layers) == 1
     small, sx = torch.nn.Linear(512, 512).half().to(DEV).requires_grad_(False), x[:, :512].contiguous()
-    small(sx)
-    torch.cuda.synchronize()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
+    for _ in range(2):                                # a size that pays
         ops.linear(sx, small)
-    assert len(ops._left_to_layers) == 1
-    launches, fn = [], _lib.lib.miniattn_linear
-    monkeypatch.setattr(ops._lib, "lib", type("Lib", (), {"miniattn_linear": staticmethod(
-        lambda *args: launches.append(fn(*args)) or launches[-1])}))
-    ops.linear(sx, small)
-    assert launches == [_lib.OK]
+    assert len(seen) == 3 and len(ops._left_to_layers) == 1
 
 
 @pytest.mark.parametrize("S,heads,names", [(300, (12, 4), ["w_q+kv", "w_o"]), (1554, (24, 8), []), (4768, (16, 4), ["w_q+kv"])])
